@@ -473,9 +473,11 @@ struct hgb_ilu {
     double *piv = nullptr;      // FP64 pivots for the F32/BF16 stores of an FP64 factor
     int *diag = nullptr;
     Schedule L, U;
-    void *tmp = nullptr;        // forward-solve output, kept in the pending state between applies
-    bool tmp_ready = false;
-    unsigned tmp_epoch = 0;     // context error epoch at the last refill of tmp
+    // forward-solve output of the 'N' and 'T' applies: between applies, every entry that the sweeps
+    // poll through memory is in the pending state (which entries depends on the pair of sweeps)
+    void *tmp = nullptr, *tmpT = nullptr;
+    bool tmp_ready = false, tmpT_ready = false;
+    unsigned tmp_epoch = 0;     // context error epoch at the last refill of tmp and tmpT
     // transposed view (built on first trans='T' apply)
     bool has_T = false;
     Transpose T;
@@ -506,6 +508,7 @@ static void ilu_free(hgb_ilu *M) {
     cudaFree(M->piv);
     cudaFree(M->diag);
     cudaFree(M->tmp);
+    cudaFree(M->tmpT);
     M->L.release();
     M->U.release();
     if (M->has_T) {
@@ -536,10 +539,9 @@ static int ilu_apply_n(hgb_ilu *M, const void *x, void *r, const int *skip) {
         M->tmp_epoch = c->error_epoch;
     }
     if (M->use_bs) {
-        // forward: unit lower, tmp <- L^-1 x (r reset to pending); backward: r <- U^-1 tmp
-        HGB_TRY(bsolve_launch<V, X>(c, M->BL, MODE_ILU, 1, X(1), (const X *)x, tmp, (X *)r, skip));
-        HGB_TRY(bsolve_launch<V, X>(c, M->BU, MODE_ILU, 0, X(1), tmp, (X *)r, tmp, skip));
-        return HGB_OK;
+        // forward: unit lower, tmp <- L^-1 x (the watched entries of r reset); backward: r <- U^-1 tmp
+        HGB_TRY(bsolve_launch<X>(c, M->BL, MODE_ILU, X(1), (const X *)x, tmp, (X *)r, skip));
+        return bsolve_launch<X>(c, M->BU, MODE_ILU, X(1), tmp, (X *)r, tmp, skip);
     }
     SolveArgs A{};
     A.pntr = M->pntr;
@@ -578,14 +580,20 @@ static int ilu_build_T(hgb_ilu *M) {
     HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 1, M->LT));
     HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 0, M->UT));
     if (M->use_bs) {
-        const int R = bsolve_rows(c, (int)xsize(M->store), M->n);
-        int st = bsolve_analyse(c, M->n, M->nnz, M->T.pntr, M->T.row, M->diagT, 1, 0, R, (int)xsize(M->store), M->BLT);
-        if (!st) st = bsolve_analyse(c, M->n, M->nnz, M->T.pntr, M->T.row, M->diagT, 0, 1, R, (int)xsize(M->store), M->BUT);
-        if (!st) st = bsolve_load_values(c, M->BLT, M->svalsT, (int)vsize(M->store), M->piv);
-        if (!st) st = bsolve_load_values(c, M->BUT, M->svalsT, (int)vsize(M->store), nullptr);
+        std::vector<int> hp(M->n + 1), hi(std::max(M->nnz, 1)), hd(M->n);
+        HGB_CUDA(cudaMemcpyAsync(hp.data(), M->T.pntr, sizeof(int) * (M->n + 1), cudaMemcpyDeviceToHost, c->stream));
+        HGB_CUDA(cudaMemcpyAsync(hi.data(), M->T.row, sizeof(int) * (size_t)M->nnz, cudaMemcpyDeviceToHost, c->stream));
+        HGB_CUDA(cudaMemcpyAsync(hd.data(), M->diagT, sizeof(int) * M->n, cudaMemcpyDeviceToHost, c->stream));
+        HGB_CUDA(cudaStreamSynchronize(c->stream));
+        BsPlanPair *plan = nullptr;
+        int st = bsolve_plan_pair(c, M->n, M->nnz, hp.data(), hi.data(), hd.data(), 1, 0, 1, (int)xsize(M->store), &plan);
+        if (!st) st = bsolve_load(c, plan->A, M->BLT, M->T.pntr, M->diagT, M->svalsT, (int)vsize(M->store), M->piv);
+        if (!st) st = bsolve_load(c, plan->B, M->BUT, M->T.pntr, M->diagT, M->svalsT, (int)vsize(M->store), nullptr);
+        bsolve_plan_pair_free(plan);
         if (st == HGB_OK) M->use_bsT = true;
         else if (st != HGB_ERR_UNSUPPORTED) return st;
     }
+    HGB_CUDA(cudaMalloc(&M->tmpT, xsize(M->store) * M->n));
     M->has_T = true;
     return HGB_OK;
 }
@@ -597,16 +605,15 @@ template <typename V, typename X>
 static int ilu_apply_t(hgb_ilu *M, const void *x, void *r, const int *skip) {
     hgb_ctx *c = M->ctx;
     if (!M->has_T) HGB_TRY(ilu_build_T(M));
-    X *tmp = (X *)M->tmp;
-    if (!M->tmp_ready) {
+    X *tmp = (X *)M->tmpT;
+    if (!M->tmpT_ready) {
         HGB_TRY(fill_pending<X>(c, M->n, tmp));
-        M->tmp_ready = true;
+        M->tmpT_ready = true;
         M->tmp_epoch = c->error_epoch;
     }
     if (M->use_bsT) {
-        HGB_TRY(bsolve_launch<V, X>(c, M->BLT, MODE_TRSV, 0, X(1), (const X *)x, tmp, (X *)r, skip));
-        HGB_TRY(bsolve_launch<V, X>(c, M->BUT, MODE_TRSV, 1, X(1), tmp, (X *)r, tmp, skip));
-        return HGB_OK;
+        HGB_TRY(bsolve_launch<X>(c, M->BLT, MODE_TRSV, X(1), (const X *)x, tmp, (X *)r, skip));
+        return bsolve_launch<X>(c, M->BUT, MODE_TRSV, X(1), tmp, (X *)r, tmp, skip);
     }
     SolveArgs A{};
     A.pntr = M->T.pntr;
@@ -713,7 +720,6 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
             int bs = HGB_OK;
             BsPlanPair *own = nullptr;
             if (!plan) {   // planned here, from host copies of the pattern
-                const int R = bsolve_rows(c, (int)xsize(store), n);
                 std::vector<int> hp(n + 1), hi(nnz), hd(n);
                 if (cudaMemcpyAsync(hp.data(), pntr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
                     cudaMemcpyAsync(hi.data(), indx, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
@@ -722,13 +728,12 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
                     st = cuda_fail(cudaGetLastError(), "ilu0_create");
                     break;
                 }
-                bs = bsolve_plan_pair(c, n, nnz, hp.data(), hi.data(), hd.data(), R, (int)xsize(store), &own);
+                bs = bsolve_plan_pair(c, n, nnz, hp.data(), hi.data(), hd.data(), 0, 1, 0, (int)xsize(store), &own);
                 plan = own;
             }
-            if (!bs) bs = bsolve_upload_pair(plan, M->BL, M->BU);
+            if (!bs) bs = bsolve_load(c, plan->A, M->BL, pntr, M->diag, M->svals, (int)vsize(store), nullptr);
+            if (!bs) bs = bsolve_load(c, plan->B, M->BU, pntr, M->diag, M->svals, (int)vsize(store), M->piv);
             bsolve_plan_pair_free(own);
-            if (!bs) bs = bsolve_load_values(c, M->BL, M->svals, (int)vsize(store), nullptr);
-            if (!bs) bs = bsolve_load_values(c, M->BU, M->svals, (int)vsize(store), M->piv);
             if (bs == HGB_OK) M->use_bs = true;
             else if (bs != HGB_ERR_UNSUPPORTED) { st = bs; break; }
         }
@@ -827,8 +832,7 @@ int hgb_ilu0_create_host(hgb_ctx *c, int n, int nnz, const int *pntr_h, const in
     const bool cplx = (vals_dtype == HGB_C128 || vals_dtype == HGB_C64);
     BsPlanPair *plan = nullptr;
     const int pst = cplx ? HGB_ERR_UNSUPPORTED
-                         : bsolve_plan_pair(c, n, nnz, pntr_h, indx_h, diag.data(),
-                                            bsolve_rows(c, (int)xsize(store), n), (int)xsize(store), &plan);
+                         : bsolve_plan_pair(c, n, nnz, pntr_h, indx_h, diag.data(), 0, 1, 0, (int)xsize(store), &plan);
     copier.join();
     int st = copy_status ? fail(copy_status, "%s", copy_msg.c_str()) : HGB_OK;
     int zero_pivot = 0;
@@ -857,7 +861,7 @@ namespace hgb {
 int ilu_apply_internal(hgb_ilu *M, char trans, const void *x, void *r, const int *skip) {
     if (!M || !x || !r) return fail(HGB_ERR_ARG, "ilu0_apply: bad arguments");
     DeviceGuard g(M->ctx->device);
-    if (M->tmp_epoch != M->ctx->error_epoch) M->tmp_ready = false;   // an earlier launch failed
+    if (M->tmp_epoch != M->ctx->error_epoch) M->tmp_ready = M->tmpT_ready = false;   // an earlier launch failed
     bool nt = (trans == 'N' || trans == 'n');
     bool tt = (trans == 'T' || trans == 't' || trans == 'C' || trans == 'c');
     if (!nt && !tt) return fail(HGB_ERR_ARG, "ilu0_apply: trans '%c'", trans);
