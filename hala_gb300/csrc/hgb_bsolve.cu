@@ -666,14 +666,7 @@ static int bs_mail(hgb_ctx *c, const BlockSolve &S, int init) {
 }
 
 void BlockSolve::release() {
-    cudaFree(blk);
-    cudaFree(strip);
-    cudaFree(packets);
-    cudaFree(watch);
-    cudaFree(mail);
-    cudaFree(ext_codes);
-    cudaFree(ext_vals);
-    cudaFree(ticket);
+    cudaFree(base);
     *this = BlockSolve();
 }
 
@@ -757,10 +750,18 @@ int bsolve_plan_pair(hgb_ctx *c, int n, int nnz, const int *pntr, const int *ind
 
 void bsolve_plan_pair_free(BsPlanPair *P) { delete P; }
 
-template <typename T>
-static int upload(hgb_ctx *c, T **dst, const std::vector<T> &src) {
-    HGB_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(src.size(), 1)));
-    if (!src.empty()) HGB_CUDA(cudaMemcpyAsync(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice, c->stream));
+// parts of one device allocation, each on a 256-byte boundary
+struct BsParts {
+    size_t total = 0;
+    size_t add(size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    }
+};
+template <typename A>
+static int upload(hgb_ctx *c, void *dst, const A &src) {
+    if (!src.empty()) HGB_CUDA(cudaMemcpyAsync(dst, src.data(), sizeof(*src.data()) * src.size(), cudaMemcpyHostToDevice, c->stream));
     return HGB_OK;
 }
 
@@ -787,38 +788,47 @@ int bsolve_load(hgb_ctx *c, const BsPlan &P, BlockSolve &S, const int *pntr, con
     S.nonunit = P.nonunit;
     S.deep = P.deep;
     S.dv_recip = (piv != nullptr && P.xsize == 4) ? 1 : 0;
-    int4 *chunk = nullptr, *step = nullptr, *pk = nullptr;
-    int *ext_map = nullptr;
+    BsParts dev, tmp;   // what stays, and what only the packing needs
+    const size_t o_blk = dev.add(sizeof(int4) * P.blk.size()), o_strip = dev.add(sizeof(int4) * P.strip.size()),
+                 o_watch = dev.add(sizeof(int2) * P.watch.size()), o_codes = dev.add(sizeof(int) * P.ext_codes.size()),
+                 o_vals = dev.add((size_t)P.xsize * P.ext_map.size()), o_pack = dev.add((size_t)P.units * 16),
+                 o_mail = dev.add((size_t)P.mail_units * 16), o_ticket = dev.add(sizeof(int) * 2);
+    const size_t t_chunk = tmp.add(sizeof(int4) * P.chunk.size()), t_step = tmp.add(sizeof(int4) * P.step.size()),
+                 t_pk = tmp.add(sizeof(int4) * P.pk.size()), t_map = tmp.add(sizeof(int) * P.ext_map.size());
+    HGB_CUDA(cudaMalloc(&S.base, dev.total));
+    S.blk = (int4 *)(S.base + o_blk);
+    S.strip = (int4 *)(S.base + o_strip);
+    S.watch = (int2 *)(S.base + o_watch);
+    S.ext_codes = (int *)(S.base + o_codes);
+    S.ext_vals = S.base + o_vals;
+    S.packets = S.base + o_pack;
+    S.mail = S.base + o_mail;
+    S.ticket = (int *)(S.base + o_ticket);
+    S.mail_n = P.mail_units * (16 / P.xsize);
+    S.mail_epoch = c->error_epoch;
+    unsigned char *w = nullptr;
+    if (ws_alloc(c, &w, tmp.total)) return cuda_fail(cudaErrorMemoryAllocation, "triangular plan");
     auto load = [&]() -> int {
-        HGB_TRY(upload(c, &S.blk, P.blk));
-        HGB_TRY(upload(c, &S.strip, P.strip));
-        HGB_TRY(upload(c, &S.watch, P.watch));
-        S.mail_n = P.mail_units * (16 / P.xsize);
-        HGB_CUDA(cudaMalloc(&S.mail, (size_t)std::max<long>(P.mail_units, 1) * 16));
-        HGB_TRY(bs_mail(c, S, 1));
-        S.mail_epoch = c->error_epoch;
-        HGB_TRY(upload(c, &S.ext_codes, P.ext_codes));
-        HGB_CUDA(cudaMalloc(&S.packets, (size_t)std::max<long>(P.units, 1) * 16));
-        HGB_CUDA(cudaMalloc(&S.ext_vals, (size_t)P.xsize * std::max<size_t>(P.ext_map.size(), 1)));
-        HGB_CUDA(cudaMalloc(&S.ticket, sizeof(int) * 2));
+        HGB_TRY(upload(c, w + t_chunk, P.chunk));
+        HGB_TRY(upload(c, w + t_step, P.step));
+        HGB_TRY(upload(c, w + t_pk, P.pk));
+        HGB_TRY(upload(c, w + t_map, P.ext_map));
+        HGB_TRY(upload(c, S.blk, P.blk));
+        HGB_TRY(upload(c, S.strip, P.strip));
+        HGB_TRY(upload(c, S.watch, P.watch));
+        HGB_TRY(upload(c, S.ext_codes, P.ext_codes));
         HGB_CUDA(cudaMemsetAsync(S.ticket, 0, sizeof(int) * 2, c->stream));
-        HGB_TRY(upload(c, &chunk, P.chunk));
-        HGB_TRY(upload(c, &step, P.step));
-        HGB_TRY(upload(c, &pk, P.pk));
-        HGB_TRY(upload(c, &ext_map, P.ext_map));
-        const BsPackArgs A{(int)P.chunk.size(), P.lower, P.rev, P.nonunit, chunk, step, pk, pntr, diag, piv, S.packets, S.blk, S.mail};
+        HGB_TRY(bs_mail(c, S, 1));
+        const BsPackArgs A{(int)P.chunk.size(), P.lower, P.rev, P.nonunit, (int4 *)(w + t_chunk), (int4 *)(w + t_step),
+                           (int4 *)(w + t_pk), pntr, diag, piv, S.packets, S.blk, S.mail};
         const long next = (long)P.ext_map.size();
-        if (vsize == 8) HGB_TRY((bs_pack<double, double>(c, A, svals, next, ext_map, S.ext_vals)));
-        else if (vsize == 4) HGB_TRY((bs_pack<float, float>(c, A, svals, next, ext_map, S.ext_vals)));
-        else HGB_TRY((bs_pack<uint16_t, float>(c, A, svals, next, ext_map, S.ext_vals)));
-        HGB_CUDA(cudaStreamSynchronize(c->stream));   // the staging arrays go
-        return HGB_OK;
+        const int *ext_map = (const int *)(w + t_map);
+        if (vsize == 8) return bs_pack<double, double>(c, A, svals, next, ext_map, S.ext_vals);
+        if (vsize == 4) return bs_pack<float, float>(c, A, svals, next, ext_map, S.ext_vals);
+        return bs_pack<uint16_t, float>(c, A, svals, next, ext_map, S.ext_vals);
     };
     const int st = load();
-    cudaFree(chunk);
-    cudaFree(step);
-    cudaFree(pk);
-    cudaFree(ext_map);
+    ws_free(c, w);
     return st;
 }
 

@@ -4,6 +4,7 @@
 #include "hgb_internal.cuh"
 
 #include <functional>
+#include <memory>
 #include <vector>
 
 namespace hgb {
@@ -39,6 +40,24 @@ constexpr int kBsFar = 1 << 11;   // << k: entry k comes from another strip or b
 // arrays; entry 0 / entry 2 of every other row is far (or padding); no row has an entry 2
 constexpr int kBsStepExt = 1 << 8, kBsEarly0 = 1 << 9, kBsEarly2 = 1 << 10, kBsNo2 = 1 << 11;
 
+// A host array whose elements start undefined: the pages of a large one are first touched by the threads
+// that fill it.
+template <typename T>
+struct BsArray {
+    std::unique_ptr<T[]> p;
+    size_t count = 0;
+    void resize(size_t n) {
+        p.reset(new T[n]);
+        count = n;
+    }
+    T *data() { return p.get(); }
+    const T *data() const { return p.get(); }
+    size_t size() const { return count; }
+    bool empty() const { return count == 0; }
+    T &operator[](size_t i) { return p[i]; }
+    const T &operator[](size_t i) const { return p[i]; }
+};
+
 // The schedule of one sweep as the host plans it (structure only).
 struct BsPlan {
     // deep: the pattern of a 3D grid (hgb_bsplan.cu)
@@ -51,10 +70,10 @@ struct BsPlan {
                                     // unit, 0} {units of its first chunks, 16 bits each}
     std::vector<int4> chunk;        // [steps], warp by warp: {first unit, step, units of the chunk D ahead, lowest row}
     std::vector<int4> step;         // [steps] {first packet, rows | flags, step whose rows it names or -1, block}
-    std::vector<int4> pk;           // [packets] the first piece of every packet
+    BsArray<int4> pk;               // [packets] the first piece of every packet
     std::vector<int2> watch;        // {global row, slot}, by block in the order of their first use
     std::vector<int> ext_codes, ext_map;
-    std::vector<int> pk_of_row;     // packet of every row
+    BsArray<int> pk_of_row;     // packet of every row
     std::vector<unsigned char> watched;   // rows that other blocks read through memory
 };
 
@@ -66,6 +85,7 @@ struct BsPlanPair {
 // Device copy of a plan with the values in the packets.
 struct BlockSolve {
     int n = 0, nblk = 0, cl = 1, nslots = 0, nflag = 0, xsize = 8, nonunit = 0, dv_recip = 0, deep = 0;
+    unsigned char *base = nullptr;   // the one allocation that holds all of the below
     int4 *blk = nullptr, *strip = nullptr;
     unsigned char *packets = nullptr;
     int2 *watch = nullptr;

@@ -4,9 +4,11 @@
 // atomic ticket in an order where everything a row depends on was handed out earlier, so a warp
 // only ever waits on warps that are already running, and each wait is bounded.
 //
-//  * Factorisation (and the forward level sets): warps take chunks of 32 consecutive rows in
+//  * Factorisation (and the forward level sets): warps take chunks of up to 32 consecutive rows in
 //    natural order and process them row by row; a row waits on the completion flags of the rows
-//    named by its strictly-lower entries.  The update order of every entry is the pivot order of
+//    named by its strictly-lower entries.  Chunks end at the end of a grid line (where the next row
+//    has no entry in the row before): a chunk that went on into the next line would make that
+//    line wait for the whole one before it.  The update order of every entry is the pivot order of
 //    factorize_ilu_array (sparse/hala_sparse_utils.hpp:229-255), with separately rounded multiply
 //    and subtract, so the factor is bit-identical to the reference CPU factor.
 //  * Triangular solves: rows are grouped by level into tasks of up to 32 rows of ONE level; a
@@ -53,18 +55,45 @@ __device__ __forceinline__ void st_relaxed_int(int *p, int v) {
     asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// bounded wait until lev[j] >= 0; acquire so that data published before the flag is visible
-__device__ __forceinline__ int wait_level(const int *lev, int j, int *err) {
-    int v = ld_acquire(lev + j);
-    int spins = 0;
-    while (v < 0) {
-        if (++spins > kSpinLimit) {
-            atomicOr(err, DEV_ERR_TIMEOUT);
-            return 0;
-        }
+// Bounded wait for a row's completion flag (>= 0): lane 0 polls, with pauses that grow with the wait (all
+// the chunks of the matrix that fit are resident, most of them waiting); its acquire and the warp
+// barrier order the other lanes' reads of that row behind it.
+__device__ __forceinline__ int wait_row(const int *lev, int j, int lane, int *err) {
+    int v = 0;
+    if (lane == 0) {
         v = ld_acquire(lev + j);
+        for (int spins = 0; v < 0; spins++) {
+            if (spins > kSpinLimit || ((spins & 255) == 255 && (*(volatile int *)err & DEV_ERR_TIMEOUT))) {
+                atomicOr(err, DEV_ERR_TIMEOUT);
+                v = 0;
+                break;
+            }
+            __nanosleep(spins < 8 ? 20 : (spins < 64 ? 100 : 400));
+            v = ld_acquire(lev + j);
+        }
     }
-    return v;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// Starts of the chunks (by position in solve order): every 32nd position, and the rows without an entry in
+// the row before (columns are sorted: it would sit beside the diagonal).
+__global__ void chunk_flag_kernel(int n, const int *__restrict__ pntr, const int *__restrict__ indx,
+                                  const int *__restrict__ diag, int lower, int *flag) {
+    for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos <= n; pos += gridDim.x * blockDim.x) {
+        if (pos == n) {
+            flag[pos] = 0;
+            continue;
+        }
+        const int i = lower ? pos : n - 1 - pos, d = diag[i];
+        const bool chained = lower ? (d > pntr[i] && indx[d - 1] == i - 1) : (d + 1 < pntr[i + 1] && indx[d + 1] == i + 1);
+        flag[pos] = (pos & 31) == 0 || !chained;
+    }
+}
+__global__ void chunk_fill_kernel(int n, const int *__restrict__ at, int *start) {
+    for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += gridDim.x * blockDim.x)
+        if (at[pos + 1] != at[pos]) start[at[pos]] = pos;
+    if (blockIdx.x == 0 && threadIdx.x == 0) start[at[n]] = n;
 }
 
 // Level sets over the pattern: lower: deps are entries [pntr_i, diag_i) and rows are taken in
@@ -73,33 +102,28 @@ __device__ __forceinline__ int wait_level(const int *lev, int j, int *err) {
 __global__ void __launch_bounds__(256) levels_kernel(int n, const int *__restrict__ pntr,
                                                      const int *__restrict__ indx,
                                                      const int *__restrict__ diag, int lower, int *lev,
+                                                     const int *__restrict__ start, const int *__restrict__ nchunks_d,
                                                      int *ticket, int *err) {
     __shared__ int chunk_lev[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nchunks = (n + 31) / 32;
+    const int nchunks = __ldg(nchunks_d);
     for (;;) {
         int c = 0;
         if (lane == 0) c = atomicAdd(ticket, 1);
         c = __shfl_sync(0xffffffffu, c, 0);
         if (c >= nchunks) break;
-        // chunk c covers processing positions [32c, 32c+32)
-        for (int k = 0; k < 32; k++) {
-            int pos = c * 32 + k;
-            if (pos >= n) break;
-            int row = lower ? pos : n - 1 - pos;
-            int a = lower ? __ldg(pntr + row) : __ldg(diag + row) + 1;
-            int b = lower ? __ldg(diag + row) : __ldg(pntr + row + 1);
+        const int p0 = __ldg(start + c), p1 = __ldg(start + c + 1);
+        for (int pos = p0; pos < p1; pos++) {
+            const int row = lower ? pos : n - 1 - pos;
+            const int a = lower ? __ldg(pntr + row) : __ldg(diag + row) + 1;
+            const int b = lower ? __ldg(diag + row) : __ldg(pntr + row + 1);
             int m = -1;
-            for (int p = a + lane; p < b; p += 32) {
-                int j = __ldg(indx + p);
-                int jpos = lower ? j : n - 1 - j;
-                int lj = (jpos >= c * 32) ? chunk_lev[w][jpos - c * 32] : wait_level(lev, j, err);
-                m = max(m, lj);
+            for (int p = a; p < b; p++) {
+                const int j = __ldg(indx + p), jpos = lower ? j : n - 1 - j;
+                m = max(m, jpos >= p0 ? chunk_lev[w][jpos - p0] : wait_row(lev, j, lane, err));
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (lane == 0) {
-                chunk_lev[w][k] = m + 1;
+                chunk_lev[w][pos - p0] = m + 1;
                 st_release(lev + row, m + 1);
             }
             __syncwarp();
@@ -116,35 +140,33 @@ __global__ void __launch_bounds__(256) levels_kernel(int n, const int *__restric
     }
 }
 
-
 template <typename T> __device__ __forceinline__ T ld_val(const T *p) { return ld_relaxed(p); }
 
-// Row-wise IKJ ILU(0) in place on f (a copy of the matrix values) + forward level sets.
+// Row-wise IKJ ILU(0) in place on f (a copy of the matrix values) + forward level sets.  A row is a chain
+// of dependent L2 reads (flag, diagonal, the pivot row's columns and values) of about 4 us; what
+// counts is that the rows of a wavefront are all in flight.
 template <typename T>
 __global__ void __launch_bounds__(256) ilu_factor_kernel(int n, const int *__restrict__ pntr,
                                                          const int *__restrict__ indx,
                                                          const int *__restrict__ diag, T *f, int *lev,
+                                                         const int *__restrict__ start, const int *__restrict__ nchunks_d,
                                                          int *ticket, int *err) {
     __shared__ int chunk_lev[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nchunks = (n + 31) / 32;
+    const int nchunks = __ldg(nchunks_d);
     for (;;) {
         int c = 0;
         if (lane == 0) c = atomicAdd(ticket, 1);
         c = __shfl_sync(0xffffffffu, c, 0);
         if (c >= nchunks) break;
-        for (int k = 0; k < 32; k++) {
-            const int i = c * 32 + k;
-            if (i >= n) break;
+        const int i0 = __ldg(start + c), i1 = __ldg(start + c + 1);
+        for (int i = i0; i < i1; i++) {
             const int a = __ldg(pntr + i), b = __ldg(pntr + i + 1), d = __ldg(diag + i);
             int m = -1;
             for (int p = a; p < d; p++) {          // pivots in ascending column order
                 const int kr = __ldg(indx + p);
-                int lk;
-                if (kr >= c * 32) lk = chunk_lev[w][kr - c * 32];
-                else lk = wait_level(lev, kr, err);   // every lane waits: acquire per lane
-                m = max(m, lk);
                 const int dk = __ldg(diag + kr), ek = __ldg(pntr + kr + 1);
+                m = max(m, kr >= i0 ? chunk_lev[w][kr - i0] : wait_row(lev, kr, lane, err));
                 const T ukk = ld_val(f + dk);
                 // owner lane of position p scales a_ik; everyone gets l from it
                 const int owner = (p - a) & 31;
@@ -173,7 +195,7 @@ __global__ void __launch_bounds__(256) ilu_factor_kernel(int n, const int *__res
             __threadfence();
             __syncwarp();
             if (lane == 0) {
-                chunk_lev[w][k] = m + 1;
+                chunk_lev[w][i - i0] = m + 1;
                 st_release(lev + i, m + 1);
             }
             __syncwarp();
@@ -284,14 +306,38 @@ static int sync_grid(hgb_ctx *c, int work_items, int per_block) {
     return std::max(1, std::min(g, c->num_sms * 8));
 }
 
+// The chunk list of a pattern and direction: *start (n + 1 positions) and the device count, from the
+// context's pool; both are freed with ws_free(*work).
+static int make_chunks(hgb_ctx *c, int n, const int *pntr, const int *indx, const int *diag, int lower, int **work,
+                       const int **start, const int **count) {
+    int *w = nullptr;
+    const size_t nb = (size_t)(n + 1 + 1023) / 1024 + 1;
+    if (ws_alloc(c, &w, 3 * ((size_t)n + 1) + nb + 1)) return cuda_fail(cudaErrorMemoryAllocation, "factorisation chunks");
+    int *flag = w, *at = w + n + 1, *st = at + n + 1, *scratch = st + n + 1;
+    const int g = std::max(1, std::min((n + 256) / 256, c->num_sms * 8));
+    chunk_flag_kernel<<<g, 256, 0, c->stream>>>(n, pntr, indx, diag, lower, flag);
+    const int s = exclusive_scan(c, flag, at, n + 1, scratch + nb, scratch);
+    chunk_fill_kernel<<<g, 256, 0, c->stream>>>(n, at, st);
+    *work = w;
+    *start = st;
+    *count = at + n;
+    return s ? s : launch_check("chunk_fill_kernel");
+}
+
 // Levels of one solve direction over (pntr, indx, diag), then the schedule.
 static int analyse(hgb_ctx *c, int n, const int *pntr, const int *indx, const int *diag, int lower, Schedule &S) {
     HGB_TRY(alloc_schedule(c, S, n));
-    levels_kernel<<<sync_grid(c, (n + 31) / 32, 8), 256, 0, c->stream>>>(n, pntr, indx, diag, lower, S.level,
-                                                                         S.ticket, c->err);
-    HGB_TRY(launch_check("levels_kernel"));
-    HGB_TRY(collect_dev_error(c));
-    return build_schedule(c, S, lower);
+    int *work = nullptr;
+    const int *start = nullptr, *count = nullptr;
+    int st = make_chunks(c, n, pntr, indx, diag, lower, &work, &start, &count);
+    if (!st) {
+        // up to n chunks: the full grid where the matrix is large
+        levels_kernel<<<sync_grid(c, n, 8), 256, 0, c->stream>>>(n, pntr, indx, diag, lower, S.level, start, count, S.ticket, c->err);
+        st = launch_check("levels_kernel");
+    }
+    if (!st) st = collect_dev_error(c);
+    ws_free(c, work);
+    return st ? st : build_schedule(c, S, lower);
 }
 
 // ------------------------------------------------------------ triangular solve ---------
@@ -577,8 +623,6 @@ static int ilu_build_T(hgb_ilu *M) {
     else gather_kernel<uint16_t><<<g, 256, 0, c->stream>>>(M->nnz, M->T.map, (const uint16_t *)M->svals, (uint16_t *)M->svalsT);
     HGB_TRY(launch_check("gather_kernel"));
     // U^T is the lower triangle of the transposed pattern, L^T its upper triangle
-    HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 1, M->LT));
-    HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 0, M->UT));
     if (M->use_bs) {
         std::vector<int> hp(M->n + 1), hi(std::max(M->nnz, 1)), hd(M->n);
         HGB_CUDA(cudaMemcpyAsync(hp.data(), M->T.pntr, sizeof(int) * (M->n + 1), cudaMemcpyDeviceToHost, c->stream));
@@ -592,6 +636,10 @@ static int ilu_build_T(hgb_ilu *M) {
         bsolve_plan_pair_free(plan);
         if (st == HGB_OK) M->use_bsT = true;
         else if (st != HGB_ERR_UNSUPPORTED) return st;
+    }
+    if (!M->use_bsT) {
+        HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 1, M->LT));
+        HGB_TRY(analyse(c, M->n, M->T.pntr, M->T.row, M->diagT, 0, M->UT));
     }
     HGB_CUDA(cudaMalloc(&M->tmpT, xsize(M->store) * M->n));
     M->has_T = true;
@@ -669,6 +717,13 @@ static int ilu_check_args(hgb_ctx *c, int n, int nnz, const void *pntr, const vo
     return HGB_OK;
 }
 
+// The global-level schedules: for the sweeps that have no strip plan, and for hgb_ilu0_levels.
+static int ilu_schedules(hgb_ilu *M) {
+    if (!M->L.perm) HGB_TRY(build_schedule(M->ctx, M->L, 1));   // its levels came with the factorisation
+    if (!M->U.perm) HGB_TRY(analyse(M->ctx, M->n, M->pntr, M->indx, M->diag, 0, M->U));
+    return HGB_OK;
+}
+
 // The device part of ILU(0) creation.  plan: when given, the block-solve schedules were planned on
 // the host already (from host arrays); otherwise they are planned here from D2H copies.
 static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const int *indx, const void *vals,
@@ -684,6 +739,7 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
     M->store = store;
     int st = HGB_OK;
     int zero_pivot = 0;
+    BsPlanPair *own = nullptr;
     do {
         if (cudaMalloc(&M->diag, sizeof(int) * n) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
         if ((st = hgb_diag_index(c, n, nnz, pntr, indx, M->diag))) break;
@@ -691,17 +747,37 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
         if (cudaMalloc(&M->fvals, fs * nnz) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
         if (cudaMemcpyAsync(M->fvals, vals, fs * nnz, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
         if ((st = alloc_schedule(c, M->L, n))) break;
-        int blocks = sync_grid(c, (n + 31) / 32, 8);
+        int *work = nullptr;
+        const int *start = nullptr, *count = nullptr;
+        if ((st = make_chunks(c, n, pntr, indx, M->diag, 1, &work, &start, &count))) break;
+        const int blocks = sync_grid(c, n, 8);   // up to n chunks
         if (vals_dtype == HGB_F64)
-            ilu_factor_kernel<double><<<blocks, 256, 0, c->stream>>>(n, pntr, indx, M->diag, (double *)M->fvals, M->L.level, M->L.ticket, c->err);
+            ilu_factor_kernel<double><<<blocks, 256, 0, c->stream>>>(n, pntr, indx, M->diag, (double *)M->fvals, M->L.level, start, count, M->L.ticket, c->err);
         else
-            ilu_factor_kernel<float><<<blocks, 256, 0, c->stream>>>(n, pntr, indx, M->diag, (float *)M->fvals, M->L.level, M->L.ticket, c->err);
-        if ((st = launch_check("ilu_factor_kernel"))) break;
+            ilu_factor_kernel<float><<<blocks, 256, 0, c->stream>>>(n, pntr, indx, M->diag, (float *)M->fvals, M->L.level, start, count, M->L.ticket, c->err);
+        st = launch_check("ilu_factor_kernel");
+        ws_free(c, work);
+        if (st) break;
+        // the sweeps are planned on the host while the factorisation runs
+        int bs = HGB_OK;
+        if (!plan) {
+            BsArray<int> hp, hi, hd;
+            hp.resize(n + 1);
+            hi.resize(nnz);
+            hd.resize(n);
+            if (cudaMemcpyAsync(hp.data(), pntr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, c->copy) != cudaSuccess ||
+                cudaMemcpyAsync(hi.data(), indx, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, c->copy) != cudaSuccess ||
+                cudaMemcpyAsync(hd.data(), M->diag, sizeof(int) * n, cudaMemcpyDeviceToHost, c->copy) != cudaSuccess ||
+                cudaStreamSynchronize(c->copy) != cudaSuccess) {
+                st = cuda_fail(cudaGetLastError(), "ilu0_create");
+                break;
+            }
+            bs = bsolve_plan_pair(c, n, nnz, hp.data(), hi.data(), hd.data(), 0, 1, 0, (int)xsize(store), &own);
+            plan = own;
+        }
         st = collect_dev_error(c);
         if (st == HGB_ERR_ZERO_PIVOT) { zero_pivot = 1; st = HGB_OK; }
         if (st) break;
-        if ((st = build_schedule(c, M->L, 1))) break;
-        if ((st = analyse(c, n, pntr, indx, M->diag, 0, M->U))) break;
         // store precision
         if (store == vals_dtype) {
             M->svals = M->fvals;
@@ -716,29 +792,15 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
             if ((st = launch_check("ilu store conversion"))) break;
         }
         if (cudaMalloc(&M->tmp, xsize(store) * n) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
-        {   // block-local schedules; patterns they cannot hold fall back to the global-level solve
-            int bs = HGB_OK;
-            BsPlanPair *own = nullptr;
-            if (!plan) {   // planned here, from host copies of the pattern
-                std::vector<int> hp(n + 1), hi(nnz), hd(n);
-                if (cudaMemcpyAsync(hp.data(), pntr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
-                    cudaMemcpyAsync(hi.data(), indx, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
-                    cudaMemcpyAsync(hd.data(), M->diag, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
-                    cudaStreamSynchronize(c->stream) != cudaSuccess) {
-                    st = cuda_fail(cudaGetLastError(), "ilu0_create");
-                    break;
-                }
-                bs = bsolve_plan_pair(c, n, nnz, hp.data(), hi.data(), hd.data(), 0, 1, 0, (int)xsize(store), &own);
-                plan = own;
-            }
-            if (!bs) bs = bsolve_load(c, plan->A, M->BL, pntr, M->diag, M->svals, (int)vsize(store), nullptr);
-            if (!bs) bs = bsolve_load(c, plan->B, M->BU, pntr, M->diag, M->svals, (int)vsize(store), M->piv);
-            bsolve_plan_pair_free(own);
-            if (bs == HGB_OK) M->use_bs = true;
-            else if (bs != HGB_ERR_UNSUPPORTED) { st = bs; break; }
-        }
+        // patterns that the strip plan cannot hold fall back to the global-level solve
+        if (!bs) bs = bsolve_load(c, plan->A, M->BL, pntr, M->diag, M->svals, (int)vsize(store), nullptr);
+        if (!bs) bs = bsolve_load(c, plan->B, M->BU, pntr, M->diag, M->svals, (int)vsize(store), M->piv);
+        if (bs == HGB_OK) M->use_bs = true;
+        else if (bs != HGB_ERR_UNSUPPORTED) { st = bs; break; }
+        else if ((st = ilu_schedules(M))) break;
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
     } while (0);
+    bsolve_plan_pair_free(own);
     if (zero_pivot_out) *zero_pivot_out = zero_pivot;
     return st;
 }
@@ -898,6 +960,7 @@ int hgb_ilu0_levels(hgb_ilu *M, char uplo, int *level, int *nlevels) {
     if (M->z) return fail(HGB_ERR_UNSUPPORTED, "ilu0_levels: real factors");
     hgb_ctx *c = M->ctx;
     DeviceGuard g(c->device);
+    HGB_TRY(ilu_schedules(M));
     const Schedule &S = (uplo == 'L' || uplo == 'l') ? M->L : M->U;
     if (level) HGB_CUDA(cudaMemcpyAsync(level, S.level, sizeof(int) * M->n, cudaMemcpyDeviceToDevice, c->stream));
     if (nlevels) *nlevels = S.nlevels;

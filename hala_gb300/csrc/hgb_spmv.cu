@@ -396,17 +396,31 @@ __global__ void scan_blocks_kernel(const int *__restrict__ in, int *__restrict__
     if (threadIdx.x == 1023) block_tot[blockIdx.x] = sh[1023];
 }
 
-__global__ void scan_tot_kernel(int *tot, int nb, int *grand) {
-    // sequential exclusive scan of the block totals by one thread (nb is small)
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int run = 0;
-        for (int b = 0; b < nb; b++) {
-            int t = tot[b];
-            tot[b] = run;
-            run += t;
+__global__ void __launch_bounds__(1024) scan_tot_kernel(int *tot, int nb, int *grand) {
+    // exclusive scan of the block totals by one CTA, 1024 at a time
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int run = 0;
+    for (int b0 = 0; b0 < nb; b0 += 1024) {
+        const int b = b0 + threadIdx.x, t = b < nb ? tot[b] : 0;
+        int v = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
         }
-        *grand = run;
+        if (lane == 31) wsum[w] = v;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int k = 0; k < 32; k++) {
+            if (k < w) before += wsum[k];
+            all += wsum[k];
+        }
+        if (b < nb) tot[b] = run + before + v - t;
+        run += all;
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *grand = run;
 }
 
 __global__ void scan_add_kernel(int *out, int n, const int *tot) {
@@ -451,7 +465,7 @@ int exclusive_scan(hgb_ctx *c, const int *in, int *out, int n, int *total_dev, i
     int nb = (n + 1023) / 1024;
     if (nb == 0) return HGB_OK;
     scan_blocks_kernel<<<nb, 1024, 0, c->stream>>>(in, out, n, scratch);
-    scan_tot_kernel<<<1, 32, 0, c->stream>>>(scratch, nb, total_dev);
+    scan_tot_kernel<<<1, 1024, 0, c->stream>>>(scratch, nb, total_dev);
     scan_add_kernel<<<nb, 1024, 0, c->stream>>>(out, n, scratch);
     return launch_check("exclusive_scan");
 }

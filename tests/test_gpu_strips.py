@@ -39,9 +39,24 @@ CASES = {
     "grid_32x33x70": lambda rng: P.aniso3d(32, 33, 70),       # many blocks: several clusters
     "grid_96x8x40": lambda rng: P.aniso3d(96, 8, 40),         # planes of fewer lines than a strip
     "grid_256x160x5": lambda rng: P.aniso3d(256, 160, 5),     # a plane over several blocks: two readers per row
+    # odd grid lines: the factorisation's chunks end with the line
+    "grid_63x65x61": lambda rng: P.aniso3d(63, 65, 61),
+    "grid_301x97": lambda rng: P.poisson2d(301, 97),
     "stencil27_32x21x19": lambda rng: stencil27(32, 21, 19, rng),
     "random_30000": lambda rng: P.random_csr_sparse(30000, 12, rng),
 }
+
+
+@pytest.mark.parametrize("name", ["grid_33x17", "grid_64x65x9", "grid_301x97", "random_30000"])
+def test_level_sets_of_chunked_factor(eng, rng, name):
+    # the level sets come from the factorisation's chunks (lower) and from the level kernel's (upper)
+    p, i, v = CASES[name](rng)
+    do = O.diag_index(p, i)
+    ilu = E.make_ilu(eng, T(p), T(i), T(v))
+    for uplo in "LU":
+        lev, nl = ilu.levels(uplo)
+        lo, nlo = O.levels(p, i, do, uplo)
+        assert nl == nlo and np.array_equal(lev.cpu().numpy(), lo)
 
 
 @pytest.mark.parametrize("name", list(CASES))
