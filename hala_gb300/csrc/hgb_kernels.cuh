@@ -91,13 +91,13 @@ int build_transpose(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr
                     Transpose &T);
 
 template <typename V>
-int spmv_n_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals,
+int spmv_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                   typename Val<V>::X *y, double *dot_out, const int *skip = nullptr, int *nparts = nullptr);
 // Y = alpha A X + beta Y over nrhs column-major columns, the matrix read once (each column
 // bit-identical to spmv_n_launch's product)
 template <typename V>
-int spmm_n_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals, int nrhs,
+int spmm_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals, int nrhs,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
                   typename Val<V>::X *y, long ldy);
 template <typename V>

@@ -1,9 +1,9 @@
-// CSR SpMV for sm_103a.  One warp takes 32 consecutive rows at a time: it copies the tile's whole
-// vals / indx range into its own shared-memory buffer with coalesced 16-byte cp.async (no
+// CSR SpMV and SpMM for sm_103a.  One warp takes 32 consecutive rows (a tile) at a time: it copies the
+// tile's whole vals / indx range into its own shared-memory buffer with coalesced 16-byte cp.async (no
 // handshake between warps), then every lane sums its row from shared memory, gathering x from
-// global memory (L2) kGW entries at a time.  The warp double-buffers: the copy of tile k+1 and the
-// row pointers of tile k+2 are in flight while tile k is summed.  Tiles of more than kWarpCap
-// entries read their rows directly.
+// global memory (L1 / L2).  The copies of the next kStages - 1 tiles and the row pointers of the tile
+// after them are in flight while a tile is summed.  Tiles of more than CAP entries read their rows
+// directly.
 //
 // Two arithmetic modes, chosen per context (hgb_ctx_set_spmv_mode):
 //  - exact: each row summed in column order with separately rounded multiply and add, the
@@ -19,6 +19,7 @@
 #include "hgb_complex.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <string>
 #include <vector>
@@ -27,9 +28,28 @@ namespace hgb {
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
-constexpr int kWarpCap = 256;
 constexpr int kWarpBlock = 256;   // 8 warps per CTA
-constexpr int kGW = 4;            // x gathers in flight per lane
+constexpr int kStages = 2;        // tiles per warp in shared memory; three or four measured no gain
+constexpr int kMmCols = 5;        // columns summed per pass over a tile at most
+constexpr int kCapShort = 256, kCapLong = 384;   // entries of a staged tile (spmv_long_rows)
+
+// CTAs per SM and x gathers in flight per lane and column, by vector type, columns per pass and
+// tile size.  More CTAs leave less of the 256 KB for L1, which holds the gathered part of x and the
+// rows that are read directly, and fewer registers for gathers; fewer CTAs leave HBM idle.  Measured
+// (us; 128^3 7-point FP64 / FP32, graph Laplacians of 680k rows FP64 / FP32, 5 columns on 95x97x96 FP64 / FP32):
+//   FP64, 256 entries: 3 CTAs of 4 gathers 47.8; 2: 61.5; 6: 115; 3 of 8 (spills) 76.9.
+//   FP32, 256 entries: 4 CTAs of 8 gathers 28.7; of 4 gathers 31.1; 3 of 8 36.3.
+//   384 entries (rows of 9, which 256 would send to the direct path): FP64 2 CTAs 31.6, 3: 35.2; FP32 3 CTAs of
+//   4 gathers 16.9, of 8 20.2, 2 of 4 18.5.
+//   columns: FP64 3 CTAs with one gather per column 68, with two and passes of 3 + 2 columns 78.7; FP32 3 CTAs
+//   with two 28.8, 4 with three 39.0.
+// Before (one shape for all, 4 gathers, passes of 4 columns with one): 55.4 / 29.1, 33.2 / 26.7, 108.6 / 43.1.
+template <typename X, int NC, int CAP>
+struct TileShape {
+    static constexpr bool f64 = sizeof(X) == 8, wide = CAP > kCapShort;
+    static constexpr int ctas = NC == 1 ? (f64 ? (wide ? 2 : 3) : (wide ? 3 : 4)) : (wide ? 2 : (f64 && NC == 2 ? 4 : 3));
+    static constexpr int gathers = NC == 1 ? (f64 || wide ? 4 : 8) : (f64 ? (NC == 2 ? 2 : 1) : (NC == 2 ? 6 : 12 / NC));
+};
 
 // acc += v * x in the mode's rounding
 template <bool EXACT>
@@ -40,13 +60,30 @@ template <bool EXACT>
 __device__ __forceinline__ float spmv_acc(float acc, float v, float x) {
     return EXACT ? add_rn(acc, mul_rn(v, x)) : __fmaf_rn(v, x, acc);
 }
-// alpha * acc + beta * y (y read only when beta != 0)
+// How a product ends: y = acc (alpha 1, beta 0), alpha acc, or alpha acc + beta y.  Chosen on the host: an FP64
+// comparison per row would hold the FP64 unit as long as a multiply-add.
+enum SpmvEnd : int { END_PLAIN = 0, END_SCALED = 1, END_FULL = 2 };
+template <typename X>
+static SpmvEnd spmv_end(X alpha, X beta) {
+    return beta != X(0) ? END_FULL : (alpha == X(1) ? END_PLAIN : END_SCALED);
+}
+// (EXACT: alpha acc, with beta y added, separately rounded; 1 times acc is acc)
 template <bool EXACT, typename X>
-__device__ __forceinline__ X spmv_out(X alpha, X acc, X beta, const X *yp) {
-    if (EXACT) return (beta == X(0)) ? mul_rn(alpha, acc) : add_rn(mul_rn(alpha, acc), mul_rn(beta, *yp));
-    if (beta == X(0)) return (alpha == X(1)) ? acc : mul_rn(alpha, acc);
+__device__ __forceinline__ X spmv_out(int end, X alpha, X acc, X beta, const X *yp) {
+    if (end == END_PLAIN) return acc;
+    if (end == END_SCALED) return mul_rn(alpha, acc);
+    if (EXACT) return add_rn(mul_rn(alpha, acc), mul_rn(beta, *yp));
     return spmv_acc<false>(mul_rn(beta, *yp), alpha, acc);
 }
+
+// A warp-uniform choice that stays a branch for FP64: a predicated-off FP64 instruction would hold the
+// unit like any other.
+__device__ __forceinline__ bool spmv_uniform(bool c, double) {
+    int v = c;
+    asm volatile("" : "+r"(v));
+    return v;
+}
+__device__ __forceinline__ bool spmv_uniform(bool c, float) { return c; }
 
 // The fused <x, y> (DOT): 0 none; 1 the grid reduction into *dot_out (the last CTA adds the
 // parts); 2 each CTA's part to partials[blockIdx.x], summed by the consuming kernel (in one order
@@ -62,42 +99,45 @@ __device__ __forceinline__ void spmv_dot_epilogue(double d, double *partials, un
     }
 }
 
-// y = alpha * A x + beta * y ; optionally <x, y> (square A; DOT as spmv_dot_epilogue)
-template <typename V, int DOT, bool EXACT>
-__global__ void __launch_bounds__(kWarpBlock)
-spmv_warp_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx, const V *__restrict__ vals,
-                 typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x, typename Val<V>::X beta,
-                 typename Val<V>::X *__restrict__ y, double *partials, unsigned *counter, double *dot_out,
-                 const int *skip) {
+// Y = alpha * A X + beta * Y for nrhs column-major columns (x column c at x + c * ldx), cols <= NC of them per
+// pass over a staged tile (the matrix is read once); optionally <x, y> (one column, square A; DOT as
+// spmv_dot_epilogue).  Every column is summed in column order in the mode's rounding, so each column
+// equals the single-column product bit for bit.
+template <typename V, int NC, int CAP, int DOT, bool EXACT>
+__global__ void __launch_bounds__(kWarpBlock, TileShape<typename Val<V>::X, NC, CAP>::ctas)
+spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx, const V *__restrict__ vals,
+                 int nrhs, int cols, int end_mode, typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x,
+                 long ldx, typename Val<V>::X beta, typename Val<V>::X *__restrict__ y, long ldy, double *partials,
+                 unsigned *counter, double *dot_out, const int *skip) {
     using X = typename Val<V>::X;
     constexpr int EV = 16 / (int)sizeof(V);   // values per 16-byte unit
-    constexpr int SV = kWarpCap + 2 * EV, SI = kWarpCap + 8;
+    constexpr int SV = CAP + 2 * EV, SI = CAP + 8, ST = kStages;
+    static_assert(CAP % 8 == 0, "every buffer starts on a 16-byte boundary");
     if (skip && *skip) return;
-    __shared__ __align__(16) V s_vals[kWarpBlock / 32][2][SV];
-    __shared__ __align__(16) int s_idx[kWarpBlock / 32][2][SI];
+    extern __shared__ __align__(16) unsigned char spmv_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    V *const s_vals = (V *)spmv_smem + wib * ST * SV;
+    int *const s_idx = (int *)((V *)spmv_smem + (kWarpBlock / 32) * ST * SV) + wib * ST * SI;
     const int nnz = __ldg(pntr + n_rows);
-    const long ntiles = ((long)n_rows + 31) / 32;
-    const long nwarps = (long)gridDim.x * (kWarpBlock / 32);
-    const long per = (ntiles + nwarps - 1) / nwarps;
-    const long tb = ((long)blockIdx.x * (kWarpBlock / 32) + wib) * per;
-    const long te = min(ntiles, tb + per);
+    const int ntiles = (int)(((long)n_rows + 31) / 32);
+    const int nwarps = gridDim.x * (kWarpBlock / 32);
+    const int per = (ntiles + nwarps - 1) / nwarps;
+    const int tb = (blockIdx.x * (kWarpBlock / 32) + wib) * per;
+    const int te = min(ntiles, tb + per);
     DotAcc<X> dacc;   // fused <x, y> (per-thread partial)
 
     // lane's row pointers of tile k (loads only; nothing waits on them yet)
-    auto load_ptrs = [&](long k, int &ps, int &pe) {
-        const int row = (int)(k * 32) + lane;
+    auto load_ptrs = [&](int k, int &ps, int &pe) {
+        const int row = min(k, ntiles) * 32 + lane;
         ps = __ldg(pntr + min(row, n_rows));
         pe = __ldg(pntr + min(row + 1, n_rows));
     };
-    // the tile's entry range, and its copy into buffer buf when it fits
-    auto start_tile = [&](long k, int ps, int pe, int buf, int &base, int &end) {
-        const int nr = min(32, n_rows - (int)(k * 32));
-        base = __shfl_sync(0xffffffffu, ps, 0);
-        end = __shfl_sync(0xffffffffu, pe, nr - 1);
-        if (end - base <= kWarpCap) {
-            V *sv = s_vals[wib][buf];
-            int *si = s_idx[wib][buf];
+    // tile k's copy into buffer buf when it fits (one commit per call)
+    auto stage = [&](int k, int ps, int pe, int buf) {
+        const int base = __shfl_sync(0xffffffffu, ps, 0), end = __shfl_sync(0xffffffffu, pe, 31);
+        if (k < te && end - base <= CAP) {
+            V *sv = s_vals + buf * SV;
+            int *si = s_idx + buf * SI;
             const int av = base & ~(EV - 1), ai = base & ~3;
             for (int g = av + lane * EV; g < end; g += 32 * EV) {
                 if (g + EV <= nnz) cp_async16(sv + (g - av), vals + g);
@@ -114,180 +154,106 @@ spmv_warp_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
     };
 
     if (tb < te) {
-        int ps0, pe0, ps1 = 0, pe1 = 0, base0, end0;
-        load_ptrs(tb, ps0, pe0);
-        start_tile(tb, ps0, pe0, 0, base0, end0);
-        if (tb + 1 < te) load_ptrs(tb + 1, ps1, pe1);
-        for (long k = tb; k < te; k++) {
-            const int buf = (int)((k - tb) & 1);
-            int base1 = 0, end1 = 0, ps2 = 0, pe2 = 0;
-            if (k + 1 < te) start_tile(k + 1, ps1, pe1, buf ^ 1, base1, end1);
-            else cp_async_commit();
-            if (k + 2 < te) load_ptrs(k + 2, ps2, pe2);
-            cp_async_wait<1>();   // tile k has landed
+        int ps[ST + 1], pe[ST + 1];   // row pointers of tiles k ... k + ST
+#pragma unroll
+        for (int s = 0; s < ST; s++) load_ptrs(tb + s, ps[s], pe[s]);
+#pragma unroll
+        for (int s = 0; s < ST - 1; s++) stage(tb + s, ps[s], pe[s], s);
+        int buf = 0, fill = ST - 1;
+        for (int k = tb; k < te; k++) {
+            stage(k + ST - 1, ps[ST - 1], pe[ST - 1], fill);
+            load_ptrs(k + ST, ps[ST], pe[ST]);
+            cp_async_wait<ST - 1>();   // tile k has landed
             __syncwarp();
-            const int row = (int)(k * 32) + lane;
-            X acc = X(0);
-            if (row < n_rows) {
-                if (end0 - base0 <= kWarpCap) {
-                    const V *sv = s_vals[wib][buf];
-                    const int *si = s_idx[wib][buf];
-                    const int ov = base0 & ~(EV - 1), oi = base0 & ~3;
-                    for (int j0 = ps0; j0 < pe0; j0 += kGW) {
-                        X xv[kGW], vv[kGW];
+            const int row = k * 32 + lane;
+            const int first = __shfl_sync(0xffffffffu, ps[0], 0), end = __shfl_sync(0xffffffffu, pe[0], 31);
+            const int cnt = pe[0] - ps[0];
+            const int most = __reduce_max_sync(0xffffffffu, cnt);
+            for (int c0 = 0; c0 < (NC == 1 ? 1 : nrhs); c0 += cols) {
+                const int nc = NC == 1 ? 1 : min(cols, nrhs - c0);
+                const X *xc = x + (long)c0 * ldx;
+                X acc[NC];
 #pragma unroll
-                        for (int q = 0; q < kGW; q++)
-                            if (j0 + q < pe0) {
-                                vv[q] = Val<V>::get(sv[j0 + q - ov]);
-                                xv[q] = __ldg(x + si[j0 + q - oi]);
+                for (int m = 0; m < NC; m++) acc[m] = X(0);
+                // the row's entries, GW at a time, from vp / ip (its first entry in the buffer or in memory), in step
+                // across the warp; not for several columns of a direct tile, whose long rows leave few lanes active
+                auto sum = [&](const V *vp, const int *ip, auto staged) {
+                    constexpr bool in_step = decltype(staged)::value || NC == 1;
+                    constexpr int GW = TileShape<X, NC, CAP>::gathers;
+                    const int upto = in_step ? most : cnt;
+                    for (int j0 = 0; j0 < upto; j0 += GW) {
+                        X xv[GW][NC], vv[GW];
+#pragma unroll
+                        for (int q = 0; q < GW; q++)
+                            if (j0 + q < cnt) {
+                                V v;
+                                int col;
+                                if constexpr (decltype(staged)::value) {
+                                    v = vp[j0 + q];
+                                    col = ip[j0 + q];
+                                } else {
+                                    v = __ldg(vp + j0 + q);
+                                    col = __ldg(ip + j0 + q);
+                                }
+                                vv[q] = Val<V>::get(v);
+                                const X *xp = xc + col;
+#pragma unroll
+                                for (int m = 0; m < NC; m++)
+                                    if (m < nc) xv[q][m] = __ldg(xp + (long)m * ldx);
                             }
 #pragma unroll
-                        for (int q = 0; q < kGW; q++)
-                            if (j0 + q < pe0) acc = spmv_acc<EXACT>(acc, vv[q], xv[q]);
-                    }
-                } else {
-                    for (int j0 = ps0; j0 < pe0; j0 += kGW) {
-                        X xv[kGW], vv[kGW];
+                        for (int q = 0; q < GW; q++)
+                            if (!in_step || spmv_uniform(j0 + q < most, X(0))) {
 #pragma unroll
-                        for (int q = 0; q < kGW; q++)
-                            if (j0 + q < pe0) {
-                                vv[q] = Val<V>::get(__ldg(vals + j0 + q));
-                                xv[q] = __ldg(x + __ldg(indx + j0 + q));
+                                for (int m = 0; m < NC; m++)
+                                    if (NC == 1 || !in_step || spmv_uniform(m < nc, X(0)))
+                                        if (j0 + q < cnt) acc[m] = spmv_acc<EXACT>(acc[m], vv[q], xv[q][m]);
                             }
-#pragma unroll
-                        for (int q = 0; q < kGW; q++)
-                            if (j0 + q < pe0) acc = spmv_acc<EXACT>(acc, vv[q], xv[q]);
                     }
+                };
+                if (end - first <= CAP)
+                    sum(s_vals + buf * SV + (ps[0] - (first & ~(EV - 1))), s_idx + buf * SI + (ps[0] - (first & ~3)),
+                        std::true_type());
+                else
+                    sum(vals + ps[0], indx + ps[0], std::false_type());
+                if (row < n_rows) {
+#pragma unroll
+                    for (int m = 0; m < NC; m++)
+                        if (m < nc) {
+                            X *yp = y + (long)(c0 + m) * ldy + row;
+                            const X out = spmv_out<EXACT>(end_mode, alpha, acc[m], beta, yp);
+                            *yp = out;
+                            if (DOT) dacc.add(__ldg(x + row), out);
+                        }
                 }
-                const X out = spmv_out<EXACT>(alpha, acc, beta, y + row);
-                y[row] = out;
-                if (DOT) dacc.add(__ldg(x + row), out);
             }
-            __syncwarp();   // buffer buf is refilled by tile k+2
-            ps0 = ps1;
-            pe0 = pe1;
-            base0 = base1;
-            end0 = end1;
-            ps1 = ps2;
-            pe1 = pe2;
+            __syncwarp();   // the buffer is refilled next
+            fill = buf;
+            buf = buf + 1 == ST ? 0 : buf + 1;
+#pragma unroll
+            for (int s = 0; s < ST; s++) {
+                ps[s] = ps[s + 1];
+                pe[s] = pe[s + 1];
+            }
         }
     }
     cp_async_wait<0>();
     if (DOT) spmv_dot_epilogue<DOT>(dacc.get(), partials, counter, dot_out);
 }
-
-// Y = alpha * A X + beta * Y for nrhs column-major columns (x column c at x + c * ldx): the tiles
-// of spmv_warp_kernel, each staged in shared memory once and summed for kMmCols columns at a time
-// (the matrix is read once, not once per column).  Every column is summed in column order in
-// the mode's rounding, so each column equals the single-column product bit for bit.
-constexpr int kMmCols = 4;   // columns summed per pass over a tile (gathers in flight per lane)
-template <typename V, bool EXACT>
-__global__ void __launch_bounds__(kWarpBlock)
-spmm_warp_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx, const V *__restrict__ vals,
-                 int nrhs, typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x, long ldx,
-                 typename Val<V>::X beta, typename Val<V>::X *__restrict__ y, long ldy) {
-    using X = typename Val<V>::X;
-    constexpr int EV = 16 / (int)sizeof(V);
-    constexpr int SV = kWarpCap + 2 * EV, SI = kWarpCap + 8;
-    __shared__ __align__(16) V s_vals[kWarpBlock / 32][2][SV];
-    __shared__ __align__(16) int s_idx[kWarpBlock / 32][2][SI];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int nnz = __ldg(pntr + n_rows);
-    const long ntiles = ((long)n_rows + 31) / 32;
-    const long nwarps = (long)gridDim.x * (kWarpBlock / 32);
-    const long per = (ntiles + nwarps - 1) / nwarps;
-    const long tb = ((long)blockIdx.x * (kWarpBlock / 32) + wib) * per;
-    const long te = min(ntiles, tb + per);
-    auto load_ptrs = [&](long k, int &ps, int &pe) {
-        const int row = (int)(k * 32) + lane;
-        ps = __ldg(pntr + min(row, n_rows));
-        pe = __ldg(pntr + min(row + 1, n_rows));
-    };
-    auto start_tile = [&](long k, int ps, int pe, int buf, int &base, int &end) {
-        const int nr = min(32, n_rows - (int)(k * 32));
-        base = __shfl_sync(0xffffffffu, ps, 0);
-        end = __shfl_sync(0xffffffffu, pe, nr - 1);
-        if (end - base <= kWarpCap) {
-            V *sv = s_vals[wib][buf];
-            int *si = s_idx[wib][buf];
-            const int av = base & ~(EV - 1), ai = base & ~3;
-            for (int g = av + lane * EV; g < end; g += 32 * EV) {
-                if (g + EV <= nnz) cp_async16(sv + (g - av), vals + g);
-                else
-                    for (int q = 0; q < EV && g + q < end; q++) sv[g - av + q] = vals[g + q];
-            }
-            for (int g = ai + lane * 4; g < end; g += 32 * 4) {
-                if (g + 4 <= nnz) cp_async16(si + (g - ai), indx + g);
-                else
-                    for (int q = 0; q < 4 && g + q < end; q++) si[g - ai + q] = indx[g + q];
-            }
-        }
-        cp_async_commit();
-    };
-    if (tb >= te) return;
-    int ps0, pe0, ps1 = 0, pe1 = 0, base0, end0;
-    load_ptrs(tb, ps0, pe0);
-    start_tile(tb, ps0, pe0, 0, base0, end0);
-    if (tb + 1 < te) load_ptrs(tb + 1, ps1, pe1);
-    for (long k = tb; k < te; k++) {
-        const int buf = (int)((k - tb) & 1);
-        int base1 = 0, end1 = 0, ps2 = 0, pe2 = 0;
-        if (k + 1 < te) start_tile(k + 1, ps1, pe1, buf ^ 1, base1, end1);
-        else cp_async_commit();
-        if (k + 2 < te) load_ptrs(k + 2, ps2, pe2);
-        cp_async_wait<1>();   // tile k has landed
-        __syncwarp();
-        const int row = (int)(k * 32) + lane;
-        if (row < n_rows) {
-            const bool staged = end0 - base0 <= kWarpCap;
-            const V *sv = s_vals[wib][buf];
-            const int *si = s_idx[wib][buf];
-            const int ov = base0 & ~(EV - 1), oi = base0 & ~3;
-            for (int c0 = 0; c0 < nrhs; c0 += kMmCols) {
-                const int nc = min(kMmCols, nrhs - c0);
-                const X *xc = x + (long)c0 * ldx;
-                X acc[kMmCols];
-#pragma unroll
-                for (int q = 0; q < kMmCols; q++) acc[q] = X(0);
-                for (int j = ps0; j < pe0; j++) {
-                    const X v = staged ? Val<V>::get(sv[j - ov]) : Val<V>::get(__ldg(vals + j));
-                    const int col = staged ? si[j - oi] : __ldg(indx + j);
-                    X xv[kMmCols];
-#pragma unroll
-                    for (int q = 0; q < kMmCols; q++)
-                        if (q < nc) xv[q] = __ldg(xc + (long)q * ldx + col);
-#pragma unroll
-                    for (int q = 0; q < kMmCols; q++)
-                        if (q < nc) acc[q] = spmv_acc<EXACT>(acc[q], v, xv[q]);
-                }
-#pragma unroll
-                for (int q = 0; q < kMmCols; q++)
-                    if (q < nc) {
-                        X *yp = y + (long)(c0 + q) * ldy + row;
-                        *yp = spmv_out<EXACT>(alpha, acc[q], beta, yp);
-                    }
-            }
-        }
-        __syncwarp();   // buffer buf is refilled by tile k+2
-        ps0 = ps1;
-        pe0 = pe1;
-        base0 = base1;
-        end0 = end1;
-        ps1 = ps2;
-        pe1 = pe2;
-    }
-    cp_async_wait<0>();
+template <typename V, int CAP>
+constexpr size_t spmv_smem_bytes() {
+    return (size_t)(kWarpBlock / 32) * kStages * ((CAP + 2 * (16 / sizeof(V))) * sizeof(V) + (CAP + 8) * sizeof(int));
 }
 
 // Arrays that are not 16-byte aligned cannot be staged with cp.async: one row per thread,
 // grid-stride, the row's vals/indx and x gathers (8 at a time) straight from global memory
-// through L1.  Same arithmetic as spmv_warp_kernel.
+// through L1.  Same arithmetic as spmv_tile_kernel.
 template <typename V, int DOT, bool EXACT>
 __global__ void __launch_bounds__(256)
 spmv_direct_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx,
-                   const V *__restrict__ vals, typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x,
-                   typename Val<V>::X beta, typename Val<V>::X *__restrict__ y, double *partials, unsigned *counter,
-                   double *dot_out, const int *skip) {
+                   const V *__restrict__ vals, int end_mode, typename Val<V>::X alpha,
+                   const typename Val<V>::X *__restrict__ x, typename Val<V>::X beta, typename Val<V>::X *__restrict__ y,
+                   double *partials, unsigned *counter, double *dot_out, const int *skip) {
     using X = typename Val<V>::X;
     if (skip && *skip) return;
     DotAcc<X> dacc;   // fused <x, y> (per-thread partial)
@@ -306,7 +272,7 @@ spmv_direct_kernel(int n_rows, const int *__restrict__ pntr, const int *__restri
             for (int k = 0; k < 8; k++)
                 if (j0 + k < pe) acc = spmv_acc<EXACT>(acc, vv[k], xv[k]);
         }
-        const X out = spmv_out<EXACT>(alpha, acc, beta, y + r);
+        const X out = spmv_out<EXACT>(end_mode, alpha, acc, beta, y + r);
         y[r] = out;
         if (DOT) dacc.add(__ldg(x + r), out);
     }
@@ -337,24 +303,56 @@ __global__ void scale_or_zero_kernel(long n, X beta, X *y) {
 // original row, which is the accumulation order of sparse_gemv_array<'T'> (utils:113-118).
 // FUSE_DOT additionally reduces <x', y> with x' = the vector y is paired with (dot_x, indexed by
 // column), for the CG on the transposed operator.
+// Bound by the FP64 unit (separately rounded operations, the oracle's) and the latency of the chain
+// pointers -> map / rows -> values / x: the scaling by alpha, and the comparisons with alpha and beta, are
+// left out where end_mode says that they do nothing; three entries' loads are in flight per lane, in 32 registers, so
+// that an SM holds 64 warps (512^2 5-point FP64: 12.4 -> 10.3 us; 97x96^2 7-point FP32: 17.0 -> 14.2; five or eight
+// entries in flight in fewer warps: 10.3 to 14.4 and 14.4 to 16.4).  The loop is warp-uniform (spmv_uniform).
 template <typename V, bool FUSE_DOT>
-__global__ void spmv_t_cached_kernel(int n_cols, const int *__restrict__ pntrT, const int *__restrict__ rowT,
-                                     const int *__restrict__ mapT, const V *__restrict__ vals,
-                                     typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x,
-                                     typename Val<V>::X beta, typename Val<V>::X *__restrict__ y,
-                                     const typename Val<V>::X *__restrict__ dot_x, double *partials,
-                                     unsigned *counter, double *dot_out, const int *skip) {
+__global__ void __launch_bounds__(256, 8)
+spmv_t_cached_kernel(int n_cols, const int *__restrict__ pntrT, const int *__restrict__ rowT,
+                     const int *__restrict__ mapT, const V *__restrict__ vals, int end_mode,
+                     typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x,
+                     typename Val<V>::X beta, typename Val<V>::X *__restrict__ y,
+                     const typename Val<V>::X *__restrict__ dot_x, double *partials,
+                     unsigned *counter, double *dot_out, const int *skip) {
     using X = typename Val<V>::X;
+    constexpr int G = 3;
     if (skip && *skip) return;
     DotAcc<X> dacc;   // fused <x, y> (per-thread partial)
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cols; c += gridDim.x * blockDim.x) {
-        X acc = (beta == X(0)) ? X(0) : mul_rn(beta, y[c]);
-        for (int p = __ldg(pntrT + c); p < __ldg(pntrT + c + 1); p++) {
-            int i = __ldg(rowT + p);
-            acc = add_rn(acc, mul_rn(mul_rn(alpha, __ldg(x + i)), Val<V>::get(__ldg(vals + __ldg(mapT + p)))));
+    for (int cb = blockIdx.x * blockDim.x + (threadIdx.x & ~31); cb < n_cols; cb += gridDim.x * blockDim.x) {
+        const int c = cb + (threadIdx.x & 31);
+        const int ps = __ldg(pntrT + min(c, n_cols)), cnt = __ldg(pntrT + min(c + 1, n_cols)) - ps;
+        const int most = __reduce_max_sync(0xffffffffu, cnt);
+        X acc = X(0);
+        if (end_mode == END_FULL && c < n_cols) acc = mul_rn(beta, y[c]);
+        for (int j0 = 0; j0 < most; j0 += G) {
+            int at[G];
+            X xv[G], vv[G];
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (j0 + q < cnt) {
+                    at[q] = __ldg(mapT + ps + j0 + q);
+                    xv[q] = __ldg(x + __ldg(rowT + ps + j0 + q));
+                }
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (j0 + q < cnt) vv[q] = Val<V>::get(__ldg(vals + at[q]));
+            if (end_mode != END_PLAIN) {
+#pragma unroll
+                for (int q = 0; q < G; q++)
+                    if (spmv_uniform(j0 + q < most, X(0)))
+                        if (j0 + q < cnt) xv[q] = mul_rn(alpha, xv[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < G; q++)
+                if (spmv_uniform(j0 + q < most, X(0)))
+                    if (j0 + q < cnt) acc = add_rn(acc, mul_rn(xv[q], vv[q]));
         }
-        y[c] = acc;
-        if (FUSE_DOT) dacc.add(dot_x[c], acc);
+        if (c < n_cols) {
+            y[c] = acc;
+            if (FUSE_DOT) dacc.add(dot_x[c], acc);
+        }
     }
     if (FUSE_DOT) {
         double dsum[1] = {dacc.get()};
@@ -515,94 +513,118 @@ void Transpose::release() {
     pntr = row = map = nullptr;
 }
 
+// Tiles of rows of 7 entries fit kCapShort; where rows average more than 7.5, kCapLong keeps those up to 12
+// staged.  (Tiles cut into chunks, or longer buffers, were slower than the direct reads for longer rows: the lanes
+// whose row is not in the chunk idle.)
+static bool spmv_long_rows(int n_rows, long nnz) { return 2 * nnz > 15L * n_rows; }
+
+// The staged kernel's launch: a persistent grid of the resident CTAs of every SM (occupancy queried once per
+// kernel and device).
+template <typename V, int NC, int CAP, int DOT, bool EXACT>
+static int spmv_tile_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals, int nrhs, int cols,
+                            typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
+                            typename Val<V>::X *y, long ldy, double *partials, unsigned *counter, double *dot_out,
+                            const int *skip, int *nparts) {
+    constexpr size_t smem = spmv_smem_bytes<V, CAP>();
+    constexpr int most = TileShape<typename Val<V>::X, NC, CAP>::ctas;
+    auto kernel = spmv_tile_kernel<V, NC, CAP, DOT, EXACT>;
+    static std::atomic<int> occ_dev[64];
+    if (c->device < 0 || c->device >= 64) return fail(HGB_ERR_UNSUPPORTED, "spmv: device ordinal %d", c->device);
+    int occ = occ_dev[c->device].load();
+    if (!occ) {
+        HGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        HGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      std::min(100, (int)(most * (smem + 1024) * 100 / (228 * 1024)) + 1)));
+        HGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kWarpBlock, smem));
+        occ = std::min(std::max(occ, 1), most);
+        occ_dev[c->device] = occ;
+    }
+    const long tiles = ((long)n_rows + 31) / 32;
+    const int g = (int)std::max<long>(1, std::min<long>((tiles + 7) / 8, std::min(c->num_sms * occ, kMaxReduceBlocks)));
+    if (nparts) *nparts = g;
+    kernel<<<g, kWarpBlock, smem, c->stream>>>(n_rows, pntr, indx, vals, nrhs, cols, spmv_end(alpha, beta), alpha, x, ldx, beta,
+                                               y, ldy, partials, counter, dot_out, skip);
+    return launch_check("spmv_tile_kernel");
+}
+
 template <typename V, int DOT, bool EXACT>
-static int spmv_n_launch_mode(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals,
+static int spmv_n_launch_mode(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
                               typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                               typename Val<V>::X *y, double *dot_out, const int *skip, int *nparts) {
     // DOT 2: the per-CTA parts of <x, y> stay in the context's parts slots (their count to *nparts)
     double *partials = DOT == 2 ? c->partials + kSpmvPartsOffset : (DOT == 1 ? c->partials : nullptr);
     unsigned *counter = DOT == 1 ? c->counter : nullptr;
-    if (aligned16(vals) && aligned16(indx)) {
-        // persistent grid: the resident CTAs of every SM (occupancy queried once per kernel)
-        static int occ = 0;
-        if (!occ) {
-            HGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, spmv_warp_kernel<V, DOT, EXACT>, kWarpBlock, 0));
-            occ = std::max(occ, 1);
-        }
-        const long tiles = ((long)n_rows + 31) / 32;
-        const int g = (int)std::max<long>(1, std::min<long>((tiles + 7) / 8, std::min(c->num_sms * occ, kMaxReduceBlocks)));
-        if (nparts) *nparts = g;
-        spmv_warp_kernel<V, DOT, EXACT><<<g, kWarpBlock, 0, c->stream>>>(n_rows, pntr, indx, vals, alpha, x, beta, y,
-                                                                            partials, counter, dot_out, skip);
-        return launch_check("spmv_warp_kernel");
-    }
+    if (aligned16(vals) && aligned16(indx))
+        return spmv_long_rows(n_rows, nnz)
+                   ? spmv_tile_launch<V, 1, kCapLong, DOT, EXACT>(c, n_rows, pntr, indx, vals, 1, 1, alpha, x, 0, beta, y, 0, partials,
+                                                             counter, dot_out, skip, nparts)
+                   : spmv_tile_launch<V, 1, kCapShort, DOT, EXACT>(c, n_rows, pntr, indx, vals, 1, 1, alpha, x, 0, beta, y, 0, partials,
+                                                             counter, dot_out, skip, nparts);
     const int g = std::min((n_rows + 255) / 256, std::min(c->num_sms * 8, kMaxReduceBlocks));
     if (nparts) *nparts = g;
-    spmv_direct_kernel<V, DOT, EXACT><<<g, 256, 0, c->stream>>>(n_rows, pntr, indx, vals, alpha, x, beta, y, partials,
-                                                                   counter, dot_out, skip);
+    spmv_direct_kernel<V, DOT, EXACT><<<g, 256, 0, c->stream>>>(n_rows, pntr, indx, vals, spmv_end(alpha, beta), alpha, x, beta, y,
+                                                                   partials, counter, dot_out, skip);
     return launch_check("spmv_direct_kernel");
 }
 
 template <typename V>
-int spmv_n_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals,
+int spmv_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                   typename Val<V>::X *y, double *dot_out, const int *skip, int *nparts) {
     if (nparts) *nparts = 0;
     if (n_rows <= 0) return HGB_OK;
     const bool exact = c->spmv_mode == HGB_SPMV_EXACT;
     if (nparts)
-        return exact ? spmv_n_launch_mode<V, 2, true>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts)
-                     : spmv_n_launch_mode<V, 2, false>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts);
+        return exact ? spmv_n_launch_mode<V, 2, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts)
+                     : spmv_n_launch_mode<V, 2, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts);
     if (dot_out)
-        return exact ? spmv_n_launch_mode<V, 1, true>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr)
-                     : spmv_n_launch_mode<V, 1, false>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr);
-    return exact ? spmv_n_launch_mode<V, 0, true>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr)
-                 : spmv_n_launch_mode<V, 0, false>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr);
+        return exact ? spmv_n_launch_mode<V, 1, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr)
+                     : spmv_n_launch_mode<V, 1, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr);
+    return exact ? spmv_n_launch_mode<V, 0, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr)
+                 : spmv_n_launch_mode<V, 0, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr);
 }
 
 template <typename V>
-int spmm_n_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals, int nrhs,
+int spmm_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals, int nrhs,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
                   typename Val<V>::X *y, long ldy) {
     if (n_rows <= 0 || nrhs <= 0) return HGB_OK;
     if (!aligned16(vals) || !aligned16(indx)) {   // no staging: the single-column products
         for (int k = 0; k < nrhs; k++)
-            HGB_TRY(spmv_n_launch<V>(c, n_rows, pntr, indx, vals, alpha, x + (long)k * ldx, beta, y + (long)k * ldy,
+            HGB_TRY(spmv_n_launch<V>(c, n_rows, nnz, pntr, indx, vals, alpha, x + (long)k * ldx, beta, y + (long)k * ldy,
                                      nullptr));
         return HGB_OK;
     }
     const bool exact = c->spmv_mode == HGB_SPMV_EXACT;
-    static int occ_dev[2][64] = {};
-    if (c->device < 0 || c->device >= 64) return fail(HGB_ERR_UNSUPPORTED, "spmm: device ordinal %d", c->device);
-    int &occ = occ_dev[exact ? 1 : 0][c->device];
-    if (!occ) {
-        HGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &occ, exact ? (const void *)spmm_warp_kernel<V, true> : (const void *)spmm_warp_kernel<V, false>,
-            kWarpBlock, 0));
-        occ = std::max(occ, 1);
+    const int passes = (nrhs + kMmCols - 1) / kMmCols, cols = (nrhs + passes - 1) / passes;   // columns split evenly
+#define HGB_SPMM2(NC, CAP, EXACT)                                                                                   \
+    spmv_tile_launch<V, NC, CAP, 0, EXACT>(c, n_rows, pntr, indx, vals, nrhs, cols, alpha, x, ldx, beta, y, ldy, nullptr, \
+                                           nullptr, nullptr, nullptr, nullptr)
+#define HGB_SPMM(NC)                                                                               \
+    (spmv_long_rows(n_rows, nnz) ? (exact ? HGB_SPMM2(NC, kCapLong, true) : HGB_SPMM2(NC, kCapLong, false)) \
+                                 : (exact ? HGB_SPMM2(NC, kCapShort, true) : HGB_SPMM2(NC, kCapShort, false)))
+    switch (cols) {
+        case 1: return HGB_SPMM(1);
+        case 2: return HGB_SPMM(2);
+        case 3: return HGB_SPMM(3);
+        case 4: return HGB_SPMM(4);
+        default: return HGB_SPMM(kMmCols);
     }
-    const long tiles = ((long)n_rows + 31) / 32;
-    const int g = (int)std::max<long>(1, std::min<long>((tiles + 7) / 8, (long)c->num_sms * occ));
-    if (exact)
-        spmm_warp_kernel<V, true><<<g, kWarpBlock, 0, c->stream>>>(n_rows, pntr, indx, vals, nrhs, alpha, x, ldx,
-                                                                    beta, y, ldy);
-    else
-        spmm_warp_kernel<V, false><<<g, kWarpBlock, 0, c->stream>>>(n_rows, pntr, indx, vals, nrhs, alpha, x, ldx,
-                                                                     beta, y, ldy);
-    return launch_check("spmm_warp_kernel");
+#undef HGB_SPMM2
+#undef HGB_SPMM
 }
 
-template int spmv_n_launch<double>(hgb_ctx *, int, const int *, const int *, const double *, double,
+template int spmv_n_launch<double>(hgb_ctx *, int, long, const int *, const int *, const double *, double,
                                    const double *, double, double *, double *, const int *, int *);
-template int spmv_n_launch<float>(hgb_ctx *, int, const int *, const int *, const float *, float,
+template int spmv_n_launch<float>(hgb_ctx *, int, long, const int *, const int *, const float *, float,
                                   const float *, float, float *, double *, const int *, int *);
-template int spmv_n_launch<uint16_t>(hgb_ctx *, int, const int *, const int *, const uint16_t *, float,
+template int spmv_n_launch<uint16_t>(hgb_ctx *, int, long, const int *, const int *, const uint16_t *, float,
                                      const float *, float, float *, double *, const int *, int *);
-template int spmm_n_launch<double>(hgb_ctx *, int, const int *, const int *, const double *, int, double,
+template int spmm_n_launch<double>(hgb_ctx *, int, long, const int *, const int *, const double *, int, double,
                                    const double *, long, double, double *, long);
-template int spmm_n_launch<float>(hgb_ctx *, int, const int *, const int *, const float *, int, float,
+template int spmm_n_launch<float>(hgb_ctx *, int, long, const int *, const int *, const float *, int, float,
                                   const float *, long, float, float *, long);
-template int spmm_n_launch<uint16_t>(hgb_ctx *, int, const int *, const int *, const uint16_t *, int, float,
+template int spmm_n_launch<uint16_t>(hgb_ctx *, int, long, const int *, const int *, const uint16_t *, int, float,
                                      const float *, long, float, float *, long);
 
 template <typename V>
@@ -613,7 +635,7 @@ int spmv_t_launch(hgb_ctx *c, int n_rows, int n_cols, const int *pntr, const int
     if (n_cols <= 0) return HGB_OK;
     int gc = std::max(1, std::min((n_cols + 255) / 256, c->num_sms * 8));
     if (T) {
-        spmv_t_cached_kernel<V, false><<<gc, 256, 0, c->stream>>>(n_cols, T->pntr, T->row, T->map, vals, alpha, x,
+        spmv_t_cached_kernel<V, false><<<gc, 256, 0, c->stream>>>(n_cols, T->pntr, T->row, T->map, vals, spmv_end(alpha, beta), alpha, x,
                                                                  beta, y, nullptr, nullptr, nullptr, nullptr, nullptr);
         return launch_check("spmv_t_cached_kernel");
     }
@@ -672,10 +694,10 @@ int spmv_t_fused_launch(hgb_csr *A, typename Val<V>::X alpha, const typename Val
     int gc = std::max(1, std::min((n + 255) / 256, std::min(c->num_sms * 8, kMaxReduceBlocks)));
     if (dot_out)
         spmv_t_cached_kernel<V, true><<<gc, 256, 0, c->stream>>>(n, A->T.pntr, A->T.row, A->T.map, (const V *)A->vals,
-                                                                alpha, x, beta, y, dot_x, c->partials, c->counter, dot_out, skip);
+                                                                spmv_end(alpha, beta), alpha, x, beta, y, dot_x, c->partials, c->counter, dot_out, skip);
     else
         spmv_t_cached_kernel<V, false><<<gc, 256, 0, c->stream>>>(n, A->T.pntr, A->T.row, A->T.map, (const V *)A->vals,
-                                                                 alpha, x, beta, y, nullptr, nullptr, nullptr, nullptr, skip);
+                                                                 spmv_end(alpha, beta), alpha, x, beta, y, nullptr, nullptr, nullptr, nullptr, skip);
     return launch_check("spmv_t_cached_kernel");
 }
 template int spmv_t_fused_launch<double>(hgb_csr *, double, const double *, double, double *, const double *, double *, const int *);
@@ -711,7 +733,7 @@ int hgb_spmv_f64(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, const 
                  const double *vals, double alpha, const double *x, double beta, double *y) {
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     DeviceGuard g(c->device);
-    if (trans == 'N' || trans == 'n') return spmv_n_launch<double>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    if (trans == 'N' || trans == 'n') return spmv_n_launch<double>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
     return spmv_t_launch<double>(c, n_rows, n_cols, pntr, indx, vals, alpha, x, beta, y, nullptr);
 }
 
@@ -719,7 +741,7 @@ int hgb_spmv_f32(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, const 
                  const float *vals, float alpha, const float *x, float beta, float *y) {
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     DeviceGuard g(c->device);
-    if (trans == 'N' || trans == 'n') return spmv_n_launch<float>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    if (trans == 'N' || trans == 'n') return spmv_n_launch<float>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
     return spmv_t_launch<float>(c, n_rows, n_cols, pntr, indx, vals, alpha, x, beta, y, nullptr);
 }
 
@@ -728,7 +750,7 @@ int hgb_spmv_bf16f32(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, co
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     if (trans != 'N' && trans != 'n') return fail(HGB_ERR_UNSUPPORTED, "spmv_bf16f32: only trans 'N'");
     DeviceGuard g(c->device);
-    return spmv_n_launch<uint16_t>(c, n_rows, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    return spmv_n_launch<uint16_t>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
 }
 
 int hgb_csr_create(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx,
@@ -765,9 +787,9 @@ int hgb_csr_gemv(hgb_csr *A, char trans, double alpha, const void *x, double bet
     }
     if (nt) {
         switch (A->dtype) {
-            case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->pntr, A->indx, (const double *)A->vals, alpha, (const double *)x, beta, (double *)y, nullptr, nullptr);
-            case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->pntr, A->indx, (const float *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
-            default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->pntr, A->indx, (const uint16_t *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
+            case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const double *)A->vals, alpha, (const double *)x, beta, (double *)y, nullptr, nullptr);
+            case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const float *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
+            default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const uint16_t *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
         }
     }
     if (A->dtype == HGB_BF16) return fail(HGB_ERR_UNSUPPORTED, "csr_gemv: transpose of a bf16 matrix");
@@ -821,9 +843,9 @@ int hgb_csr_gemv_dot(hgb_csr *A, const void *x, void *y, double *dot_out) {
     hgb_ctx *c = A->ctx;
     DeviceGuard g(c->device);
     switch (A->dtype) {
-        case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->pntr, A->indx, (const double *)A->vals, 1.0, (const double *)x, 0.0, (double *)y, dot_out, nullptr);
-        case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->pntr, A->indx, (const float *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
-        default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->pntr, A->indx, (const uint16_t *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
+        case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const double *)A->vals, 1.0, (const double *)x, 0.0, (double *)y, dot_out, nullptr);
+        case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const float *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
+        default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const uint16_t *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
     }
 }
 
