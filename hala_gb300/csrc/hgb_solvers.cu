@@ -255,108 +255,226 @@ static int cg_iteration(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, CgWork<X> &w, X *x, 
 // Unpreconditioned CG on a system whose matrix and vectors stay in L2 (the 256^2 Poisson class):
 // there the graph-replayed iteration is bound by its launches and their reductions' tails
 // (about 27 us per iteration for six launches), not by bytes.  One cooperative launch runs up to
-// kCgpChunk iterations with two grid barriers each: after the x / r update (||r||^2 complete, and
-// r in memory for the next product) and after the direction update (<p, Ap> complete).  The
-// product is taken of r, s = A r, and the new direction's product follows by the recurrence
-// Ap = beta Ap + s beside p = beta p + r, so no barrier waits for the new p (a launch starts
-// with Ap = A p).  Every CTA keeps its rows for the whole launch, writes one partial per reduction
-// and, after the barrier, sums all CTAs' partials in the same order, so every CTA takes the same
-// decision with the same bits and no CTA waits on a single finisher.  The updates are the graph
-// path's (DotAcc partials per thread, separately rounded, the product in the context's SpMV
-// mode), with z = r, so <r, z> is ||r||^2; the Ap recurrence rounds differently from A p, so the
-// iteration count can differ from the graph path's by a few.  Barriers are bounded: a barrier
-// that runs out of polls sets DEV_ERR_TIMEOUT and every CTA returns.
+// kCgpChunk iterations.  Every CTA keeps its rows for the whole launch.  What bounds an iteration is the latency of
+// its exchanges between CTAs and of FP64 instructions (each holds an SM quarter's unit for 62 cycles), so
+// it has one reduction (Chronopoulos and Gear's form of the method):
+//   x += a p, r -= a q                       (q = A p)
+//   s = A r, with the neighbours' r taken as they arrive (below), and <r, r> and <r, s> in one reduction
+//   b = <r, r> / <r, r>_old,  <p, A p> = <r, s> - b <r, r> / a,  a = <r, r> / <p, A p>
+//   p = r + b p, q = s + b q
+// FP32 vectors take <p, q> by a second reduction instead: the difference loses the condition number's share of
+// the digits, which FP64 has to spare and FP32 has not.  A launch starts with q = A p and <p, q> itself.  Every CTA sums all CTAs' parts in the same order, so
+// every CTA takes the same decision with the same bits.  Rounding differs from the graph path's, so the iteration
+// count can differ from it by a few.  Every wait is bounded: one that runs out of polls sets DEV_ERR_TIMEOUT and
+// every CTA returns.
+// Per iteration, before (two reductions by a counter that every CTA polls) and now: 24x24 7.5 -> 4.1 us, 256^2
+// 9.5 -> 5.9, 300^2 15.5 -> 7.3, 500^2 21.5 -> 16.1; FP32 256^2 8.3 -> 8.3.  Of the 12,000 cycles at 256^2 the mail
+// takes 2100, the neighbours' r 1300 to 2300, FP64 instructions of the rows 3100, and the sums with one
+// division 5000.
 constexpr int kCgpThreads = 256;
-constexpr int kCgpChunk = 4096;                 // iterations per launch (the barrier counter stays small)
+constexpr int kCgpChunk = 4096;                 // iterations per launch
 constexpr long kCgpMaxRows = 1L << 20;          // larger systems take the graph path
 constexpr size_t kCgpMaxBytes = 48u << 20;      // matrix + vectors resident in L2 (129 MB)
+constexpr int kCgpCluster = 8;                  // CTAs of a cluster at most (8, 4 or 2)
+constexpr int kCgpLead = 4;                     // the warp that posts and polls
+constexpr int kCgpMail = 4;                     // mail entries per lane: at most 64 clusters
 
 // acc += v * x: separately rounded (the exact SpMV mode) or one fused multiply-add
 template <bool EXACT, typename X>
 __device__ __forceinline__ X cgp_acc(X acc, X v, X x) {
     return EXACT ? add_rn(acc, mul_rn(v, x)) : fma(v, x, acc);
 }
+__device__ __forceinline__ void cgp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cgp_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// A value and the number of its step, complete when the number is right: 64-bit words are written whole, so a
+// double goes as two words of half the value and the number each, whatever the order in which they arrive,
+// and value and arrival come with one load.
+struct CgpWord {
+    unsigned long long x, y;
+};
+__device__ __forceinline__ CgpWord cgp_tag(double v, unsigned number) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v), n = (unsigned long long)number << 32;
+    return {n | (bits & 0xffffffffu), n | (bits >> 32)};
+}
+__device__ __forceinline__ bool cgp_whole(const CgpWord &w, unsigned number, double &v) {
+    v = __longlong_as_double((long long)(w.y << 32 | (w.x & 0xffffffffu)));
+    return (unsigned)(w.x >> 32) == number && (unsigned)(w.y >> 32) == number;
+}
+__device__ __forceinline__ void cgp_store(CgpWord *p, const CgpWord &w) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(w.x), "l"(w.y) : "memory");
+}
+__device__ __forceinline__ CgpWord cgp_load(const CgpWord *p) {
+    CgpWord w;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "l"(p) : "memory");
+    return w;
+}
+// the tagged residual: 16 bytes an FP64 entry, 8 an FP32 one
+template <typename X> struct CgpR;
+template <> struct CgpR<double> {
+    using T = CgpWord;
+    static __device__ __forceinline__ void put(T *p, double v, unsigned number) { cgp_store(p, cgp_tag(v, number)); }
+    static __device__ __forceinline__ bool get(const T *p, unsigned number, double &v) { return cgp_whole(cgp_load(p), number, v); }
+};
+template <> struct CgpR<float> {
+    using T = unsigned long long;
+    static __device__ __forceinline__ void put(T *p, float v, unsigned number) {
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)number << 32 | __float_as_uint(v)) : "memory");
+    }
+    static __device__ __forceinline__ bool get(const T *p, unsigned number, float &v) {
+        T w;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+        v = __uint_as_float((unsigned)w);
+        return (unsigned)(w >> 32) == number;
+    }
+};
+// false when the wait is over its bound, or another CTA's was
+__device__ __forceinline__ bool cgp_wait_on(int &spins, const int *err) {
+    if (++spins > kSpinLimit) return false;
+    return (spins & 1023) != 0 || !(*(const volatile int *)err & DEV_ERR_TIMEOUT);
+}
+
+// A warp-uniform choice that stays a branch: the assembler turns short conditional blocks into predicated
+// instructions, and a predicated-off FP64 instruction holds the unit like any other.
+__device__ __forceinline__ int cgp_opaque(int v) {
+    asm volatile("" : "+r"(v));
     return v;
 }
+#define CGP_UNIFORM_IF(cond) _Pragma("unroll 1") for (int z_ = cgp_opaque((cond) ? 1 : 0); z_ > 0; z_ = cgp_opaque(z_ - 1))
 
-// One reduction of the persistent CG: the CTA's partial of v (warp sums, then warp 0), the
-// arrival of every CTA (a grid barrier, bounded), then the sum of all G partials in one fixed
-// order (lane b takes partials b, b + 32, ..., then the warp's butterfly), the same bits in every
-// CTA.  Two CTA barriers: the first orders every thread's earlier global writes before warp 0's
-// release, the second publishes the sum.  False when the wait ran out (DEV_ERR_TIMEOUT set).
-__device__ __forceinline__ bool cgp_reduce(double v, double *part, unsigned *count, unsigned target, int *err,
-                                           double &sum) {
-    __shared__ double wsh[32], res;
-    __shared__ int ok;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    v = warp_sum(v);
-    if (lane == 0) wsh[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        const double t = warp_sum(lane < (int)(blockDim.x >> 5) ? wsh[lane] : 0.0);
-        if (lane == 0) {
-            part[blockIdx.x] = t;
-            // release at GPU scope, cumulative over the CTA's writes that the bar.sync ordered before it
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-        }
-        // every lane polls (one coalesced load), so each lane's own acquire orders its loads below
-        int spins = 0, good = 1;
-        while (!__all_sync(0xFFFFFFFFu, ld_acquire_u32(count) >= target)) {
-            if (++spins > kSpinLimit || ((spins & 1023) == 0 && (*(volatile int *)err & DEV_ERR_TIMEOUT))) {
-                good = 0;
-                break;
-            }
-        }
-        good = __all_sync(0xFFFFFFFFu, good);
-        double acc = 0.0;
-        if (good)
-            for (int b = lane; b < (int)gridDim.x; b += 32) acc += __ldcg(part + b);
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            if (!good) atomicOr(err, DEV_ERR_TIMEOUT);
-            res = acc;
-            ok = good;
-        }
+// A reduction of two sums: the CTAs of a cluster exchange theirs through distributed shared memory, then the CTAs of
+// equal rank exchange the clusters' through mailboxes in memory (every CTA has its own, one entry per cluster).
+// 256^2, 128 CTAs: 2100 cycles for the mail, where 128 CTAs polling one set of entries waited 6500 and each its own
+// mailbox of 128 entries 5000.  Two sets of entries take turns: a CTA posts to a set again only after every CTA
+// has posted to the other one, which each does after reading this one.
+// The sums are shaped to have few FP64 instructions in a row: the upper four warps' values are folded into the
+// lower four (one per quarter), whose lanes then add one of the two sums each, the first in lanes 0 to 15, the
+// second in 16 to 31, here and in the steps after it; the lead warp adds the warps' sums, posts, polls, and adds
+// the rest in one order, the same bits in every CTA.
+struct CgpShared {
+    CgpWord peer[2][kCgpCluster][2];
+    double fold[2][kCgpThreads / 2], warp[8], sum, alpha, beta;
+    int ok;
+};
+__device__ __forceinline__ double cgp_add_xor(double v, int o) { return v + __shfl_xor_sync(0xffffffffu, v, o); }
+// All threads call it.  ORDER: what every CTA wrote before is in memory for all after the caller's next barrier.
+// meanwhile(): the lead warp's work between posting and polling.  The lead warp gets both sums;
+// false when a wait ran out.
+template <bool ORDER, typename F>
+__device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned number, CgpWord *mail, int *err, CgpShared &sh,
+                                             F meanwhile, double (&sum)[2]) {
+    const int tid = threadIdx.x, wid = tid >> 5, set = number & 1;
+    const unsigned lane = tid & 31, half = lane >> 4, at = lane & 15;
+    if (tid >= kCgpThreads / 2) {
+        sh.fold[0][tid - kCgpThreads / 2] = v0;
+        sh.fold[1][tid - kCgpThreads / 2] = v1;
     }
     __syncthreads();
-    sum = res;
-    return ok != 0;
+    if (tid < kCgpThreads / 2) {
+        v0 += sh.fold[0][tid];
+        v1 += sh.fold[1][tid];
+        const double other = __shfl_xor_sync(0xffffffffu, half ? v0 : v1, 16);
+        double v = (half ? v1 : v0) + other;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v = cgp_add_xor(v, o);
+        if (at == 0) sh.warp[half * 4 + wid] = v;
+    } else if (ORDER && wid == kCgpLead) {
+        cgp_fence();   // the CTA's writes, ordered before this by the barrier, before the posts below
+    }
+    __syncthreads();
+    if (wid != kCgpLead) return true;
+    unsigned rank, size, clusters;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(clusters));
+    double t = sh.warp[half * 4 + (lane & 3)];
+    t = cgp_add_xor(cgp_add_xor(t, 1), 2);
+    if (at < size) {
+        unsigned to;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"((unsigned)__cvta_generic_to_shared(&sh.peer[set][rank][half])), "r"(at));
+        const CgpWord w = cgp_tag(t, number);
+        asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(to), "l"(w.x), "l"(w.y) : "memory");
+    }
+    const unsigned from = (unsigned)__cvta_generic_to_shared(&sh.peer[set][at & (size - 1)][half]);
+    for (int spins = 0;;) {
+        CgpWord w;
+        asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "r"(from) : "memory");
+        if (__all_sync(0xffffffffu, cgp_whole(w, number, t))) break;
+        if (__any_sync(0xffffffffu, !cgp_wait_on(spins, err))) return false;
+    }
+    for (unsigned o = 1; o < size; o *= 2) t = cgp_add_xor(t, o);
+    if (ORDER) cgp_fence();   // what the peers ordered before their posts, before this CTA's
+    if (clusters > 1) {
+        mail += (size_t)set * gridDim.x * clusters * 2;
+        for (unsigned k = at; k < clusters; k += 16)
+            cgp_store(mail + ((size_t)(k * size + rank) * clusters + blockIdx.x / size) * 2 + half, cgp_tag(t, number));
+    }
+    meanwhile();
+    if (clusters > 1) {
+        mail += (size_t)blockIdx.x * clusters * 2 + half;
+        double part[kCgpMail];
+        for (int spins = 0;;) {
+            bool here = true;
+#pragma unroll
+            for (int q = 0; q < kCgpMail; q++) {
+                CgpWord w = {(unsigned long long)number << 32, (unsigned long long)number << 32};   // whole, and zero
+                if (16 * q + at < clusters) w = cgp_load(mail + 2 * (16 * q + at));
+                here = cgp_whole(w, number, part[q]) && here;
+            }
+            if (__all_sync(0xffffffffu, here)) break;
+            if (__any_sync(0xffffffffu, !cgp_wait_on(spins, err))) return false;
+        }
+        if (ORDER) cgp_fence();
+        t = part[0];
+        CGP_UNIFORM_IF(clusters > 16) t += part[1];
+        CGP_UNIFORM_IF(clusters > 32) t += part[2] + part[3];
+        for (unsigned o = 1; o < clusters && o < 16; o *= 2) t = cgp_add_xor(t, o);
+    }
+    sum[0] = __shfl_sync(0xffffffffu, t, 0);
+    sum[1] = __shfl_sync(0xffffffffu, t, 16);
+    return true;
 }
-
-// RPT > 0: thread t owns rows t, t + stride, ... (RPT of them: 1, 2 or 4) for the whole launch and keeps their
-// x, r, p and (rows of at most kCgpMaxE entries) their matrix entries in registers: an iteration
-// then reads only the neighbours' p from L2.  RPT = 0: the rows are walked with grid-stride loops
-// and every vector lives in memory (systems too large for one register-resident row set).
+// RPT > 0: a CTA owns RPT * 256 consecutive rows (RPT: 1, 2 or 4 per thread) for the whole launch and keeps their
+// x, r, p, q and (rows of at most kCgpMaxE entries) their matrix entries in registers; r goes to shared memory for the
+// CTA's own rows and to memory tagged with the iteration for the others', and a row's sum waits for its neighbours'
+// entries alone.  RPT = 0: the rows are walked with grid-stride loops and every vector lives in memory (systems too
+// large for one register-resident row set; rt is s there); a reduction orders the writes of r before the products.
 constexpr int kCgpMaxE = 8;
 
 template <typename V, typename X, bool EXACT, int RPT>
-__global__ void __launch_bounds__(kCgpThreads)
+__global__ void __launch_bounds__(kCgpThreads, RPT == 0 ? 4 : 1)
 cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict__ indx, const V *__restrict__ vals,
-                     X *x, X *r, X *p, X *Ap, SolverScalars *s, double *part, unsigned *count, int *err) {
+                     X *x, X *r, X *p, X *Ap, typename CgpR<X>::T *rt, SolverScalars *s, CgpWord *mail, int *err) {
+    __shared__ CgpShared sh;
+    __shared__ X own[RPT > 0 ? RPT * kCgpThreads : 1];   // r of the CTA's rows
     const int G = gridDim.x;
-    if (s->done) return;
-    double zr = s->zr, rrv = s->rr;
+    if (s->done) return;   // the whole grid
+    double zr = s->zr, rrv = s->rr, alpha = 0.0, beta = 0.0;
     int it = s->it;
     const int max_iter = s->max_iter;
     const double tol2 = s->tol2;
-    double *partA = part, *partB = part + G;
     const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long)G * blockDim.x;
-    unsigned target = 0;
-    bool done = false;
+    const int first = blockIdx.x * RPT * kCgpThreads;   // the CTA's rows (RPT > 0)
+    unsigned number = 0;   // of the last exchange
+    bool done = false, good = true;
+    const bool lead = threadIdx.x >> 5 == kCgpLead;
+    if (threadIdx.x == 0) sh.ok = 1;
+    if (threadIdx.x < 2 * kCgpCluster * 2) (&sh.peer[0][0][0])[threadIdx.x] = CgpWord{0, 0};
+    cgp_cluster_sync();   // before a peer's first post
+    constexpr bool ONE = sizeof(X) == 8;   // one reduction per iteration
     constexpr int K = RPT > 0 ? RPT : 1;
     long row[K];
-    int beg[K], len[K], ci[K][kCgpMaxE];
-    X cv[K][kCgpMaxE], xr[K], rr[K], pr[K];
+    int beg[K], len[K], most[K], ci[K][kCgpMaxE];
+    X cv[K][kCgpMaxE], xv[K][kCgpMaxE], xr[K], rr[K], pr[K], qr[K], sr[K];
     if (RPT > 0) {
 #pragma unroll
         for (int k = 0; k < K; k++) {
-            row[k] = t0 + k * stride;
+            row[k] = first + k * kCgpThreads + threadIdx.x;
             len[k] = 0;
             beg[k] = 0;
+            xr[k] = rr[k] = pr[k] = qr[k] = sr[k] = X(0);
             if (row[k] < n) {
                 beg[k] = pntr[row[k]];
                 len[k] = pntr[row[k] + 1] - beg[k];
@@ -366,105 +484,210 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
 #pragma unroll
                 for (int e = 0; e < kCgpMaxE; e++)
                     if (e < len[k]) {
-                        ci[k][e] = indx[beg[k] + e];
+                        ci[k][e] = indx[beg[k] + e];   // below: -1 - its place among the CTA's own rows
                         cv[k][e] = Val<V>::get(vals[beg[k] + e]);
                     }
             }
+            most[k] = __reduce_max_sync(0xffffffffu, len[k] <= kCgpMaxE ? len[k] : 0);
         }
     }
-    // row k of this thread (RPT > 0) or row i (RPT = 0) times the vector v, whose entries other
-    // CTAs wrote during this launch (__ldcg: from L2)
-    auto row_product = [&](int k, long i, const X *v) -> X {
+    // row k of this thread (RPT > 0) times the vector whose entries are in xv, or far(column) for longer rows
+    auto row_product = [&](int k, auto far) -> X {
         X acc = X(0);
-        if (RPT > 0 && len[k] <= kCgpMaxE) {
-            X xv[kCgpMaxE];
-#pragma unroll
-            for (int e = 0; e < kCgpMaxE; e++)
-                if (e < len[k]) xv[e] = __ldcg(v + ci[k][e]);
-#pragma unroll
-            for (int e = 0; e < kCgpMaxE; e++)
-                if (e < len[k]) acc = cgp_acc<EXACT, X>(acc, cv[k][e], xv[e]);
-        } else {
-            const int jb = RPT > 0 ? beg[k] : pntr[i], je = RPT > 0 ? beg[k] + len[k] : pntr[i + 1];
-            for (int j = jb; j < je; j++) acc = cgp_acc<EXACT, X>(acc, Val<V>::get(vals[j]), __ldcg(v + indx[j]));
-        }
+        auto term = [&](int e) {
+            if (len[k] <= kCgpMaxE && e < len[k]) acc = cgp_acc<EXACT, X>(acc, cv[k][e], xv[k][e]);
+        };
+        term(0), term(1), term(2);
+        CGP_UNIFORM_IF(most[k] > 3) term(3);
+        CGP_UNIFORM_IF(most[k] > 4) term(4);
+        CGP_UNIFORM_IF(most[k] > 5) { term(5); term(6); term(7); }
+        if (len[k] > kCgpMaxE)
+            for (int j = beg[k]; j < beg[k] + len[k]; j++) acc = cgp_acc<EXACT, X>(acc, Val<V>::get(vals[j]), far(indx[j]));
         return acc;
     };
-    // q = A p for the direction the launch starts from, and <p, q>
-    X qr[K];
-    double pAp;
+    // row i (RPT = 0) times v, whose entries other CTAs wrote during this launch (__ldcg: from L2)
+    auto memory_product = [&](long i, const X *v) -> X {
+        X acc = X(0);
+        for (int j = pntr[i]; j < pntr[i + 1]; j++) acc = cgp_acc<EXACT, X>(acc, Val<V>::get(vals[j]), __ldcg(v + indx[j]));
+        return acc;
+    };
+    // The lead warp's last step: b = sum / den0 and a = sum / den1, one division in two lanes; then every thread's
+    auto finish = [&](bool ok, double sum, double den0, double den1) {
+        if (lead) {
+            const double q = sum / (threadIdx.x & 1 ? den1 : den0);
+            if ((threadIdx.x & 31) == 0) {
+                if (!ok) sh.ok = 0;
+                sh.sum = sum;
+                sh.beta = q;
+            }
+            if ((threadIdx.x & 31) == 1) sh.alpha = q;
+        }
+        __syncthreads();
+        alpha = (double)(X)sh.alpha;
+        beta = sh.beta;
+        good = sh.ok != 0;
+    };
+    auto nothing = [] {};
+    double sum[2] = {0.0, 0.0};
+    // q = A p for the direction the launch starts from, and a = <r, r> / <p, q>
     {
         DotAcc<X> pq;
         if (RPT > 0) {
 #pragma unroll
-            for (int k = 0; k < K; k++)
-                if (row[k] < n) {
-                    qr[k] = row_product(k, row[k], p);
-                    pq.add(pr[k], qr[k]);
-                }
-        } else {
-            for (long i = t0; i < n; i += stride) {
-                const X q = row_product(0, i, p);
-                Ap[i] = q;
-                pq.add(p[i], q);
-            }
-        }
-        target += G;
-        if (!cgp_reduce(pq.get(), partA, count, target, err, pAp)) return;
-    }
-    for (int c = 0; c < kCgpChunk; c++) {
-        // a = <r,z> / <p,Ap>; x += a p; r -= a Ap; ||r||^2 (r to memory: the next product reads it)
-        const X a = (X)(zr / pAp), ma = -a;
-        DotAcc<X> rrd;
-        if (RPT > 0) {
-#pragma unroll
             for (int k = 0; k < K; k++) {
-                if (row[k] >= n) continue;
-                xr[k] = add_rn(xr[k], mul_rn(a, pr[k]));
-                rr[k] = add_rn(rr[k], mul_rn(ma, qr[k]));
-                r[row[k]] = rr[k];
-                rrd.add(rr[k], rr[k]);
-            }
-        } else {
-            for (long i = t0; i < n; i += stride) {
-                x[i] = add_rn(x[i], mul_rn(a, p[i]));
-                const X ri = add_rn(r[i], mul_rn(ma, Ap[i]));
-                r[i] = ri;
-                rrd.add(ri, ri);
-            }
-        }
-        target += G;
-        if (!cgp_reduce(rrd.get(), partB, count, target, err, rrv)) return;
-        it++;
-        done = (it >= max_iter) || (rrv < tol2) || !(rrv == rrv);
-        if (done) break;
-        // z = r: <r, z> = ||r||^2; p = (zr_new / zr_old) p + z and, with s = A r, the product of the
-        // new direction by the same recurrence: Ap = (zr_new / zr_old) Ap + s.  So the product reads
-        // r, complete at the barrier above, and no barrier waits for the new p.
-        const X bta = (X)(rrv / zr);
-        DotAcc<X> pq;
-        if (RPT > 0) {
 #pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (row[k] >= n) continue;
-                const X sk = row_product(k, row[k], r);
-                pr[k] = add_rn(mul_rn(bta, pr[k]), rr[k]);
-                qr[k] = add_rn(mul_rn(bta, qr[k]), sk);
+                for (int e = 0; e < kCgpMaxE; e++)
+                    if (len[k] <= kCgpMaxE && e < len[k]) {
+                        xv[k][e] = __ldcg(p + ci[k][e]);
+                        const int at = ci[k][e] - first;
+                        if (at >= 0 && at < RPT * kCgpThreads) ci[k][e] = -1 - at;
+                    }
+                qr[k] = row_product(k, [&](int c) { return __ldcg(p + c); });
                 pq.add(pr[k], qr[k]);
             }
         } else {
             for (long i = t0; i < n; i += stride) {
-                const X si = row_product(0, i, r);
-                const X pi = add_rn(mul_rn(bta, p[i]), r[i]);
-                const X qi = add_rn(mul_rn(bta, Ap[i]), si);
-                p[i] = pi;
-                Ap[i] = qi;
-                pq.add(pi, qi);
+                const X q = memory_product(i, p);
+                Ap[i] = q;
+                pq.add(p[i], q);
             }
         }
+        number++;
+        const bool ok = cgp_exchange<false>(pq.get(), 0.0, number, mail, err, sh, nothing, sum);
+        finish(ok, zr, 1.0, sum[0]);
+    }
+    for (int c = 0; c < kCgpChunk && good; c++) {
+        const X a = (X)alpha, ma = -a, bta = (X)beta;
+        const double alpha_was = alpha;
+        const bool next = ONE && c > 0;   // p and q of this direction are still to be formed
+        DotAcc<X> rrd, rsd;
+        if (RPT > 0) {
+            const unsigned tag = c + 1;
+            X was[K];   // r first: the others wait for it
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (next) qr[k] = cgp_acc<EXACT, X>(sr[k], bta, qr[k]);
+                was[k] = rr[k];
+                rr[k] = cgp_acc<EXACT, X>(rr[k], ma, qr[k]);
+                own[k * kCgpThreads + threadIdx.x] = rr[k];
+                if (row[k] < n) CgpR<X>::put(rt + row[k], rr[k], tag);
+            }
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (next) pr[k] = cgp_acc<EXACT, X>(was[k], bta, pr[k]);
+                xr[k] = cgp_acc<EXACT, X>(xr[k], a, pr[k]);
+                rrd.add(rr[k], rr[k]);
+            }
+            __syncthreads();
+            // the neighbours' r: the whole warp waits as one (lanes leaving a loop one by one would stay apart)
+            constexpr int KG = K < 2 ? K : 2;   // rows with their loads in flight together (registers)
+#pragma unroll
+            for (int kb = 0; kb < K; kb += KG) {
+                for (int spins = 0;;) {
+                    bool here = true;
+#pragma unroll
+                    for (int k = kb; k < kb + KG; k++)
+#pragma unroll
+                        for (int e = 0; e < kCgpMaxE; e++)
+                            if (len[k] <= kCgpMaxE && e < len[k]) {
+                                if (ci[k][e] >= 0) here = CgpR<X>::get(rt + ci[k][e], tag, xv[k][e]) && here;
+                                else xv[k][e] = own[-1 - ci[k][e]];
+                            }
+                    if (__all_sync(0xffffffffu, here)) break;
+                    if (__any_sync(0xffffffffu, !cgp_wait_on(spins, err))) {
+                        sh.ok = 0;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int k = kb; k < kb + KG; k++) {
+                    sr[k] = row_product(k, [&](int col) {
+                        X v;
+                        for (int spins = 0; !CgpR<X>::get(rt + col, tag, v);)
+                            if (!cgp_wait_on(spins, err)) {
+                                sh.ok = 0;
+                                break;
+                            }
+                        return v;
+                    });
+                    rsd.add(rr[k], sr[k]);
+                }
+            }
+        } else {
+            for (long i = t0; i < n; i += stride) {
+                X pi = p[i], qi = Ap[i], ri = r[i];
+                if (next) {
+                    p[i] = pi = cgp_acc<EXACT, X>(ri, bta, pi);
+                    Ap[i] = qi = cgp_acc<EXACT, X>(((const X *)rt)[i], bta, qi);
+                }
+                x[i] = cgp_acc<EXACT, X>(x[i], a, pi);
+                r[i] = ri = cgp_acc<EXACT, X>(ri, ma, qi);
+                rrd.add(ri, ri);
+            }
+            number++;
+            const bool ok = cgp_exchange<true>(rrd.get(), 0.0, number, mail, err, sh, nothing, sum);
+            finish(ok, sum[0], zr, 1.0);
+            if (!good) break;
+            for (long i = t0; i < n; i += stride) {
+                const X si = memory_product(i, r);
+                rsd.add(r[i], si);
+                ((X *)rt)[i] = si;
+            }
+        }
+        if (ONE || RPT > 0) {
+            number++;
+            double ig = 0.0, ia = 0.0;
+            const bool ok = cgp_exchange<false>(rrd.get(), rsd.get(), number, mail, err, sh, [&] {
+                if (!ONE) return;
+                const double inv = 1.0 / (threadIdx.x & 1 ? alpha_was : zr);
+                ig = __shfl_sync(0xffffffffu, inv, 0);
+                ia = __shfl_sync(0xffffffffu, inv, 1);
+            }, sum);
+            finish(ok, sum[0], zr, sum[1] - (sum[0] * ig) * (sum[0] * ia));
+            if (!good) break;
+        }
+        rrv = sh.sum;
+        it++;
+        done = (it >= max_iter) || (rrv < tol2) || !(rrv == rrv);
+        if (done) break;
         zr = rrv;
-        target += G;
-        if (!cgp_reduce(pq.get(), partA, count, target, err, pAp)) return;
+        if (!ONE) {
+            const X bt = (X)beta;
+            DotAcc<X> pq;
+            if (RPT > 0) {
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    pr[k] = cgp_acc<EXACT, X>(rr[k], bt, pr[k]);
+                    qr[k] = cgp_acc<EXACT, X>(sr[k], bt, qr[k]);
+                    pq.add(pr[k], qr[k]);
+                }
+            } else {
+                for (long i = t0; i < n; i += stride) {
+                    const X pi = cgp_acc<EXACT, X>(r[i], bt, p[i]);
+                    const X qi = cgp_acc<EXACT, X>(((const X *)rt)[i], bt, Ap[i]);
+                    p[i] = pi;
+                    Ap[i] = qi;
+                    pq.add(pi, qi);
+                }
+            }
+            number++;
+            const bool ok = cgp_exchange<false>(pq.get(), 0.0, number, mail, err, sh, nothing, sum);
+            finish(ok, zr, 1.0, sum[0]);
+        }
+    }
+    if (ONE && good && !done) {   // the chunk's end: the next launch starts from this direction
+        const X bt = (X)beta;
+        if (RPT > 0) {
+#pragma unroll
+            for (int k = 0; k < K; k++) pr[k] = cgp_acc<EXACT, X>(rr[k], bt, pr[k]);
+        } else {
+            for (long i = t0; i < n; i += stride) p[i] = cgp_acc<EXACT, X>(r[i], bt, p[i]);
+        }
+    }
+    cgp_cluster_sync();   // no CTA ends before its peers' last posts to it
+    if (!good) {
+        if (threadIdx.x == 0) atomicOr(err, DEV_ERR_TIMEOUT);
+        return;
     }
     if (RPT > 0) {
 #pragma unroll
@@ -484,34 +707,58 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
     }
 }
 
+template <typename V, typename X, bool EXACT>
+static const void *cgp_kernel(int rpt) {
+    return rpt == 1   ? (const void *)cg_persistent_kernel<V, X, EXACT, 1>
+           : rpt == 2 ? (const void *)cg_persistent_kernel<V, X, EXACT, 2>
+           : rpt == 4 ? (const void *)cg_persistent_kernel<V, X, EXACT, 4>
+                      : (const void *)cg_persistent_kernel<V, X, EXACT, 0>;
+}
+
+static cudaLaunchConfig_t cgp_config(int grid, int cluster, cudaStream_t stream, cudaLaunchAttribute (&at)[2]) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kCgpThreads);
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+
 // Launch shape of the persistent CG: {grid, rows per thread (0: grid-stride)}; grid 0 when no
-// co-resident grid exists.  Every CTA costs each barrier one more arrival on the counter and each
-// reduction one more part, every row of a thread one more serial stretch of its phase: one row per
-// thread up to one CTA per SM, two up to two CTAs per SM, four up to two, else grid-stride loops.
-// (256^2 Poisson: 11.1 us per iteration with two rows per thread on 128 CTAs, 13.2 with four on 64.)
+// co-resident grid exists.  Every row of a thread is one more serial stretch of its phase, so as few rows per
+// thread as the co-resident clusters at one CTA per SM hold: one, two or four; else grid-stride loops.
+// Clusters of eight, or of four or two where more CTAs are needed than clusters of eight fit (15, 36 and 76 of them on
+// 152 SMs).  256^2: 5.9 us per iteration with two rows per thread on 128 CTAs, 9.9 (of an earlier form at 7.4) with four on 64.
 struct CgpShape {
-    int grid = 0, rpt = 0;
+    int grid = 0, rpt = 0, cluster = 0;
 };
 template <typename V, typename X, bool EXACT>
-static CgpShape cgp_shape(hgb_ctx *c, long n) {
+static CgpShape cgp_shape(long n) {
     CgpShape sh;
-    int nb[4] = {0, 0, 0, 0};
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], cg_persistent_kernel<V, X, EXACT, 0>, kCgpThreads, 0) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], cg_persistent_kernel<V, X, EXACT, 1>, kCgpThreads, 0) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[2], cg_persistent_kernel<V, X, EXACT, 2>, kCgpThreads, 0) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[3], cg_persistent_kernel<V, X, EXACT, 4>, kCgpThreads, 0)) {
-        cudaGetLastError();
-        return sh;
-    }
-    const long g1 = (n + kCgpThreads - 1) / kCgpThreads;
-    const long g2 = (n + 2L * kCgpThreads - 1) / (2L * kCgpThreads), g4 = (n + 4L * kCgpThreads - 1) / (4L * kCgpThreads);
-    if (g1 <= std::min<long>((long)nb[1] * c->num_sms, (long)c->num_sms)) return CgpShape{(int)g1, 1};
-    if (g2 <= std::min<long>((long)nb[2] * c->num_sms, 2L * c->num_sms)) return CgpShape{(int)g2, 2};
-    if (g4 <= std::min<long>((long)nb[3] * c->num_sms, 2L * c->num_sms)) return CgpShape{(int)g4, 4};
-    // about four rows per thread: fewer CTAs make cheaper barriers, the data are in L2 anyway
-    const long want = std::max<long>(1, (n + 4L * kCgpThreads - 1) / (4L * kCgpThreads));
-    sh.grid = (int)std::min<long>(want, (long)nb[0] * c->num_sms);
-    sh.rpt = 0;
+    for (int rpt : {1, 2, 4, 0})
+        for (int cluster = kCgpCluster; cluster > 1; cluster /= 2) {
+            cudaLaunchAttribute at[2];
+            const cudaLaunchConfig_t cfg = cgp_config(cluster, cluster, nullptr, at);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, cgp_kernel<V, X, EXACT>(rpt), &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                return sh;
+            }
+            clusters = std::min(clusters, 16 * kCgpMail);
+            const long rows = (rpt ? rpt : 4) * (long)kCgpThreads * cluster;   // of a cluster
+            const long want = (n + rows - 1) / rows;
+            if (clusters < 1 || (rpt && want > clusters)) continue;
+            sh.grid = (int)std::min<long>(want, clusters) * cluster;
+            sh.rpt = rpt;
+            sh.cluster = cluster;
+            return sh;
+        }
     return sh;
 }
 
@@ -522,38 +769,34 @@ static bool cgp_eligible(hgb_csr *A, hgb_ilu *M, bool trans) {
     return !M && !trans && n > 0 && n <= kCgpMaxRows && bytes <= kCgpMaxBytes;
 }
 
-template <typename V, typename X, bool EXACT>
-static const void *cgp_kernel(int rpt) {
-    return rpt == 1   ? (const void *)cg_persistent_kernel<V, X, EXACT, 1>
-           : rpt == 2 ? (const void *)cg_persistent_kernel<V, X, EXACT, 2>
-           : rpt == 4 ? (const void *)cg_persistent_kernel<V, X, EXACT, 4>
-                      : (const void *)cg_persistent_kernel<V, X, EXACT, 0>;
-}
-
 // Runs the loop of an initialised CgWork (r, p, the scalars' zr / it / tol2) to the end.
 template <typename V, typename X>
 static int cgp_run(hgb_ctx *c, hgb_csr *A, CgWork<X> &w, X *x, long n, long long *launches, SolverScalars &hs) {
     const bool exact = (c->spmv_mode == HGB_SPMV_EXACT);
-    const CgpShape sh = exact ? cgp_shape<V, X, true>(c, n) : cgp_shape<V, X, false>(c, n);
+    const CgpShape sh = exact ? cgp_shape<V, X, true>(n) : cgp_shape<V, X, false>(n);
     const int G = sh.grid;
     if (G < 1) return fail(HGB_ERR_UNSUPPORTED, "persistent cg: no co-resident grid");
-    double *part = nullptr;
-    unsigned *count = nullptr;
+    CgpWord *mail = nullptr;   // two sets of an entry (two words) per CTA and cluster
+    typename CgpR<X>::T *rt = nullptr;
+    const size_t nmail = 2 * (size_t)G * (G / sh.cluster) * 2;
     int st = HGB_OK;
-    if (ws_alloc(c, &part, 2 * (size_t)G) || ws_alloc(c, &count, 1)) st = cuda_fail(cudaErrorMemoryAllocation, "persistent cg");
+    if (ws_alloc(c, &mail, nmail) || ws_alloc(c, &rt, n)) st = cuda_fail(cudaErrorMemoryAllocation, "persistent cg");
     const int *pntr = csr_pntr(A), *indx = csr_indx(A);
     const V *vals = (const V *)csr_vals(A);
     SolverScalars *s = c->scal;
     int *err = c->err;
     X *r = w.r, *p = w.p, *Ap = w.Ap;
-    void *args[] = {&n, &pntr, &indx, &vals, &x, &r, &p, &Ap, &s, &part, &count, &err};
+    void *args[] = {&n, &pntr, &indx, &vals, &x, &r, &p, &Ap, &rt, &s, &mail, &err};
     while (!st) {
-        if (cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream) != cudaSuccess) {
+        if (cudaMemsetAsync(mail, 0, sizeof(CgpWord) * nmail, c->stream) != cudaSuccess ||
+            cudaMemsetAsync(rt, 0, sizeof(typename CgpR<X>::T) * n, c->stream) != cudaSuccess) {
             st = cuda_fail(cudaGetLastError(), "persistent cg");
             break;
         }
         const void *fn = exact ? cgp_kernel<V, X, true>(sh.rpt) : cgp_kernel<V, X, false>(sh.rpt);
-        if (cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kCgpThreads), args, 0, c->stream) != cudaSuccess) {
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = cgp_config(G, sh.cluster, c->stream, at);
+        if (cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess) {
             st = cuda_fail(cudaGetLastError(), "persistent cg launch");
             break;
         }
@@ -567,8 +810,8 @@ static int cgp_run(hgb_ctx *c, hgb_csr *A, CgWork<X> &w, X *x, long n, long long
         if ((st = collect_dev_error(c))) break;
         if (hs.done) break;
     }
-    ws_free(c, part);
-    ws_free(c, count);
+    ws_free(c, mail);
+    ws_free(c, rt);
     return st;
 }
 
