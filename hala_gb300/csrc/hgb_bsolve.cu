@@ -270,13 +270,6 @@ __device__ __forceinline__ X bs_wait_slot(uint32_t a, X v, int *err) {
 // turn behind it, or computes both sides of a (warp-uniform) choice and selects.
 __device__ __forceinline__ void bs_pin(double &v) { asm volatile("" : "+d"(v)); }
 __device__ __forceinline__ void bs_pin(float &v) { asm volatile("" : "+f"(v)); }
-// A warp-uniform choice that stays a branch: the assembler turns short conditional blocks into predicated
-// instructions, and a predicated-off FP64 instruction holds the unit like any other.
-__device__ __forceinline__ int bs_opaque(int v) {
-    asm volatile("" : "+r"(v));
-    return v;
-}
-#define BS_UNIFORM_IF(cond) _Pragma("unroll 1") for (int z_ = bs_opaque((cond) ? 1 : 0); z_ > 0; z_ = bs_opaque(z_ - 1))
 // one product taken into the sum
 template <int MODE, typename X>
 __device__ __forceinline__ X bs_term(X acc, X m) {
@@ -483,11 +476,11 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                             x2 = bs_slot(p.w & kBsFar << 2 ? a2 : sbase, X(0));
                     early = !__any_sync(0xFFFFFFFFu, bs_pending(x0) || bs_pending(x1) || bs_pending(x2));
                     if (XS == 8) {
-                        BS_UNIFORM_IF(early && early0) {
+                        HGB_UNIFORM_IF(early && early0) {
                             acc = bs_term<MODE>(acc, mul_rn(rw.v[0], x0));
                             bs_pin(acc);
                         }
-                        BS_UNIFORM_IF(early && early2 && !no2) {
+                        HGB_UNIFORM_IF(early && early2 && !no2) {
                             m2 = mul_rn(rw.v[2], x2);
                             bs_pin(m2);
                         }
@@ -514,16 +507,16 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                 if (XS == 8) {
                     X m1 = mul_rn(rw.v[1], x1);
                     bs_pin(m1);
-                    BS_UNIFORM_IF(!early || !early0) {
+                    HGB_UNIFORM_IF(!early || !early0) {
                         acc = bs_term<MODE>(acc, mul_rn(rw.v[0], x0));
                         bs_pin(acc);
                     }
-                    BS_UNIFORM_IF((!early || !early2) && !no2) {
+                    HGB_UNIFORM_IF((!early || !early2) && !no2) {
                         m2 = mul_rn(rw.v[2], x2);
                         bs_pin(m2);
                     }
                     acc = bs_term<MODE>(acc, m1);
-                    BS_UNIFORM_IF(!no2) {
+                    HGB_UNIFORM_IF(!no2) {
                         acc = bs_term<MODE>(acc, m2);
                         bs_pin(acc);
                     }

@@ -49,7 +49,7 @@ template <> struct Val<uint16_t> {   // bfloat16 bit pattern
 // memory; the float partials of 16 terms keep the per-thread error at the FP32 level of the data.
 template <typename X> struct DotAcc {
     double d = 0.0;
-    __device__ __forceinline__ void add(X a, X b) { d += (double)a * (double)b; }
+    __device__ __forceinline__ void add(X a, X b) { d = fma((double)a, (double)b, d); }
     __device__ __forceinline__ double get() const { return d; }
 };
 template <> struct DotAcc<float> {
@@ -76,6 +76,14 @@ __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, 
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 
+
+// A warp-uniform choice that stays a branch: the assembler turns short conditional blocks into predicated
+// instructions, and a predicated-off FP64 instruction holds the unit like any other.
+__device__ __forceinline__ int hgb_opaque(int v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+#define HGB_UNIFORM_IF(cond) _Pragma("unroll 1") for (int z_ = hgb_opaque((cond) ? 1 : 0); z_ > 0; z_ = hgb_opaque(z_ - 1))
 
 // Cached transpose of a CSR pattern: pntr[n+1], row[nnz] (original row of each entry, ascending
 // inside a transposed row) and map[nnz] (position of the entry in the original arrays).

@@ -187,7 +187,7 @@ __global__ void residual_norm_kernel(long n, const double *__restrict__ r, doubl
                                      double *out) {
     double acc[1] = {0.0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        acc[0] += r[i] * r[i];
+        acc[0] = fma(r[i], r[i], acc[0]);
     grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) { *out = v[0]; });
 }
 
@@ -336,14 +336,6 @@ __device__ __forceinline__ bool cgp_wait_on(int &spins, const int *err) {
     return (spins & 1023) != 0 || !(*(const volatile int *)err & DEV_ERR_TIMEOUT);
 }
 
-// A warp-uniform choice that stays a branch: the assembler turns short conditional blocks into predicated
-// instructions, and a predicated-off FP64 instruction holds the unit like any other.
-__device__ __forceinline__ int cgp_opaque(int v) {
-    asm volatile("" : "+r"(v));
-    return v;
-}
-#define CGP_UNIFORM_IF(cond) _Pragma("unroll 1") for (int z_ = cgp_opaque((cond) ? 1 : 0); z_ > 0; z_ = cgp_opaque(z_ - 1))
-
 // A reduction of two sums: the CTAs of a cluster exchange theirs through distributed shared memory, then the CTAs of
 // equal rank exchange the clusters' through mailboxes in memory (every CTA has its own, one entry per cluster).
 // 256^2, 128 CTAs: 2100 cycles for the mail, where 128 CTAs polling one set of entries waited 6500 and each its own
@@ -428,8 +420,8 @@ __device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned numb
         }
         if (ORDER) cgp_fence();
         t = part[0];
-        CGP_UNIFORM_IF(clusters > 16) t += part[1];
-        CGP_UNIFORM_IF(clusters > 32) t += part[2] + part[3];
+        HGB_UNIFORM_IF(clusters > 16) t += part[1];
+        HGB_UNIFORM_IF(clusters > 32) t += part[2] + part[3];
         for (unsigned o = 1; o < clusters && o < 16; o *= 2) t = cgp_add_xor(t, o);
     }
     sum[0] = __shfl_sync(0xffffffffu, t, 0);
@@ -498,9 +490,9 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
             if (len[k] <= kCgpMaxE && e < len[k]) acc = cgp_acc<EXACT, X>(acc, cv[k][e], xv[k][e]);
         };
         term(0), term(1), term(2);
-        CGP_UNIFORM_IF(most[k] > 3) term(3);
-        CGP_UNIFORM_IF(most[k] > 4) term(4);
-        CGP_UNIFORM_IF(most[k] > 5) { term(5); term(6); term(7); }
+        HGB_UNIFORM_IF(most[k] > 3) term(3);
+        HGB_UNIFORM_IF(most[k] > 4) term(4);
+        HGB_UNIFORM_IF(most[k] > 5) { term(5); term(6); term(7); }
         if (len[k] > kCgpMaxE)
             for (int j = beg[k]; j < beg[k] + len[k]; j++) acc = cgp_acc<EXACT, X>(acc, Val<V>::get(vals[j]), far(indx[j]));
         return acc;
@@ -1099,7 +1091,7 @@ __global__ void ru_replace_kernel(long n, SolverScalars *s, const double *__rest
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const double v = r64[i];
         r[i] = (float)v;
-        acc[0] += v * v;
+        acc[0] = fma(v, v, acc[0]);
     }
     grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
         const double rr = v[0];
@@ -1354,7 +1346,7 @@ __global__ void gm_start_kernel(long n, GmresState *st, const X *__restrict__ r,
     if (st->done) return;
     double acc[1] = {0.0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        acc[0] += (double)r[i] * (double)r[i];
+        acc[0] = fma((double)r[i], (double)r[i], acc[0]);
     grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
         double beta = __dsqrt_rn(v[0]);
         if (st->first) {
@@ -1385,38 +1377,129 @@ __global__ void gm_scale_kernel(long n, const GmresState *__restrict__ st, X *__
     }
 }
 
+// The basis kernels below read k columns of n and do one FP64 operation per entry (two a warp-wide instruction, 62
+// cycles of an SM quarter's unit each, were it rounded separately): at 96^3 a column costs 1.4 us of the unit
+// and 1.0 us of HBM.  So they take fused multiply-adds, keep instructions for absent columns as branches
+// (HGB_UNIFORM_IF), and sum 32 lanes' 32 columns with 31 additions a lane instead of 160.
+
+// Sums v[j] over the warp for KMAX columns j: column lane % KMAX's sum in v[0].  Each step adds two lanes' halves of the
+// columns and leaves each lane one of them.
+template <int KMAX>
+__device__ __forceinline__ void gm_warp_columns(double (&v)[KMAX]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o >= KMAX; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < KMAX; j++) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+#pragma unroll
+    for (int o = KMAX < 32 ? KMAX / 2 : 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < o; j++) {
+            const double keep = lane & o ? v[j + o] : v[j], send = lane & o ? v[j] : v[j + o];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+}
+
 // cf[0..k] = W[:, 0..k]^T r   (krylov_project's gemv 'T', :67-70), for the k1 columns from W and cf
-// on (one group of up to 64 columns per launch)
+// on (one group of up to 32 columns per launch).  All columns' loads of a row are in flight together; 96^3 FP64,
+// 30 columns: 180 -> 62 us.
 template <typename X, int KMAX>
-__global__ void gm_dots_kernel(long n, int k1, const GmresState *__restrict__ st, const X *__restrict__ W,
-                               const X *__restrict__ r, double *cf, double *partials, unsigned *counter) {
+__global__ void __launch_bounds__(256, 32 / KMAX)
+gm_dots_kernel(long n, int k1, const GmresState *__restrict__ st, const X *__restrict__ W,
+               const X *__restrict__ r, double *cf, double *partials, unsigned *counter) {
     if (st->stop) return;
+    __shared__ double sh[8 * KMAX];
+    __shared__ bool last;
     double acc[KMAX];
 #pragma unroll
     for (int j = 0; j < KMAX; j++) acc[j] = 0.0;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const double ri = (double)r[i];
+    const int tid = threadIdx.x;
+    const long stride = (long)gridDim.x * 256;
+    X wn[KMAX], rn = X(0);   // the next row's
+    auto load = [&](long i) {
+        rn = i < n ? r[i] : X(0);
 #pragma unroll
-        for (int j = 0; j < KMAX; j++)
-            if (j < k1) acc[j] += (double)W[(long)j * n + i] * ri;
+        for (int j = 0; j < KMAX; j++) wn[j] = j < k1 && i < n ? W[(long)j * n + i] : X(0);
+    };
+    long ib = (long)blockIdx.x * 256 + (tid & ~31);
+    load(ib + (tid & 31));
+    for (; ib < n; ib += stride) {
+        const double ri = (double)rn;
+        X w[KMAX];
+#pragma unroll
+        for (int j = 0; j < KMAX; j++) w[j] = wn[j];
+        load(ib + stride + (tid & 31));
+#pragma unroll
+        for (int j = 0; j < KMAX; j += 2)
+            HGB_UNIFORM_IF(j < k1) {
+                acc[j] = fma((double)w[j], ri, acc[j]);
+                acc[j + 1] = fma((double)w[j + 1], ri, acc[j + 1]);
+            }
     }
-    grid_sum<KMAX>(acc, partials, counter, [&](double (&s)[KMAX]) {
-        for (int j = 0; j < k1; j++) cf[j] = s[j];
-    });
+    gm_warp_columns<KMAX>(acc);
+    if ((tid & 31) < KMAX) sh[(tid >> 5) * KMAX + (tid & 31)] = acc[0];
+    __syncthreads();
+    auto column = [&] {
+        double t = sh[tid];
+#pragma unroll
+        for (int w = 1; w < 8; w++) t += sh[w * KMAX + tid];
+        return t;
+    };
+    if (tid < 32) {
+        if (tid < KMAX) {
+            partials[blockIdx.x * KMAX + tid] = column();
+            __threadfence();
+        }
+        __syncwarp();
+        if (tid == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;   // the last CTA: column tid % KMAX, every (256 / KMAX)-th CTA's part
+    for (int b = tid / KMAX; b < (int)gridDim.x; b += 256 / KMAX) t += __ldcg(partials + b * KMAX + tid % KMAX);
+#pragma unroll
+    for (int o = KMAX; o < 32; o *= 2) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((tid & 31) < KMAX) sh[(tid >> 5) * KMAX + (tid & 31)] = t;
+    __syncthreads();
+    if (tid < k1) cf[tid] = column();
+    if (tid == 0) *counter = 0u;
+}
+
+// v + sum over j < k of c[j] W[j * n + i], column by column; eight columns' loads in flight
+template <typename X>
+__device__ __forceinline__ X gm_combine(X v, long n, long i, int k, const X *__restrict__ W, const X *c) {
+    for (int j0 = 0; j0 < k; j0 += 8) {
+        X w[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (j0 + q < k) w[q] = W[(long)(j0 + q) * n + i];
+#pragma unroll
+        for (int q = 0; q < 8; q++) HGB_UNIFORM_IF(j0 + q < k) v = fma(c[j0 + q], w[q], v);
+    }
+    return v;
 }
 
 // r -= W cf (krylov_project's gemv 'N', :71-76), ||r||, then in the last CTA the Givens step of
-// solve_gmres (:190-216) for column k of the Hessenberg matrix.
+// solve_gmres (:190-216) for column k of the Hessenberg matrix.  96^3 FP64, 30 columns: 123 -> 66 us.
 template <typename X>
-__global__ void gm_update_kernel(long n, int k, GmresState *st, const X *__restrict__ W, const double *__restrict__ cf,
-                                 X *__restrict__ r, double *partials, unsigned *counter) {
+__global__ void __launch_bounds__(256, 4)
+gm_update_kernel(long n, int k, GmresState *st, const X *__restrict__ W, const double *__restrict__ cf,
+                 X *__restrict__ r, double *partials, unsigned *counter) {
     if (st->stop) return;
+    __shared__ X c[kGmresMaxRestart];
+    __shared__ double cs[2][kGmresMaxRestart];   // the previous rotations, for the last CTA's chain
+    for (int j = threadIdx.x; j <= k; j += 256) {
+        c[j] = (X)-cf[j];
+        cs[0][j] = st->C[j];
+        cs[1][j] = st->S[j];
+    }
+    __syncthreads();
     double acc[1] = {0.0};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        X ri = r[i];
-        for (int j = 0; j <= k; j++) ri = add_rn(ri, mul_rn((X)-cf[j], W[(long)j * n + i]));
+    for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += gridDim.x * 256L) {
+        const X ri = gm_combine(r[i], n, i, k + 1, W, c);
         r[i] = ri;
-        acc[0] += (double)ri * (double)ri;
+        acc[0] = fma((double)ri, (double)ri, acc[0]);
     }
     grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
         const double nrm = __dsqrt_rn(v[0]);
@@ -1425,7 +1508,7 @@ __global__ void gm_update_kernel(long n, int k, GmresState *st, const X *__restr
         double hi = cf[0];
         for (int i = 0; i < k; i++) {
             double hn = cf[i + 1];
-            gm_rot(hi, hn, st->C[i], st->S[i]);
+            gm_rot(hi, hn, cs[0][i], cs[1][i]);
             Hk[i] = hi;
             hi = hn;
         }
@@ -1451,52 +1534,52 @@ __global__ void gm_update_kernel(long n, int k, GmresState *st, const X *__restr
     });
 }
 
-// End of a cycle: tpsv('U','N','N', k, H, Z) (:219-223), the restart bookkeeping (:225-229)
+// End of a cycle: tpsv('U','N','N', k, H, Z) (:219-223), the restart bookkeeping (:225-229).  One warp: a column's
+// subtractions in parallel (restart 30: 77 -> 32 us)
 __global__ void gm_end_kernel(GmresState *st) {
     if (st->done) return;
-    const int nz = st->k;
-    if (nz > 0) {
-        long kk = (long)nz * (nz + 1) / 2 - 1;
-        for (int j = nz - 1; j >= 0; j--) {
-            if (st->Z[j] != 0.0) {
-                st->Z[j] = __ddiv_rn(st->Z[j], st->H[kk]);
-                const double tt = st->Z[j];
-                long q = kk - 1;
-                for (int i = j - 1; i >= 0; i--, q--) st->Z[i] = __dsub_rn(st->Z[i], __dmul_rn(tt, st->H[q]));
-            }
-            kk -= j + 1;
+    const int nz = st->k, lane = threadIdx.x;
+    for (int j = nz - 1; j >= 0; j--) {
+        const double *Hj = st->H + (long)j * (j + 1) / 2;
+        if (st->Z[j] != 0.0) {
+            const double tt = __ddiv_rn(st->Z[j], Hj[j]);
+            __syncwarp();   // every lane has read Z[j]
+            for (int i = lane; i < j; i += 32) st->Z[i] = __dsub_rn(st->Z[i], __dmul_rn(tt, Hj[i]));
+            if (lane == 0) st->Z[j] = tt;
         }
-        st->upd = 1;
+        __syncwarp();
     }
-    st->outer += 1;
-    st->outer_res = st->inner_res;
-    st->done = !(st->outer_res > st->tol && st->outer < st->max_outer);
+    if (lane == 0) {
+        if (nz > 0) st->upd = 1;
+        st->outer += 1;
+        st->outer_res = st->inner_res;
+        st->done = !(st->outer_res > st->tol && st->outer < st->max_outer);
+    }
 }
 
 // x += W[:, 0..k-1] Z   (krylov_combine, :53-60), column by column in the reference's order
 template <typename X>
-__global__ void gm_xupdate_kernel(long n, const GmresState *__restrict__ st, const X *__restrict__ W, X *__restrict__ x) {
+__global__ void __launch_bounds__(256, 4)
+gm_xupdate_kernel(long n, const GmresState *__restrict__ st, const X *__restrict__ W, X *__restrict__ x) {
     if (!st->upd) return;
+    __shared__ X c[kGmresMaxRestart];
     const int nz = st->k;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        X xi = x[i];
-        for (int j = 0; j < nz; j++) xi = add_rn(xi, mul_rn((X)st->Z[j], W[(long)j * n + i]));
-        x[i] = xi;
-    }
+    for (int j = threadIdx.x; j < nz; j += 256) c[j] = (X)st->Z[j];
+    __syncthreads();
+    for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += gridDim.x * 256L) x[i] = gm_combine(x[i], n, i, nz, W, c);
 }
 
 template <typename X>
 static int gm_dots_launch(hgb_ctx *c, long n, int k1, const GmresState *st, const X *W, const X *r, double *cf) {
-    // up to 64 partial sums per CTA: the grid stays below the SpMV parts of the context's partials
-    const int grid = std::min(reduce_grid(c, n, 256 * 8), (int)(kSpmvPartsOffset / 64));
-    for (int j0 = 0; j0 < k1; j0 += 64) {   // groups of up to 64 columns, one grid reduction each
-        const int kk = std::min(64, k1 - j0);
+    for (int j0 = 0; j0 < k1; j0 += 32) {   // groups of up to 32 columns, one grid reduction each
+        const int kk = std::min(32, k1 - j0);
         const X *Wj = W + (long)j0 * n;
         double *cj = cf + j0;
-        if (kk <= 8) gm_dots_kernel<X, 8><<<grid, 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
-        else if (kk <= 16) gm_dots_kernel<X, 16><<<grid, 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
-        else if (kk <= 32) gm_dots_kernel<X, 32><<<grid, 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
-        else gm_dots_kernel<X, 64><<<grid, 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
+        // resident CTAs (KMAX loads and sums a thread: 32 / KMAX CTAs per SM); at most 32 parts per CTA
+        auto grid = [&](int kmax) { return (int)std::max<long>(1, std::min<long>((n + 255) / 256, (long)c->num_sms * (32 / kmax))); };
+        if (kk <= 8) gm_dots_kernel<X, 8><<<grid(8), 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
+        else if (kk <= 16) gm_dots_kernel<X, 16><<<grid(16), 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
+        else gm_dots_kernel<X, 32><<<grid(32), 256, 0, c->stream>>>(n, kk, st, Wj, r, cj, c->partials, c->counter);
         HGB_TRY(launch_check("gm_dots_kernel"));
     }
     return HGB_OK;
@@ -1550,7 +1633,7 @@ static int gmres_run(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, int restart, const X *b
                 gm_scale_kernel<X><<<ew_grid(c, n), 256, 0, c->stream>>>(n, st, r, W);
             }
             if (rc) break;
-            gm_end_kernel<<<1, 1, 0, c->stream>>>(st);
+            gm_end_kernel<<<1, 32, 0, c->stream>>>(st);
             gm_xupdate_kernel<X><<<ew_grid(c, n), 256, 0, c->stream>>>(n, st, W, x);
             rc = launch_check("gmres cycle");
         } while (0);
