@@ -46,7 +46,7 @@ constexpr long kPartialsDoubles = (long)kMaxReduceBlocks * 64;
 
 // Scalars kept on the device by the fused solvers (one set per context).
 struct SolverScalars {
-    double zr, pap, rr, nzr;     // CG recurrences
+    double zr, pap, rr, nzr;     // CG recurrences (nzr: the newest <r, z>; zr: the one before it)
     double tol2;                 // stopping threshold on ||r||^2
     double r0;                   // first residual norm of the current inner solve
     double rel;                  // inner relative tolerance (IR); 0 = absolute test only

@@ -21,43 +21,114 @@ namespace hgb {
 constexpr int kItersPerGraph = 16;
 
 // Elements a thread takes per round in the CG vector kernels, their loads issued together: the
-// kernels are short and latency-bound (about 14 elements per thread at 128^3), so one element per
-// round left a thread waiting on one memory round trip per element.
+// kernels are short and latency-bound (14 elements per thread at 128^3), so a round's loads are all that one
+// memory round trip brings.
 template <typename X, int NARR = 2> __host__ __device__ constexpr int ew_unroll() {
-    return (sizeof(X) == 8 ? 4 : 8) / (NARR > 2 ? 2 : 1);   // NARR: vectors read per element
+    return (sizeof(X) == 8 ? 4 : 8) / (NARR > 2 ? 2 : 1);   // NARR: vectors read or written per element
 }
-// their grids are num_sms x 4 CTAs of 256 threads: the register budget keeps all four resident
-// (unbounded, the batched loads took up to 86 registers and the grid ran in two waves)
-constexpr int kEwThreads = 256, kEwCtasPerSm = 4;
+// Two CTAs of 512 threads per SM, and sums and quotients in as few warps as do: an FP64 instruction takes an SM
+// quarter's unit for 62 cycles, whichever of the warps repeats it.  With four CTAs of 256 threads each warp summed,
+// divided and reduced: 128^3 FP32, from start to start of the launches, the d / r update 21.5 us, <r, z> 18.6; now
+// 17 and 13.  (Shapes of 256 to 1,024 threads and 4 to 16 loads a round: the whole mixed solve within 1.5 %.)
+constexpr int kEwThreads = 512, kEwCtas = 2;
+static inline int vec_grid(const hgb_ctx *c, long n) {
+    return (int)std::max<long>(1, std::min<long>((n + kEwThreads - 1) / kEwThreads, (long)c->num_sms * kEwCtas));
+}
 
-// <p, Ap>: the SpMV's per-CTA parts summed in one order in every CTA (pap_n > 0), or the value
-// its grid reduction stored (pap_n == 0: the transposed product)
-__device__ __forceinline__ double parts_sum(const double *part, int np, double stored) {
-    if (np == 0) return stored;
-    __shared__ double res;
-    double v[1] = {0.0};
-    for (int b = threadIdx.x; b < np; b += blockDim.x) v[0] += part[b];
-    block_sum<1>(v);
-    if (threadIdx.x == 0) res = v[0];
+// The sum of np parts, or the value a grid reduction stored (np == 0), mapped by f in one thread and
+// given to all: four warps, one per SM quarter, add the parts.
+template <typename F>
+__device__ __forceinline__ double vec_scalar(const double *part, int np, double stored, F f) {
+    __shared__ double sh[4], res;
+    const int tid = threadIdx.x;
+    if (np > 0 && tid < 128) {
+        double v = 0.0;
+        for (int b = tid; b < np; b += 128) v += part[b];
+        v = warp_sum(v);
+        if ((tid & 31) == 0) sh[tid >> 5] = v;
+    }
+    __syncthreads();
+    if (tid == 0) res = f(np > 0 ? (sh[0] + sh[1]) + (sh[2] + sh[3]) : stored);
     __syncthreads();
     return res;
 }
 
+// As grid_sum for NV values of kEwThreads threads: every CTA's part, the last CTA adds them in one order and runs
+// fin(sums) in thread 0.  128 threads add four values each before a warp's lanes are added.
+template <int NV, bool PARTS = false, typename Fin>
+__device__ __forceinline__ void vec_grid_sum(const double (&v)[NV], double *partials, unsigned *counter, Fin fin) {
+    __shared__ double sh[NV][kEwThreads], shw[NV][4];
+    __shared__ bool last;
+    const int tid = threadIdx.x, G = gridDim.x;
+    auto finish = [&](double (&t)[NV]) {   // 128 threads' values -> thread 0
+        if (tid < 128) {
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                t[k] = warp_sum(t[k]);
+                if ((tid & 31) == 0) shw[k][tid >> 5] = t[k];
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int k = 0; k < NV; k++) t[k] = (shw[k][0] + shw[k][1]) + (shw[k][2] + shw[k][3]);
+        }
+    };
+    double t[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) sh[k][tid] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; k++) t[k] = 0.0;
+    if (tid < 128) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            t[k] = sh[k][tid];
+#pragma unroll
+            for (int w = 128; w < kEwThreads; w += 128) t[k] += sh[k][tid + w];
+        }
+    }
+    finish(t);
+    if (tid == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) partials[blockIdx.x * NV + k] = t[k];
+    }
+    if (PARTS) return;   // the parts are the result
+    if (tid == 0) {
+        __threadfence();
+        last = atomicAdd(counter, 1u) == (unsigned)G - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < NV; k++) t[k] = 0.0;
+    if (tid < 128)
+        for (int b = tid; b < G; b += 128)
+#pragma unroll
+            for (int k = 0; k < NV; k++) t[k] += __ldcg(partials + b * NV + k);
+    finish(t);
+    if (tid == 0) {
+        *counter = 0u;
+        fin(t);
+    }
+}
+
+// acc + a x: one fused multiply-add in FP64 (half the unit's time), separately rounded in FP32
+__device__ __forceinline__ double vec_axpy(double acc, double a, double x) { return fma(a, x, acc); }
+__device__ __forceinline__ float vec_axpy(float acc, float a, float x) { return add_rn(acc, mul_rn(a, x)); }
+
 template <typename X>
-__global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_update_kernel(long n, const SolverScalars *__restrict__ s_in, SolverScalars *s,
+__global__ void __launch_bounds__(kEwThreads, kEwCtas) cg_update_kernel(long n, const SolverScalars *__restrict__ s_in, SolverScalars *s,
                                  const X *__restrict__ p, const X *__restrict__ Ap, X *__restrict__ x,
                                  X *__restrict__ r, double *partials, unsigned *counter, const double *pap_part,
                                  int pap_n) {
     if (s_in->done) return;
-    const double pap = parts_sum(pap_part, pap_n, s_in->pap);
-    // a = <r,z> / <p,Ap>; x += a p; r -= a Ap  (axpy(a,p,x), axpy(-a,Ap,r))
-    const X a = (X)(s_in->zr / pap);
-    const X ma = -a;
-    DotAcc<X> rr;
     constexpr int U = ew_unroll<X, 4>();
     const long T = (long)gridDim.x * blockDim.x;
-    for (long base = blockIdx.x * (long)blockDim.x + threadIdx.x; base < n; base += T * U) {
-        X pv[U], av[U], xv[U], rv[U];
+    long base = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    X pv[U], av[U], xv[U], rv[U];
+    auto load = [&] {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
@@ -68,30 +139,44 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_update_kernel(lon
                 rv[u] = r[i];
             }
         }
+    };
+    load();   // in flight while the scalar is summed
+    // a = <r,z> / <p,Ap>; x += a p; r -= a Ap  (axpy(a,p,x), axpy(-a,Ap,r))
+    double pap = 0.0;   // thread 0's
+    const X a = (X)vec_scalar(pap_part, pap_n, s_in->pap, [&](double v) { pap = v; return s_in->nzr / v; });
+    const X ma = -a;
+    DotAcc<X> rr;
+    while (base < n) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
             if (i < n) {
-                x[i] = add_rn(xv[u], mul_rn(a, pv[u]));
-                const X ri = add_rn(rv[u], mul_rn(ma, av[u]));
+                x[i] = vec_axpy(xv[u], a, pv[u]);
+                const X ri = vec_axpy(rv[u], ma, av[u]);
                 r[i] = ri;
                 rr.add(ri, ri);
             }
         }
+        base += T * U;
+        load();
     }
     double acc[1] = {rr.get()};
-    grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
+    vec_grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
         s->pap = pap;
+        s->zr = s->nzr;
         s->rr = v[0];
         s->it += 1;
         s->done = (s->it >= s->max_iter) || (v[0] < s->tol2) || !(v[0] == v[0]);
     });
 }
 
-template <typename X>
-__global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_rz_kernel(long n, SolverScalars *s, const X *__restrict__ r, const X *__restrict__ z,
-                             double *partials, unsigned *counter, int init) {
-    if (!init && s->done) return;
+// <r, z>.  In the loop (RZ_PARTS) every CTA leaves its part and the direction update sums them: no last CTA holds the
+// launch up.  Before it, one launch stores the first <r, z> (RZ_FIRST), and for the plain CG ||r||^2 with it (RZ_INIT).
+enum RzMode { RZ_PARTS, RZ_FIRST, RZ_INIT };
+template <typename X, RzMode MODE>
+__global__ void __launch_bounds__(kEwThreads, kEwCtas) cg_rz_kernel(long n, SolverScalars *s, const X *__restrict__ r, const X *__restrict__ z,
+                             double *partials, unsigned *counter) {
+    if (MODE == RZ_PARTS && s->done) return;
     DotAcc<X> rz, rr;
     constexpr int U = ew_unroll<X>();
     const long T = (long)gridDim.x * blockDim.x;
@@ -109,17 +194,18 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_rz_kernel(long n,
         for (int u = 0; u < U; u++) {
             if (base + u * T < n) {
                 rz.add(rv[u], zv[u]);
-                if (init) rr.add(rv[u], rv[u]);
+                if (MODE == RZ_INIT) rr.add(rv[u], rv[u]);
             }
         }
     }
-    double acc[2] = {rz.get(), rr.get()};
-    grid_sum<2>(acc, partials, counter, [&](double (&v)[2]) {
-        s->nzr = s->zr;      // previous <r,z>, used by the p update
-        s->zr = v[0];
-        if (init) {
-            s->rr = v[1];
-            s->r0 = sqrt(v[1]);
+    constexpr int NV = MODE == RZ_INIT ? 2 : 1;
+    double acc[NV] = {rz.get()};
+    if (MODE == RZ_INIT) acc[NV - 1] = rr.get();
+    vec_grid_sum<NV, MODE == RZ_PARTS>(acc, partials, counter, [&](double (&v)[NV]) {
+        s->zr = s->nzr = v[0];
+        if (MODE == RZ_INIT) {
+            s->rr = v[NV - 1];
+            s->r0 = sqrt(v[NV - 1]);
             if (s->rel > 0.0) {
                 double t = s->rel * s->r0;
                 s->tol2 = fmax(s->tol2, t * t);
@@ -128,15 +214,16 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_rz_kernel(long n,
     });
 }
 
-// p = (zr_new / zr_old) p + z   (scal(a, p); axpy(1, z, p))
+// p = (zr_new / zr_old) p + z   (scal(a, p); axpy(1, z, p)); the new <r, z> from its parts, one per CTA of a grid as large
 template <typename X>
-__global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_p_kernel(long n, const SolverScalars *__restrict__ s, X *__restrict__ p, const X *__restrict__ z) {
+__global__ void __launch_bounds__(kEwThreads, kEwCtas) cg_p_kernel(long n, SolverScalars *s, X *__restrict__ p, const X *__restrict__ z,
+                                                                    const double *rz_part) {
     if (s->done) return;
-    const X bta = (X)(s->zr / s->nzr);
-    constexpr int U = ew_unroll<X>();
+    constexpr int U = ew_unroll<X, 3>();
     const long T = (long)gridDim.x * blockDim.x;
-    for (long base = blockIdx.x * (long)blockDim.x + threadIdx.x; base < n; base += T * U) {
-        X pv[U], zv[U];
+    long base = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    X pv[U], zv[U];
+    auto load = [&] {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
@@ -145,11 +232,20 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) cg_p_kernel(long n, 
                 zv[u] = z[i];
             }
         }
+    };
+    load();   // in flight while the scalar is summed
+    const X bta = (X)vec_scalar(rz_part, gridDim.x, 0.0, [&](double nzr) {
+        if (blockIdx.x == 0) s->nzr = nzr;   // the others read zr only
+        return nzr / s->zr;
+    });
+    while (base < n) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
-            if (i < n) p[i] = add_rn(mul_rn(bta, pv[u]), zv[u]);
+            if (i < n) p[i] = vec_axpy(zv[u], bta, pv[u]);
         }
+        base += T * U;
+        load();
     }
 }
 
@@ -242,12 +338,12 @@ static int cg_iteration(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, CgWork<X> &w, X *x, 
     const int *done = &s->done;
     int np = 0;
     HGB_TRY(spmv_A<V, X>(c, A, X(1), w.p, X(0), w.Ap, &s->pap, done, trans, &np));
-    cg_update_kernel<X><<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, s, w.p, w.Ap, x, w.r, c->partials,
+    cg_update_kernel<X><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, s, w.p, w.Ap, x, w.r, c->partials,
                                                                            c->counter, c->partials + kSpmvPartsOffset, np);
     X *z = M ? w.z : w.r;
     if (M) HGB_TRY(ilu_apply_internal(M, trans ? 'T' : 'N', w.r, w.z, done));
-    cg_rz_kernel<X><<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter, 0);
-    cg_p_kernel<X><<<ew_grid(c, n), 256, 0, c->stream>>>(n, s, w.p, z);
+    cg_rz_kernel<X, RZ_PARTS><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter);
+    cg_p_kernel<X><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.p, z, c->partials);
     return launch_check("cg iteration");
 }
 
@@ -833,7 +929,7 @@ static int cg_run(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, const X *b, X *x, double t
         X *z = M ? w.z : w.r;
         if (M && (st = ilu_apply_internal(M, trans ? 'T' : 'N', w.r, w.z, nullptr))) break;
         copy_kernel<X><<<ew_grid(c, n), 256, 0, c->stream>>>(n, z, w.p);
-        cg_rz_kernel<X><<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter, 1);
+        cg_rz_kernel<X, RZ_INIT><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter);
         if ((st = launch_check("cg init"))) break;
         if (cgp_eligible<V, X>(A, M, trans)) {   // small, L2-resident, unpreconditioned: one persistent launch
             st = cgp_run<V, X>(c, A, w, x, n, launches, hs);
@@ -1026,18 +1122,15 @@ __global__ void ru_init_kernel(SolverScalars *s, double tol2, double delta2, dou
 }
 
 // a = <r,z>/<p,Ap>; d += a p; r -= a Ap; ||r||^2; decide whether this iteration updates
-__global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) ru_step_kernel(long n, SolverScalars *s, const float *__restrict__ p, const float *__restrict__ Ap,
+__global__ void __launch_bounds__(kEwThreads, kEwCtas) ru_step_kernel(long n, SolverScalars *s, const float *__restrict__ p, const float *__restrict__ Ap,
                                float *__restrict__ d, float *__restrict__ r, double *partials, unsigned *counter,
                                const double *pap_part, int pap_n) {
     if (s->done) return;
-    const double pap = parts_sum(pap_part, pap_n, s->pap);
-    const float a = (float)(s->zr / pap);
-    const float ma = -a;
-    DotAcc<float> rr;
     constexpr int U = ew_unroll<float, 4>();
     const long T = (long)gridDim.x * blockDim.x;
-    for (long base = blockIdx.x * (long)blockDim.x + threadIdx.x; base < n; base += T * U) {
-        float pv[U], av[U], dv[U], rv[U];
+    long base = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    float pv[U], av[U], dv[U], rv[U];
+    auto load = [&] {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
@@ -1048,21 +1141,32 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) ru_step_kernel(long 
                 rv[u] = r[i];
             }
         }
+    };
+    load();   // in flight while the scalar is summed
+    // a = <r,z> / <p,Ap>; d += a p; r -= a Ap
+    double pap = 0.0;   // thread 0's
+    const float a = (float)vec_scalar(pap_part, pap_n, s->pap, [&](double v) { pap = v; return s->nzr / v; });
+    const float ma = -a;
+    DotAcc<float> rr;
+    while (base < n) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
             if (i < n) {
-                d[i] = __fadd_rn(dv[u], __fmul_rn(a, pv[u]));
-                const float ri = __fadd_rn(rv[u], __fmul_rn(ma, av[u]));
+                d[i] = vec_axpy(dv[u], a, pv[u]);
+                const float ri = vec_axpy(rv[u], ma, av[u]);
                 r[i] = ri;
                 rr.add(ri, ri);
             }
         }
+        base += T * U;
+        load();
     }
     double acc[1] = {rr.get()};
-    grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
+    vec_grid_sum<1>(acc, partials, counter, [&](double (&v)[1]) {
         const double rr = v[0];
         s->pap = pap;
+        s->zr = s->nzr;
         s->rr = rr;
         s->it += 1;
         s->rmax2 = fmax(s->rmax2, rr);
@@ -1108,14 +1212,14 @@ __global__ void ru_replace_kernel(long n, SolverScalars *s, const double *__rest
 }
 
 // p = beta p + z with beta = <r,z> / <r,z>_old, or p = z after a restart
-__global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) ru_p_kernel(long n, const SolverScalars *__restrict__ s, float *__restrict__ p,
-                            const float *__restrict__ z) {
+__global__ void __launch_bounds__(kEwThreads, kEwCtas) ru_p_kernel(long n, SolverScalars *s, float *__restrict__ p,
+                            const float *__restrict__ z, const double *rz_part) {
     if (s->done) return;
-    const float bta = s->restart ? 0.0f : (float)(s->zr / s->nzr);
-    constexpr int U = ew_unroll<float>();
+    constexpr int U = ew_unroll<float, 3>();
     const long T = (long)gridDim.x * blockDim.x;
-    for (long base = blockIdx.x * (long)blockDim.x + threadIdx.x; base < n; base += T * U) {
-        float pv[U], zv[U];
+    long base = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    float pv[U], zv[U];
+    auto load = [&] {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
@@ -1124,11 +1228,21 @@ __global__ void __launch_bounds__(kEwThreads, kEwCtasPerSm) ru_p_kernel(long n, 
                 zv[u] = z[i];
             }
         }
+    };
+    load();   // in flight while the scalar is summed
+    const float ratio = (float)vec_scalar(rz_part, gridDim.x, 0.0, [&](double nzr) {
+        if (blockIdx.x == 0) s->nzr = nzr;   // the others read zr only
+        return nzr / s->zr;
+    });
+    const float bta = s->restart ? 0.0f : ratio;
+    while (base < n) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const long i = base + u * T;
-            if (i < n) p[i] = __fadd_rn(__fmul_rn(bta, pv[u]), zv[u]);
+            if (i < n) p[i] = vec_axpy(zv[u], bta, pv[u]);
         }
+        base += T * U;
+        load();
     }
 }
 
@@ -1139,15 +1253,15 @@ static int ru_iteration(hgb_ctx *c, hgb_csr *A64, hgb_csr *Ai, hgb_ilu *M, CgWor
     const int *done = &s->done;
     int np = 0;
     HGB_TRY(spmv_A<V, float>(c, Ai, 1.0f, w.p, 0.0f, w.Ap, &s->pap, done, trans, &np));
-    ru_step_kernel<<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, w.p, w.Ap, d, w.r, c->partials, c->counter,
+    ru_step_kernel<<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.p, w.Ap, d, w.r, c->partials, c->counter,
                                                                       c->partials + kSpmvPartsOffset, np);
     ru_fold_kernel<<<ew_grid(c, n), 256, 0, c->stream>>>(n, s, b, d, x, r64);
     HGB_TRY(spmv_A<double, double>(c, A64, -1.0, x, 1.0, r64, nullptr, &s->ru_skip, trans));
     ru_replace_kernel<<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, r64, w.r, c->partials, c->counter);
     float *z = M ? w.z : w.r;
     if (M) HGB_TRY(ilu_apply_internal(M, trans ? 'T' : 'N', w.r, w.z, done));
-    cg_rz_kernel<float><<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter, 0);
-    ru_p_kernel<<<ew_grid(c, n), 256, 0, c->stream>>>(n, s, w.p, z);
+    cg_rz_kernel<float, RZ_PARTS><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter);
+    ru_p_kernel<<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.p, z, c->partials);
     return launch_check("ru iteration");
 }
 
@@ -1187,7 +1301,7 @@ static int ru_run(hgb_ctx *c, hgb_csr *A64, hgb_csr *Ai, hgb_ilu *M, const doubl
         if (M && (st = ilu_apply_internal(M, trans ? 'T' : 'N', w.r, w.z, nullptr))) break;
         copy_kernel<float><<<ew_grid(c, n), 256, 0, c->stream>>>(n, z, w.p);
         // <r,z> of the first direction (the rr slot keeps the FP64 residual)
-        cg_rz_kernel<float><<<reduce_grid(c, n, 256 * 4), 256, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter, 0);
+        cg_rz_kernel<float, RZ_FIRST><<<vec_grid(c, n), kEwThreads, 0, c->stream>>>(n, s, w.r, z, c->partials, c->counter);
         *launches += 5 + (M ? 2 : 0);
         if ((st = launch_check("ru init"))) break;
         if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal)) { st = cuda_fail(cudaGetLastError(), "begin capture"); break; }
