@@ -37,18 +37,18 @@ constexpr int kCapShort = 256, kCapLong = 384;   // entries of a staged tile (sp
 // tile size.  More CTAs leave less of the 256 KB for L1, which holds the gathered part of x and the
 // rows that are read directly, and fewer registers for gathers; fewer CTAs leave HBM idle.  Measured
 // (us; 128^3 7-point FP64 / FP32, graph Laplacians of 680k rows FP64 / FP32, 5 columns on 95x97x96 FP64 / FP32):
-//   FP64, 256 entries: 3 CTAs of 4 gathers 47.8; 2: 61.5; 6: 115; 3 of 8 (spills) 76.9.
+//   FP64, 256 entries: 3 CTAs of 8 gathers 45.3; of 4 gathers 47.8; 2 CTAs: 61.5; 4: 83.9 (spills); 6: 115.
 //   FP32, 256 entries: 4 CTAs of 8 gathers 28.7; of 4 gathers 31.1; 3 of 8 36.3.
-//   384 entries (rows of 9, which 256 would send to the direct path): FP64 2 CTAs 31.6, 3: 35.2; FP32 3 CTAs of
+//   384 entries (rows of 9, which 256 would send to the direct path): FP64 2 CTAs 30.8, 3: 35.2; FP32 3 CTAs of
 //   4 gathers 16.9, of 8 20.2, 2 of 4 18.5.
-//   columns: FP64 3 CTAs with one gather per column 68, with two and passes of 3 + 2 columns 78.7; FP32 3 CTAs
+//   columns: FP64 3 CTAs with one gather per column 66.6, with two and passes of 3 + 2 columns 78.7; FP32 3 CTAs
 //   with two 28.8, 4 with three 39.0.
 // Before (one shape for all, 4 gathers, passes of 4 columns with one): 55.4 / 29.1, 33.2 / 26.7, 108.6 / 43.1.
 template <typename X, int NC, int CAP>
 struct TileShape {
     static constexpr bool f64 = sizeof(X) == 8, wide = CAP > kCapShort;
     static constexpr int ctas = NC == 1 ? (f64 ? (wide ? 2 : 3) : (wide ? 3 : 4)) : (wide ? 2 : (f64 && NC == 2 ? 4 : 3));
-    static constexpr int gathers = NC == 1 ? (f64 || wide ? 4 : 8) : (f64 ? (NC == 2 ? 2 : 1) : (NC == 2 ? 6 : 12 / NC));
+    static constexpr int gathers = NC == 1 ? (wide ? 4 : 8) : (f64 ? (NC == 2 ? 2 : 1) : (NC == 2 ? 6 : 12 / NC));
 };
 
 // acc += v * x in the mode's rounding
@@ -179,6 +179,8 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
                 // across the warp; not for several columns of a direct tile, whose long rows leave few lanes active
                 auto sum = [&](const V *vp, const int *ip, auto staged) {
                     constexpr bool in_step = decltype(staged)::value || NC == 1;
+                    // FP64 values stay in shared memory until they are multiplied: registers for gathers
+                    constexpr bool late = decltype(staged)::value && sizeof(X) == 8;
                     constexpr int GW = TileShape<X, NC, CAP>::gathers;
                     const int upto = in_step ? most : cnt;
                     for (int j0 = 0; j0 < upto; j0 += GW) {
@@ -195,7 +197,7 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
                                     v = __ldg(vp + j0 + q);
                                     col = __ldg(ip + j0 + q);
                                 }
-                                vv[q] = Val<V>::get(v);
+                                if (!late) vv[q] = Val<V>::get(v);
                                 const X *xp = xc + col;
 #pragma unroll
                                 for (int m = 0; m < NC; m++)
@@ -207,7 +209,7 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
 #pragma unroll
                                 for (int m = 0; m < NC; m++)
                                     if (NC == 1 || !in_step || spmv_uniform(m < nc, X(0)))
-                                        if (j0 + q < cnt) acc[m] = spmv_acc<EXACT>(acc[m], vv[q], xv[q][m]);
+                                        if (j0 + q < cnt) acc[m] = spmv_acc<EXACT>(acc[m], late ? Val<V>::get(vp[j0 + q]) : vv[q], xv[q][m]);
                             }
                     }
                 };
