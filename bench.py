@@ -189,7 +189,7 @@ def _events_ms(stream, fn, steps, warm, flush=None):
 def other_workloads(E, eng, dev, stream, flush, peak, steps=3, warm=2):
     """The path's other workloads, timed on the device (CUDA events, setup excluded): CG on the 256^2
     Poisson system, ILU(0)-GMRES(30) on the 96^3 convection-diffusion operator (FP64 and mixed),
-    the 4,096 independent systems in one persistent launch, and the 512^2 differentiable solve
+    the 4,096 independent systems in persistent launches, and the 512^2 differentiable solve
     (forward and adjoint).  Each entry reports its time, iterations and residual."""
     import torch
     from hala_gb300 import problems as P
@@ -252,7 +252,7 @@ def other_workloads(E, eng, dev, stream, flush, peak, steps=3, warm=2):
     del A64, M64, A32, M32
 
     # 4,096 independent Erdos-Renyi Laplacians (n_i log-uniform in [64, 4096]), FP32 CG with FP64
-    # refinement to 1e-8 per system, one persistent launch replayed from a CUDA graph
+    # refinement to 1e-8 per system, persistent launches side by side replayed from a CUDA graph
     S = 4096
     sp_, p, i, v = P.er_laplacian_batch(S, 64, 4096, seed=4)
     nt = len(p) - 1
@@ -274,16 +274,19 @@ def other_workloads(E, eng, dev, stream, flush, peak, steps=3, warm=2):
     it = iters.cpu().numpy().astype(np.int64)
     ni = np.diff(sp_).astype(np.int64)
     nnz_i = (p[sp_[1:]] - p[sp_[:-1]]).astype(np.int64)
-    # algorithmic bytes: every inner iteration streams its system's matrix (FP32 values, int32
-    # columns and row pointers) and touches x and b once per system in FP64
-    mat_bytes = float(np.sum(it * (8 * nnz_i + 4 * (ni + 1)))) + float(np.sum(16 * ni))
-    gbs = mat_bytes / (msb * 1e-3) / 1e9
+    # bytes that the batch cannot do without (the matrix once, x and b in FP64), and the rate at which a
+    # form whose inner iterations stream their matrix would have to read to take the same time (systems
+    # that fit are kept on chip)
+    must = float(8 * len(i) + 4 * (nt + 1) + 16 * nt)
+    streamed = float(np.sum(it * (8 * nnz_i + 4 * (ni + 1)))) + float(np.sum(16 * ni))
+    gbs = must / (msb * 1e-3) / 1e9
     out["batch_4096"] = {"ms_per_batch": msb, "systems_per_s": S * 1e3 / msb, "rows": nt, "nnz": len(i),
                          "launch_shape": {"block_threads": shape[0], "warp_max_n": shape[1]},
                          "max_rel_residual": float(rel.max()), "iterations_total": int(it.sum()),
-                         "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s",
-                                      "frac": gbs / peak, "algorithmic_bytes": mat_bytes,
-                                      "bytes": "sum over systems of inner iterations x (8 nnz_i + 4 (n_i + 1)) + 16 n_i"}}
+                         "roofline": {"bound": "on-chip gathers and reductions", "achieved": gbs, "peak": peak,
+                                      "unit": "GB/s", "frac": gbs / peak, "algorithmic_bytes": must,
+                                      "bytes": "8 nnz + 4 (n + 1) + 16 n",
+                                      "streamed_equivalent_gbs": streamed / (msb * 1e-3) / 1e9}}
     del B
 
     # 512^2 variable-coefficient diffusion: forward mixed ILU(0)-PCG (FP32 PCG, FP64 reliable updates)
@@ -678,7 +681,7 @@ def main():
             "achieved": ach_ilu, "peak": peak, "unit": "GB/s", "frac": ach_ilu / peak,
             "traffic": prof.get("ilu_apply_bf16_bytes"), "peak_source": peak_src,
             "algorithmic_bytes": ib16, "ms_per_launch": t_ilu16 / 2, "ms_per_apply": t_ilu16}
-    spmv = {"kernel": "spmv_warp_kernel", "f64": {"ms": t_spmv64, "gbs": vb64 / (t_spmv64 * 1e-3) / 1e9,
+    spmv = {"kernel": "spmv_tile_kernel", "f64": {"ms": t_spmv64, "gbs": vb64 / (t_spmv64 * 1e-3) / 1e9,
                                                "frac": vb64 / (t_spmv64 * 1e-3) / 1e9 / peak, "bytes": vb64,
                                                "traffic": prof.get("spmv_f64_bytes")},
             "f32": {"ms": t_spmv32, "gbs": spmv_bytes(n, nnz, 4, 4) / (t_spmv32 * 1e-3) / 1e9,

@@ -46,15 +46,6 @@ struct Schedule {
     }
 };
 
-__device__ __forceinline__ int ld_relaxed_int(const int *p) {
-    int v;
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed_int(int *p, int v) {
-    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Bounded wait for a row's completion flag (>= 0): lane 0 polls, with pauses that grow with the wait (all
 // the chunks of the matrix that fit are resident, most of them waiting); its acquire and the warp
 // barrier order the other lanes' reads of that row behind it.

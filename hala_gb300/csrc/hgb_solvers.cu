@@ -1713,7 +1713,8 @@ static int gmres_run(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, int restart, const X *b
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     const int pre = M ? 2 : 1;          // ILU: L and U sweeps; none: a copy
-    const long long per_cycle = 6 + pre + (long long)restart * (4 + pre);
+    long long per_cycle = 6 + pre + (long long)restart * (3 + pre);
+    for (int k = 0; k < restart; k++) per_cycle += k / 32 + 1;   // gm_dots_launch's groups
     int rc = HGB_OK;
     do {
         if (ws_alloc(c, &t, n) || ws_alloc(c, &r, n) || ws_alloc(c, &W, (size_t)n * restart) ||

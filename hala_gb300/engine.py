@@ -596,8 +596,10 @@ def solve_ru_pcg_mixed(engine, tol, pntr_h, indx_h, vals_h, ilu_inner, b_h, x_h,
 
 
 class gpu_batch:
-    """Many independent SPD systems (block-diagonal CSR, FP32 values) solved in one persistent
-    launch with FP64 refinement (hgb_batch_*; no reference counterpart)."""
+    """Many independent SPD systems (block-diagonal CSR, FP32 values) solved in a few persistent launches
+    side by side with FP64 refinement (hgb_batch_*; no reference counterpart).  A system that fits is kept on
+    chip for its iterations; the configuration (threads per CTA, largest system of a single warp), which
+    autotune() times, is for the others."""
 
     def __init__(self, engine, sys_ptr, pntr, indx, vals):
         _need(sys_ptr, torch.int32, "sys_ptr"); _need(pntr, torch.int32, "pntr"); _need(indx, torch.int32, "indx")

@@ -349,7 +349,8 @@ int hgb_mixed_ru_pcg_solve(hgb_ctx *ctx, int n, int nnz, const int *pntr_host, c
 
 /* ------------------------------------------ batched independent systems (no reference
  * counterpart: the reference's batch is one matrix with many right-hand sides) -------------- */
-/* Launch shape of the batched solver: threads per CTA (128, 256 or 512) and the largest system
+/* Launch shape of the batched solver for systems that do not fit on chip (those that do are solved by kernels
+ * whose shape follows from their size): threads per CTA (128, 256 or 512) and the largest system
  * solved by a single warp (larger systems get a whole CTA). */
 typedef struct hgb_batch_config { int block_threads; int warp_max_n; } hgb_batch_config;
 /* A batch of S independent systems stored as one block-diagonal CSR with FP32 values and global
@@ -359,7 +360,7 @@ int hgb_batch_create(hgb_ctx *ctx, int num_systems, const int *sys_ptr, int n_to
                      const int *pntr, const int *indx, const float *vals, hgb_batch **batch);
 int hgb_batch_set_config(hgb_batch *batch, const hgb_batch_config *cfg);
 int hgb_batch_get_config(hgb_batch *batch, hgb_batch_config *cfg);
-/* Solves every system in ONE persistent kernel launch, replayed from a CUDA graph: FP32 CG
+/* Solves every system in a few persistent kernel launches that run side by side, replayed from a CUDA graph: FP32 CG
  * (inner relative tolerance inner_rtol, at most max_inner iterations) inside FP64 refinement
  * until ||b_s - A_s x_s|| <= rtol ||b_s|| for each system s (at most max_outer sweeps).  x holds
  * the initial guesses.  iters[S] / relres[S] (device, optional) receive per-system totals. */
