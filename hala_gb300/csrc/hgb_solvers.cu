@@ -12,6 +12,7 @@
 #include "hgb_complex.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cmath>
 #include <vector>
@@ -827,16 +828,22 @@ struct CgpShape {
     int grid = 0, rpt = 0, cluster = 0;
 };
 template <typename V, typename X, bool EXACT>
-static CgpShape cgp_shape(long n) {
+static CgpShape cgp_shape(const hgb_ctx *c, long n) {
+    static std::atomic<int> fit[64][5][kCgpCluster + 1];   // co-resident clusters + 1, by device, rows per thread, size
     CgpShape sh;
+    if (c->device < 0 || c->device >= 64) return sh;
     for (int rpt : {1, 2, 4, 0})
         for (int cluster = kCgpCluster; cluster > 1; cluster /= 2) {
-            cudaLaunchAttribute at[2];
-            const cudaLaunchConfig_t cfg = cgp_config(cluster, cluster, nullptr, at);
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, cgp_kernel<V, X, EXACT>(rpt), &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                return sh;
+            std::atomic<int> &known = fit[c->device][rpt][cluster];
+            int clusters = known.load() - 1;
+            if (clusters < 0) {
+                cudaLaunchAttribute at[2];
+                const cudaLaunchConfig_t cfg = cgp_config(cluster, cluster, nullptr, at);
+                if (cudaOccupancyMaxActiveClusters(&clusters, cgp_kernel<V, X, EXACT>(rpt), &cfg) != cudaSuccess) {
+                    cudaGetLastError();
+                    return sh;
+                }
+                known = clusters + 1;
             }
             clusters = std::min(clusters, 16 * kCgpMail);
             const long rows = (rpt ? rpt : 4) * (long)kCgpThreads * cluster;   // of a cluster
@@ -861,7 +868,7 @@ static bool cgp_eligible(hgb_csr *A, hgb_ilu *M, bool trans) {
 template <typename V, typename X>
 static int cgp_run(hgb_ctx *c, hgb_csr *A, CgWork<X> &w, X *x, long n, long long *launches, SolverScalars &hs) {
     const bool exact = (c->spmv_mode == HGB_SPMV_EXACT);
-    const CgpShape sh = exact ? cgp_shape<V, X, true>(n) : cgp_shape<V, X, false>(n);
+    const CgpShape sh = exact ? cgp_shape<V, X, true>(c, n) : cgp_shape<V, X, false>(c, n);
     const int G = sh.grid;
     if (G < 1) return fail(HGB_ERR_UNSUPPORTED, "persistent cg: no co-resident grid");
     CgpWord *mail = nullptr;   // two sets of an entry (two words) per CTA and cluster
