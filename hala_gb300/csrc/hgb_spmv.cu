@@ -3,7 +3,7 @@
 // handshake between warps), then every lane sums its row from shared memory, gathering x from
 // global memory (L1 / L2).  The copies of the next kStages - 1 tiles and the row pointers of the tile
 // after them are in flight while a tile is summed.  Tiles of more than CAP entries read their rows
-// directly.
+// directly, the longest of them by the whole warp (spmv_wide_row).
 //
 // Two arithmetic modes, chosen per context (hgb_ctx_set_spmv_mode):
 //  - exact: each row summed in column order with separately rounded multiply and add, the
@@ -99,6 +99,96 @@ __device__ __forceinline__ void spmv_dot_epilogue(double d, double *partials, un
     }
 }
 
+// A long row among short ones (in a tile that is not staged): alone in its lane it is bound by the latency of column
+// then x, a few entries at a time.  spmv_wide_row takes 32 of its entries at once, with the next 32 and the
+// columns after them in flight, and every lane adds them in column order (the products of EXACT are formed before,
+// one per lane), so the sum is the single lane's bit for bit, at the FP64 unit's 64 cycles per entry.  The rows of a tile
+// then come one after another: spmv_wide takes a row while it has a third (FP64) or an eighth (FP32) of the entries
+// left, by the cost of an entry alone in its lane (about 190 cycles) and here (64; FP32 about 25).
+// Such tiles wait for the end of the kernel, in a function of their own: inlined, or at their place among the
+// staged tiles, they cost the staged FP64 product 45.8 -> 49 to 54 us.
+// Rows of 7 with 0.2 % of 3000, FP64 / FP32: 100k rows 646 / 285 -> 302 / 109 us; of 300, 400k rows 115 / 79 -> 76 / 36.
+// Four FP64 columns at 100k rows: 1637 -> 1174.  FP32 columns keep the lanes' own sums: the test alone took four
+// columns of staged rows 189 -> 199 us (2M rows of 7).  The staged single-column products: 128^3 FP64 45.9 -> 46.2 us,
+// 2M rows of 7 FP64 62.1 / FP32 47.8 -> 62.1 / 49.8.
+template <typename X>
+__device__ __forceinline__ bool spmv_wide(int longest, int left) {
+    return longest >= 64 && longest >= left / (sizeof(X) == 8 ? 3 : 8);
+}
+template <typename V, bool EXACT>
+__device__ __forceinline__ typename Val<V>::X spmv_wide_row(const V *vp, const int *ip, unsigned len, const typename Val<V>::X *x) {
+    using X = typename Val<V>::X;
+    const unsigned lane = threadIdx.x & 31;
+    auto at = [&](unsigned j) { return min(j + lane, len - 1); };   // past the end: the last entry, not summed
+    X acc = X(0), v = Val<V>::get(__ldg(vp + at(0))), xv = __ldg(x + __ldg(ip + at(0)));
+    int col = __ldg(ip + at(32));
+    for (unsigned j = 0; j < len; j += 32) {
+        const X v1 = Val<V>::get(__ldg(vp + at(j + 32))), x1 = __ldg(x + col);
+        col = __ldg(ip + at(j + 64));
+        if (EXACT) xv = mul_rn(v, xv);
+        const int few = (int)min(len - j, 32u);
+#pragma unroll 4
+        for (int q = 0; q < few; q++) {
+            const X xq = __shfl_sync(0xffffffffu, xv, q);
+            acc = EXACT ? add_rn(acc, xq) : spmv_acc<false>(acc, __shfl_sync(0xffffffffu, v, q), xq);
+        }
+        v = v1;
+        xv = x1;
+    }
+    return acc;
+}
+
+template <typename V, int CAP, bool DOT, bool EXACT>
+__device__ __noinline__ DotAcc<typename Val<V>::X>
+spmv_wide_tiles(int tb, int te, int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx,
+                const V *__restrict__ vals, int nrhs, int end_mode, typename Val<V>::X alpha,
+                const typename Val<V>::X *__restrict__ x, long ldx, typename Val<V>::X beta,
+                typename Val<V>::X *__restrict__ y, long ldy, DotAcc<typename Val<V>::X> dacc) {
+    using X = typename Val<V>::X;
+    const int lane = threadIdx.x & 31;
+    for (int k = tb; k < te; k++) {
+        const int row = k * 32 + lane;
+        const int ps = __ldg(pntr + min(row, n_rows)), pe = __ldg(pntr + min(row + 1, n_rows));
+        const int total = __shfl_sync(0xffffffffu, pe, 31) - __shfl_sync(0xffffffffu, ps, 0);
+        if (total <= CAP || !spmv_wide<X>(__reduce_max_sync(0xffffffffu, pe - ps), total)) continue;
+        for (int m = 0; m < nrhs; m++) {
+            const X *xc = x + (long)m * ldx;
+            X acc = X(0);
+            int n = pe - ps, longest = __reduce_max_sync(0xffffffffu, n), left = total;
+            while (spmv_wide<X>(longest, left)) {
+                const int r = __ffs(__ballot_sync(0xffffffffu, n == longest)) - 1;
+                const int base = __shfl_sync(0xffffffffu, ps, r);
+                const X sum = spmv_wide_row<V, EXACT>(vals + base, indx + base, (unsigned)longest, xc);
+                if (lane == r) {
+                    acc = sum;
+                    n = 0;
+                }
+                left -= longest;
+                longest = __reduce_max_sync(0xffffffffu, n);
+            }
+            for (int j0 = 0; j0 < n; j0 += 4) {
+                X xv[4], vv[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (j0 + q < n) {
+                        vv[q] = Val<V>::get(__ldg(vals + ps + j0 + q));
+                        xv[q] = __ldg(xc + __ldg(indx + ps + j0 + q));
+                    }
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (j0 + q < n) acc = spmv_acc<EXACT>(acc, vv[q], xv[q]);
+            }
+            if (row < n_rows) {
+                X *yp = y + (long)m * ldy + row;
+                const X out = spmv_out<EXACT>(end_mode, alpha, acc, beta, yp);
+                *yp = out;
+                if (DOT) dacc.add(__ldg(x + row), out);
+            }
+        }
+    }
+    return dacc;
+}
+
 // Y = alpha * A X + beta * Y for nrhs column-major columns (x column c at x + c * ldx), cols <= NC of them per
 // pass over a staged tile (the matrix is read once); optionally <x, y> (one column, square A; DOT as
 // spmv_dot_epilogue).  Every column is summed in column order in the mode's rounding, so each column
@@ -124,6 +214,7 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
     const int per = (ntiles + nwarps - 1) / nwarps;
     const int tb = (blockIdx.x * (kWarpBlock / 32) + wib) * per;
     const int te = min(ntiles, tb + per);
+    int wide = te;    // tb once a tile of this warp is left for the end (spmv_wide_tiles)
     DotAcc<X> dacc;   // fused <x, y> (per-thread partial)
 
     // lane's row pointers of tile k (loads only; nothing waits on them yet)
@@ -165,10 +256,16 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
             load_ptrs(k + ST, ps[ST], pe[ST]);
             cp_async_wait<ST - 1>();   // tile k has landed
             __syncwarp();
-            const int row = k * 32 + lane;
+            int row = k * 32 + lane;
             const int first = __shfl_sync(0xffffffffu, ps[0], 0), end = __shfl_sync(0xffffffffu, pe[0], 31);
-            const int cnt = pe[0] - ps[0];
-            const int most = __reduce_max_sync(0xffffffffu, cnt);
+            int cnt = pe[0] - ps[0];
+            int most = __reduce_max_sync(0xffffffffu, cnt);
+            if ((NC == 1 || sizeof(X) == 8) &&
+                __builtin_expect(end - first > CAP && spmv_wide<X>(most, end - first), 0)) {   // no entries, no row to write
+                wide = tb;
+                row = n_rows;
+                cnt = most = 0;
+            }
             for (int c0 = 0; c0 < (NC == 1 ? 1 : nrhs); c0 += cols) {
                 const int nc = NC == 1 ? 1 : min(cols, nrhs - c0);
                 const X *xc = x + (long)c0 * ldx;
@@ -240,6 +337,9 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
         }
     }
     cp_async_wait<0>();
+    if (wide < te)   // the tiles that were left out
+        dacc = spmv_wide_tiles<V, CAP, DOT != 0, EXACT>(wide, te, n_rows, pntr, indx, vals, NC == 1 ? 1 : nrhs, end_mode, alpha, x, ldx,
+                                                        beta, y, ldy, dacc);
     if (DOT) spmv_dot_epilogue<DOT>(dacc.get(), partials, counter, dot_out);
 }
 template <typename V, int CAP>
