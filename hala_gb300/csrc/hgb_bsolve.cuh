@@ -31,6 +31,7 @@ __host__ __device__ constexpr int bs_slots_max(int xsize, int nonunit) {
     return (kBsSmemMax - bs_ring_bytes(xsize, nonunit)) / xsize;
 }
 constexpr int kBsNoSlot = 0xFFFF;
+constexpr int kBsMaxStrip = 16384;   // rows of a strip (the packets count them in 16 bits)
 // packet flags (first piece, .w): bits 0-7 blocks to the one whose slot (first piece, .z, high half) takes
 // the row's value, in shared memory (push) or through its mailbox (mail)
 constexpr int kBsExt = 1 << 8, kBsReset = 1 << 9, kBsPush = 1 << 10;

@@ -120,9 +120,10 @@ struct Scratch {   // one thread's working arrays
 // line is read off the entries' distances: the largest one at most half the bandwidth (the
 // second stride of a 3D grid), or the bandwidth itself where that is the stride of a 2D grid.
 // Where the bandwidth is a whole number of lines (a grid plane), strips are cut evenly inside it, so
-// that every plane has the same ones.
+// that every plane has the same ones.  No strip has more than kBsMaxStrip rows: a packet holds its row's
+// place in the strip in 16 bits, and a strip's own rows have to fit the slots.
 static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool &deep) {
-    constexpr int kMaxT = 16384, kMinT = 512;
+    constexpr int kMaxT = kBsMaxStrip, kMinT = 512;
     deep = d2 >= 8;
     const int u = deep ? d2 : std::max(bw, 1);
     cut.assign(1, 0);
@@ -131,7 +132,7 @@ static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool
     } else {
         T = u > kMaxT ? kMaxT : (int)std::min<long>(32L * u, (long)(kMaxT / u) * u);
         if (T < kMinT) T = (kMinT + T - 1) / T * T;
-        if (deep && bw % u == 0 && bw / u >= 16 && bw <= n) {
+        if (deep && u <= kMaxT && bw % u == 0 && bw / u >= 16 && bw <= n) {
             const int ny = bw / u, k = (bw + T - 1) / T, lines = (ny + k - 1) / k;
             T = lines * u;
             for (long p = 0; p < n; p += bw)
@@ -423,9 +424,12 @@ struct Sweep {
     // Others (2D grids): each strip runs a whole strip's width of steps behind the one before it, so
     // hand-overs are few and a CTA's strips only slow one another; one strip per CTA until they
     // no longer fit a cluster of 16 CTAs.
-    void cut_blocks(const std::function<int(int)> &cluster_of) {
+    int cut_blocks(const std::function<int(int)> &cluster_of) {
         bs_strips(n, bw, d2, cut, T, deep);
         nstrips = (int)cut.size() - 1;
+        for (int k = 0; k < nstrips; k++)
+            if (cut[k + 1] - cut[k] > kBsMaxStrip)
+                return fail(HGB_ERR_UNSUPPORTED, "triangular plan: a strip of %d rows", cut[k + 1] - cut[k]);
         const int by_rows = std::max(1, (xsize == 8 ? 20480 : 32768) / T);
         spb = std::min({kBsW, by_rows, deep ? kBsW : std::max(1, (nstrips + 15) / 16)});
         nblk = (nstrips + spb - 1) / spb;
@@ -438,6 +442,7 @@ struct Sweep {
         P.pk.resize(n);
         P.pk_of_row.resize(n);
         P.watched.assign(n, 0);
+        return HGB_OK;
     }
     void block(int b, Scratch &scr) {
         bs_plan_block(R, rev, np, xsize, cap, bw, cut.data(), b * spb, std::min(nstrips, (b + 1) * spb), P.pk.data(),
@@ -596,7 +601,7 @@ int bs_plan_sweeps(int n, const int *pntr, const int *indx, const int *diag, int
     phase(ranges, [](Sweep &s, int k) { s.scan(k, s.bw / 2); });
     for (Sweep &s : S) {
         s.d2 = s.widest();
-        s.cut_blocks(cluster_of);
+        HGB_TRY(s.cut_blocks(cluster_of));
     }
     {
         std::vector<Scratch> scr(16);
