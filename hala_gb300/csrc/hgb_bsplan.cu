@@ -147,7 +147,8 @@ static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool
     cut.push_back(n);
 }
 
-// One block: its strips' steps, slots, chunks and packets (into pk from position P0 on).
+// One block: its strips' steps, slots, chunks and packets (into pk from position P0 on).  Where the block's own
+// rows take more than cap slots, only B.nslots is set.
 static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, int bw, const int *cut, int s0, int s1,
                           int4 *pk, int *pk_of_row, BlockOut &B, Scratch &S) {
     const int P0 = cut[s0], P1 = cut[s1], rows = P1 - P0, ns = s1 - s0;
@@ -237,6 +238,8 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
             for (int r = S.head[st]; r >= 0; r = S.next[r]) S.free_q.push_back(S.tslot[r]);
         }
     }
+    B.nslots = 1 + nf + ntemp;
+    if (B.nslots > cap) return;   // its own rows do not fit: the sweep is cut into smaller blocks
     // ---- the halo in the order of its first use; the steps' times order the fetches
     S.window.resize(std::max<size_t>(S.window.size(), std::min(P0, bw)), 0);   // by distance from the block
     S.touched.clear();
@@ -245,12 +248,13 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
     for (int k = 0; k < ns; k++) {
         const int p0 = cut[s0 + k];
         // a strip's halo starts a 16-byte unit of the mailbox: a unit with values of two strips would
-        // hold the first values of one until the last ones of the other are in
-        while ((1 + nf + nh) % (16 / xsize)) {
+        // hold the first values of one until the last ones of the other are in (without room for that, the
+        // strip has no halo slots of its own)
+        while ((1 + nf + nh) % (16 / xsize) && 1 + nf + nh + ntemp < cap) {
             B.halo.push_back({-1, 1 + nf + nh, INT_MAX});
             nh++;
         }
-        B.seg[k] = 1 + nf + nh;
+        B.seg[k] = (1 + nf + nh + 16 / xsize - 1) / (16 / xsize) * (16 / xsize);
         for (int st = S.strip_steps[k]; st < S.strip_steps[k + 1]; st++) {
             int t = st > S.strip_steps[k] ? S.time[st - 1] + 1 : 0;
             for (int pass = 0; pass < 2; pass++) {   // the step's time, then its halo
@@ -383,7 +387,7 @@ struct Sweep {
     BsPlan &P;
     std::vector<int> mx, wide, cut;
     int bw = 0, d2 = 0, T = 0, nstrips = 0, spb = 1, nblk = 0, cl = 1, runs = 0;
-    bool deep = false;
+    bool deep = false, planned = false;
     std::vector<BlockOut> out;
     std::vector<std::vector<int2>> watch;
     std::vector<std::vector<Halo>> far;   // entries from earlier clusters
@@ -432,16 +436,31 @@ struct Sweep {
                 return fail(HGB_ERR_UNSUPPORTED, "triangular plan: a strip of %d rows", cut[k + 1] - cut[k]);
         const int by_rows = std::max(1, (xsize == 8 ? 20480 : 32768) / T);
         spb = std::min({kBsW, by_rows, deep ? kBsW : std::max(1, (nstrips + 15) / 16)});
-        nblk = (nstrips + spb - 1) / spb;
-        cl = cluster_of(nblk);
-        runs = (nblk + cl - 1) / cl;
-        out.resize(nblk);
-        watch.resize(nblk);
-        far.resize(nblk);
-        mailed.assign(nblk, 0);
         P.pk.resize(n);
         P.pk_of_row.resize(n);
         P.watched.assign(n, 0);
+        group(cluster_of);
+        return HGB_OK;
+    }
+    // spb strips to a block
+    void group(const std::function<int(int)> &cluster_of) {
+        nblk = (nstrips + spb - 1) / spb;
+        cl = cluster_of(nblk);
+        runs = (nblk + cl - 1) / cl;
+        out.assign(nblk, BlockOut());
+        watch.resize(nblk);
+        far.resize(nblk);
+        mailed.assign(nblk, 0);
+    }
+    // after the blocks are planned: whether all of them fit.  Where one does not, the sweep takes blocks of
+    // half as many strips (one strip fits: kBsMaxStrip rows are fewer than the slots).
+    int settle(const std::function<int(int)> &cluster_of) {
+        planned = true;
+        for (const BlockOut &B : out) planned = planned && B.nslots <= cap;
+        if (planned) return HGB_OK;
+        if (spb == 1) return fail(HGB_ERR_UNSUPPORTED, "triangular plan: a strip's rows exceed the slots");
+        spb /= 2;
+        group(cluster_of);
         return HGB_OK;
     }
     void block(int b, Scratch &scr) {
@@ -506,6 +525,7 @@ struct Sweep {
             nslots = std::max(nslots, B.nslots);
             nflag = std::max(nflag, B.nflag);
         }
+        if (nslots > cap) return fail(HGB_ERR_UNSUPPORTED, "triangular plan: a block needs %d slots of %d", nslots, cap);
         const Base &tot = base[nblk];
         if (tot.unit > INT_MAX || tot.mail > INT_MAX || tot.ext > INT_MAX)
             return fail(HGB_ERR_UNSUPPORTED, "triangular plan: packed arrays exceed 2^31 entries");
@@ -607,12 +627,17 @@ int bs_plan_sweeps(int n, const int *pntr, const int *indx, const int *diag, int
         std::vector<Scratch> scr(16);
         std::vector<std::atomic<int>> used(16);
         for (auto &u : used) u = 0;
-        phase(blocks, [&](Sweep &s, int b) {
-            int w = 0;   // at most 16 threads take items
-            for (int expect = 0; !used[w].compare_exchange_strong(expect, 1); expect = 0) w = (w + 1) % 16;
-            s.block(b, scr[w]);
-            used[w] = 0;
-        });
+        auto left = [&] { return std::any_of(S.begin(), S.end(), [](const Sweep &s) { return !s.planned; }); };
+        while (left()) {
+            phase([](Sweep &s) { return s.planned ? 0 : s.nblk; }, [&](Sweep &s, int b) {
+                int w = 0;   // at most 16 threads take items
+                for (int expect = 0; !used[w].compare_exchange_strong(expect, 1); expect = 0) w = (w + 1) % 16;
+                s.block(b, scr[w]);
+                used[w] = 0;
+            });
+            for (Sweep &s : S)
+                if (!s.planned) HGB_TRY(s.settle(cluster_of));
+        }
     }
     phase([](Sweep &s) { return s.runs; }, [](Sweep &s, int r) { s.halos(r); });
     phase([](Sweep &) { return 1; }, [](Sweep &s, int) { s.mails(); });

@@ -25,7 +25,7 @@ def values(pntr, indx, diag, rng):
     return v
 
 
-@pytest.mark.parametrize("name", ["two_fields_260x260x16", "grid_70000x16x2"])
+@pytest.mark.parametrize("name", ["two_fields_260x260x16", "grid_70000x16x2", "grid_16384x16x3", "random_100000", "arrows_420_last"])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 def test_apply_bit_exact(eng, rng, name, dtype):
     p, i, d = plan.CASES[name]()

@@ -1,7 +1,8 @@
 """The host's plan of the triangular sweeps, checked without a GPU by tests/cpp/sweep_plan_check.cu: every packet
 names its own row, all slots fit a CTA's shared memory, and a sweep over row numbers finds each entry where its
 code says.  The patterns are at the plan's limits: grid lines longer than a strip and than 65,536 rows (a
-packet's row offset has 16 bits)."""
+packet's row offset has 16 bits), blocks with more rows of other blocks than slots, blocks whose own rows need
+more slots than there are."""
 import ctypes
 import os
 import subprocess
@@ -70,15 +71,29 @@ def random(n, degree):
     return csr(sp.coo_matrix((np.ones(m), (rng.integers(0, n, m), rng.integers(0, n, m))), shape=(n, n)))
 
 
+def arrows(n, m, last):
+    """blocks of m rows with a full first (or last) row and column"""
+    i = np.arange(n)
+    hub = np.minimum(i // m * m + (m - 1 if last else 0), n - 1)
+    return csr(sp.coo_matrix((np.ones(n), (i, hub)), shape=(n, n)))
+
+
 CASES = {
     "grid_33x17x5": lambda: grid(33, 17, 5),
     "grid_64x65x30": lambda: grid(64, 65, 30),
     "grid_256x160x40": lambda: grid(256, 160, 40),
+    "grid_16384x16x3": lambda: grid(16384, 16, 3),
     "grid_16385x16x3": lambda: grid(16385, 16, 3),
     "plane_of_65536": lambda: two_fields(256, 256, 16),
     "grid_70000x16x2": lambda: grid(70000, 16, 2),
     "two_fields_260x260x16": lambda: two_fields(260, 260, 16),
     "random_30000": lambda: random(30000, 12),
+    "random_60000": lambda: random(60000, 6),
+    "random_100000": lambda: random(100000, 12),
+    "random_300000": lambda: random(300000, 3),
+    "arrows_420_first": lambda: arrows(100800, 420, False),
+    "arrows_420_last": lambda: arrows(100800, 420, True),
+    "arrows_5": lambda: arrows(120000, 5, True),
 }
 
 
