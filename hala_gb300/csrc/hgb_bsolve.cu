@@ -126,9 +126,8 @@ __device__ __forceinline__ unsigned bs_cluster_size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void bs_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void bs_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void bs_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t bs_peer(uint32_t local, unsigned rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
@@ -302,6 +301,7 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
         if (t == 0) atomicOr(A.err, DEV_ERR_CSR);
         return;
     }
+    bs_cluster_arrive();   // a peer's shared memory is written only after this CTA has started
     const int sw = warp < W * K ? warp : 0;   // solver warp
     unsigned char *ring = smem + (size_t)sw * (D * CB);
     X *rhs = (X *)(smem + (size_t)(W * K) * (D * CB)) + sw * (RA * 32) + lane;
@@ -317,17 +317,19 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
     unsigned wpar = 0;
     for (int round = 0;; round++) {
         // clusters take tickets; rank r of the cluster with ticket q solves block q * ncl + r.  The
-        // first barrier: every CTA of the cluster is done with the previous round (its slots and its
+        // first barrier: every CTA of the cluster runs and is done with the previous round (its slots and its
         // peers' are read); the second: the ticket and the pending slots are visible to all.
         __syncwarp();
-        if (round) bs_cluster_sync();
+        if (round) bs_cluster_arrive();
+        bs_cluster_wait();
         if (t == 0 && rank == 0) {
             const int q = atomicAdd(A.ticket, 1);
             for (unsigned r = 0; r < ncl; r++) bs_peer_store(bs_peer(smem_addr(&blk_sh), r), q);
         }
         for (int i = t; i < A.nflag; i += CTA) slots[i] = i == 0 ? X(0) : Pending<X>::value();
         __syncwarp();
-        bs_cluster_sync();
+        bs_cluster_arrive();
+        bs_cluster_wait();
         const int q = blk_sh;
         if (q * (int)ncl >= A.nblk) break;   // the same for the whole cluster
         const int b = q * (int)ncl + (int)rank;
