@@ -90,18 +90,24 @@ struct Transpose {
 };
 
 int exclusive_scan(hgb_ctx *c, const int *in, int *out, int n, int *total_dev, int *scratch);
-int csr_check(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx);
+// longest: the longest row's entries (optional)
+int csr_check(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx, int *longest = nullptr);
 int build_transpose(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx,
                     Transpose &T);
 
+// what the host knows of a pattern's rows
+struct CsrSize {
+    long nnz;
+    int longest = -1;   // entries of the longest row, -1: not known
+};
 template <typename V>
-int spmv_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
+int spmv_n_launch(hgb_ctx *c, int n_rows, CsrSize size, const int *pntr, const int *indx, const V *vals,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                   typename Val<V>::X *y, double *dot_out, const int *skip = nullptr, int *nparts = nullptr);
 // Y = alpha A X + beta Y over nrhs column-major columns, the matrix read once (each column
 // bit-identical to spmv_n_launch's product)
 template <typename V>
-int spmm_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals, int nrhs,
+int spmm_n_launch(hgb_ctx *c, int n_rows, CsrSize size, const int *pntr, const int *indx, const V *vals, int nrhs,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
                   typename Val<V>::X *y, long ldy);
 template <typename V>
@@ -137,6 +143,7 @@ const void *csr_vals(const hgb_csr *A);
 int csr_rows(const hgb_csr *A);
 int csr_cols(const hgb_csr *A);
 int csr_nnz(const hgb_csr *A);
+CsrSize csr_size(const hgb_csr *A);
 hgb_dtype csr_dtype(const hgb_csr *A);
 hgb_ctx *csr_ctx(const hgb_csr *A);
 

@@ -99,7 +99,7 @@ static int mr_grid(hgb_ctx *c, long total) {
 template <typename V>
 static int mr_gemm(hgb_csr *A, int nrhs, typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx,
                    typename Val<V>::X beta, typename Val<V>::X *y, long ldy) {
-    return spmm_n_launch<V>(csr_ctx(A), csr_rows(A), csr_nnz(A), csr_pntr(A), csr_indx(A), (const V *)csr_vals(A), nrhs, alpha, x,
+    return spmm_n_launch<V>(csr_ctx(A), csr_rows(A), csr_size(A), csr_pntr(A), csr_indx(A), (const V *)csr_vals(A), nrhs, alpha, x,
                             ldx, beta, y, ldy);
 }
 

@@ -321,14 +321,14 @@ static int spmv_A(hgb_ctx *c, hgb_csr *A, X alpha, const X *x, X beta, X *y, dou
         if (nparts) *nparts = 0;
         return spmv_t_fused_launch<V>(A, alpha, x, beta, y, x, dot, skip);
     }
-    return spmv_n_launch<V>(c, csr_rows(A), csr_nnz(A), csr_pntr(A), csr_indx(A), (const V *)csr_vals(A), alpha, x, beta, y,
+    return spmv_n_launch<V>(c, csr_rows(A), csr_size(A), csr_pntr(A), csr_indx(A), (const V *)csr_vals(A), alpha, x, beta, y,
                             nparts ? nullptr : dot, skip, nparts);
 }
 template <>
 int spmv_A<uint16_t, float>(hgb_ctx *c, hgb_csr *A, float alpha, const float *x, float beta, float *y, double *dot,
                            const int *skip, bool trans, int *nparts) {
     if (trans) return fail(HGB_ERR_UNSUPPORTED, "transposed product of a bf16 matrix");
-    return spmv_n_launch<uint16_t>(c, csr_rows(A), csr_nnz(A), csr_pntr(A), csr_indx(A), (const uint16_t *)csr_vals(A), alpha, x,
+    return spmv_n_launch<uint16_t>(c, csr_rows(A), csr_size(A), csr_pntr(A), csr_indx(A), (const uint16_t *)csr_vals(A), alpha, x,
                                    beta, y, nparts ? nullptr : dot, skip, nparts);
 }
 

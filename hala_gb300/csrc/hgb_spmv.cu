@@ -32,18 +32,20 @@ constexpr int kWarpBlock = 256;   // 8 warps per CTA
 constexpr int kStages = 2;        // tiles per warp in shared memory; three or four measured no gain
 constexpr int kMmCols = 5;        // columns summed per pass over a tile at most
 constexpr int kCapShort = 256, kCapLong = 384;   // entries of a staged tile (spmv_long_rows)
+constexpr int kWideMin = 64;      // entries from which a row of a tile that is not staged may be summed by its warp
 
 // CTAs per SM and x gathers in flight per lane and column, by vector type, columns per pass and
 // tile size.  More CTAs leave less of the 256 KB for L1, which holds the gathered part of x and the
 // rows that are read directly, and fewer registers for gathers; fewer CTAs leave HBM idle.  Measured
 // (us; 128^3 7-point FP64 / FP32, graph Laplacians of 680k rows FP64 / FP32, 5 columns on 95x97x96 FP64 / FP32):
-//   FP64, 256 entries: 3 CTAs of 8 gathers 45.3; of 4 gathers 47.8; 2 CTAs: 61.5; 4: 83.9 (spills); 6: 115.
-//   FP32, 256 entries: 4 CTAs of 8 gathers 28.7; of 4 gathers 31.1; 3 of 8 36.3.
+//   FP64, 256 entries: 3 CTAs of 8 gathers 45.2; of 4 gathers 47.8; 2 CTAs: 61.5; 4: 83.9 (spills); 6: 115.
+//   FP32, 256 entries: 4 CTAs of 8 gathers 28.5 (BF16 values 24.7), of 7 31.8; 5 of 4 28.9 (30.8), of 7 44.8 (spills); 6 of 4
+//   31.8 (31.6); 3 of 8 36.3.
 //   384 entries (rows of 9, which 256 would send to the direct path): FP64 2 CTAs 30.8, 3: 35.2; FP32 3 CTAs of
 //   4 gathers 16.9, of 8 20.2, 2 of 4 18.5.
 //   columns: FP64 3 CTAs with one gather per column 66.6, with two and passes of 3 + 2 columns 78.7; FP32 3 CTAs
 //   with two 28.8, 4 with three 39.0.
-// Before (one shape for all, 4 gathers, passes of 4 columns with one): 55.4 / 29.1, 33.2 / 26.7, 108.6 / 43.1.
+// One shape for all, 4 gathers, passes of 4 columns with one: 55.4 / 28.9 (25.0), 33.2 / 26.7, 108.6 / 43.1.
 template <typename X, int NC, int CAP>
 struct TileShape {
     static constexpr bool f64 = sizeof(X) == 8, wide = CAP > kCapShort;
@@ -106,14 +108,14 @@ __device__ __forceinline__ void spmv_dot_epilogue(double d, double *partials, un
 // then come one after another: spmv_wide takes a row while it has a third (FP64) or an eighth (FP32) of the entries
 // left, by the cost of an entry alone in its lane (about 190 cycles) and here (64; FP32 about 25).
 // Such tiles wait for the end of the kernel, in a function of their own: inlined, or at their place among the
-// staged tiles, they cost the staged FP64 product 45.8 -> 49 to 54 us.
+// staged tiles, they cost the staged FP64 product 45.8 -> 49 to 54 us.  Even so the test and the call cost the staged
+// products registers (128^3 FP64 45.2 -> 45.6 us, FP32 28.5 -> 32.9), so they are compiled in (WIDE) for the matrices that
+// may have such rows (spmv_may_be_wide).
 // Rows of 7 with 0.2 % of 3000, FP64 / FP32: 100k rows 646 / 285 -> 302 / 109 us; of 300, 400k rows 115 / 79 -> 76 / 36.
-// Four FP64 columns at 100k rows: 1637 -> 1174.  FP32 columns keep the lanes' own sums: the test alone took four
-// columns of staged rows 189 -> 199 us (2M rows of 7).  The staged single-column products: 128^3 FP64 45.9 -> 46.2 us,
-// 2M rows of 7 FP64 62.1 / FP32 47.8 -> 62.1 / 49.8.
+// Four FP64 columns at 100k rows: 1637 -> 1174.  FP32 columns keep the lanes' own sums.
 template <typename X>
 __device__ __forceinline__ bool spmv_wide(int longest, int left) {
-    return longest >= 64 && longest >= left / (sizeof(X) == 8 ? 3 : 8);
+    return longest >= kWideMin && longest >= left / (sizeof(X) == 8 ? 3 : 8);
 }
 template <typename V, bool EXACT>
 __device__ __forceinline__ typename Val<V>::X spmv_wide_row(const V *vp, const int *ip, unsigned len, const typename Val<V>::X *x) {
@@ -193,7 +195,7 @@ spmv_wide_tiles(int tb, int te, int n_rows, const int *__restrict__ pntr, const 
 // pass over a staged tile (the matrix is read once); optionally <x, y> (one column, square A; DOT as
 // spmv_dot_epilogue).  Every column is summed in column order in the mode's rounding, so each column
 // equals the single-column product bit for bit.
-template <typename V, int NC, int CAP, int DOT, bool EXACT>
+template <typename V, int NC, int CAP, int DOT, bool EXACT, bool WIDE>
 __global__ void __launch_bounds__(kWarpBlock, TileShape<typename Val<V>::X, NC, CAP>::ctas)
 spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict__ indx, const V *__restrict__ vals,
                  int nrhs, int cols, int end_mode, typename Val<V>::X alpha, const typename Val<V>::X *__restrict__ x,
@@ -260,8 +262,7 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
             const int first = __shfl_sync(0xffffffffu, ps[0], 0), end = __shfl_sync(0xffffffffu, pe[0], 31);
             int cnt = pe[0] - ps[0];
             int most = __reduce_max_sync(0xffffffffu, cnt);
-            if ((NC == 1 || sizeof(X) == 8) &&
-                __builtin_expect(end - first > CAP && spmv_wide<X>(most, end - first), 0)) {   // no entries, no row to write
+            if (WIDE && __builtin_expect(end - first > CAP && spmv_wide<X>(most, end - first), 0)) {   // no entries, no row to write
                 wide = tb;
                 row = n_rows;
                 cnt = most = 0;
@@ -337,7 +338,7 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
         }
     }
     cp_async_wait<0>();
-    if (wide < te)   // the tiles that were left out
+    if (WIDE && wide < te)   // the tiles that were left out
         dacc = spmv_wide_tiles<V, CAP, DOT != 0, EXACT>(wide, te, n_rows, pntr, indx, vals, NC == 1 ? 1 : nrhs, end_mode, alpha, x, ldx,
                                                         beta, y, ldy, dacc);
     if (DOT) spmv_dot_epilogue<DOT>(dacc.get(), partials, counter, dot_out);
@@ -464,10 +465,15 @@ spmv_t_cached_kernel(int n_cols, const int *__restrict__ pntrT, const int *__res
 
 // ------------------------------------------------------------- CSR validation ----------
 __global__ void csr_check_kernel(int n_rows, int n_cols, int nnz, const int *__restrict__ pntr,
-                                 const int *__restrict__ indx, int *err) {
+                                 const int *__restrict__ indx, int *err, int *longest) {
+    __shared__ int most;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    int len = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_rows; i += gridDim.x * blockDim.x) {
         int a = pntr[i], b = pntr[i + 1];
         if (a < 0 || b < a || b > nnz) { atomicOr(err, DEV_ERR_CSR); continue; }
+        len = max(len, b - a);
         int prev = -1;
         for (int p = a; p < b; p++) {
             int c = indx[p];
@@ -476,6 +482,10 @@ __global__ void csr_check_kernel(int n_rows, int n_cols, int nnz, const int *__r
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && (pntr[0] != 0 || pntr[n_rows] != nnz)) atomicOr(err, DEV_ERR_CSR);
+    if (!longest) return;
+    atomicMax(&most, len);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(longest, most);
 }
 
 // ------------------------------------------------------------- scan / transpose -------
@@ -570,12 +580,18 @@ int exclusive_scan(hgb_ctx *c, const int *in, int *out, int n, int *total_dev, i
     return launch_check("exclusive_scan");
 }
 
-int csr_check(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx) {
+int csr_check(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx, int *longest) {
+    if (longest) *longest = 0;
     if (n_rows <= 0) return HGB_OK;
+    int *most = longest ? (int *)c->result : nullptr;
+    if (most) HGB_CUDA(cudaMemsetAsync(most, 0, sizeof(int), c->stream));
     csr_check_kernel<<<std::min((n_rows + 255) / 256, c->num_sms * 8), 256, 0, c->stream>>>(n_rows, n_cols, nnz,
-                                                                                           pntr, indx, c->err);
+                                                                                           pntr, indx, c->err, most);
     HGB_TRY(launch_check("csr_check_kernel"));
-    return collect_dev_error(c);
+    if (most) HGB_CUDA(cudaMemcpyAsync(c->host_result, most, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    HGB_TRY(collect_dev_error(c));
+    if (longest) *longest = *(const int *)c->host_result;
+    return HGB_OK;
 }
 
 int build_transpose(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx,
@@ -622,14 +638,14 @@ static bool spmv_long_rows(int n_rows, long nnz) { return 2 * nnz > 15L * n_rows
 
 // The staged kernel's launch: a persistent grid of the resident CTAs of every SM (occupancy queried once per
 // kernel and device).
-template <typename V, int NC, int CAP, int DOT, bool EXACT>
+template <typename V, int NC, int CAP, int DOT, bool EXACT, bool WIDE>
 static int spmv_tile_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *indx, const V *vals, int nrhs, int cols,
                             typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
                             typename Val<V>::X *y, long ldy, double *partials, unsigned *counter, double *dot_out,
                             const int *skip, int *nparts) {
     constexpr size_t smem = spmv_smem_bytes<V, CAP>();
     constexpr int most = TileShape<typename Val<V>::X, NC, CAP>::ctas;
-    auto kernel = spmv_tile_kernel<V, NC, CAP, DOT, EXACT>;
+    auto kernel = spmv_tile_kernel<V, NC, CAP, DOT, EXACT, WIDE>;
     static std::atomic<int> occ_dev[64];
     if (c->device < 0 || c->device >= 64) return fail(HGB_ERR_UNSUPPORTED, "spmv: device ordinal %d", c->device);
     int occ = occ_dev[c->device].load();
@@ -649,19 +665,28 @@ static int spmv_tile_launch(hgb_ctx *c, int n_rows, const int *pntr, const int *
     return launch_check("spmv_tile_kernel");
 }
 
+// Whether a row may be long enough to be summed by its warp (spmv_wide).  The pattern check of a matrix handle knows the
+// longest row; the entries without a handle do not: in FP64 they take the test along (128^3 45.2 -> 45.6 us; without it
+// 100k rows of 7 with 0.2 % of 3000 take 646 us instead of 302), in FP32 and BF16, where it costs more (28.5 -> 32.9 and
+// 24.7 -> 32.9) and the rows' own lanes lose less (285 instead of 109), they do not.
+template <typename V>
+static bool spmv_may_be_wide(CsrSize size) { return size.longest < 0 ? sizeof(V) == 8 : size.longest >= kWideMin; }
+
 template <typename V, int DOT, bool EXACT>
-static int spmv_n_launch_mode(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
+static int spmv_n_launch_mode(hgb_ctx *c, int n_rows, CsrSize size, const int *pntr, const int *indx, const V *vals,
                               typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                               typename Val<V>::X *y, double *dot_out, const int *skip, int *nparts) {
     // DOT 2: the per-CTA parts of <x, y> stay in the context's parts slots (their count to *nparts)
     double *partials = DOT == 2 ? c->partials + kSpmvPartsOffset : (DOT == 1 ? c->partials : nullptr);
     unsigned *counter = DOT == 1 ? c->counter : nullptr;
-    if (aligned16(vals) && aligned16(indx))
-        return spmv_long_rows(n_rows, nnz)
-                   ? spmv_tile_launch<V, 1, kCapLong, DOT, EXACT>(c, n_rows, pntr, indx, vals, 1, 1, alpha, x, 0, beta, y, 0, partials,
-                                                             counter, dot_out, skip, nparts)
-                   : spmv_tile_launch<V, 1, kCapShort, DOT, EXACT>(c, n_rows, pntr, indx, vals, 1, 1, alpha, x, 0, beta, y, 0, partials,
-                                                             counter, dot_out, skip, nparts);
+    if (aligned16(vals) && aligned16(indx)) {
+#define HGB_SPMV(CAP, WIDE)                                                                                                    \
+    spmv_tile_launch<V, 1, CAP, DOT, EXACT, WIDE>(c, n_rows, pntr, indx, vals, 1, 1, alpha, x, 0, beta, y, 0, partials, counter, \
+                                                  dot_out, skip, nparts)
+        if (spmv_long_rows(n_rows, size.nnz)) return spmv_may_be_wide<V>(size) ? HGB_SPMV(kCapLong, true) : HGB_SPMV(kCapLong, false);
+        return spmv_may_be_wide<V>(size) ? HGB_SPMV(kCapShort, true) : HGB_SPMV(kCapShort, false);
+#undef HGB_SPMV
+    }
     const int g = std::min((n_rows + 255) / 256, std::min(c->num_sms * 8, kMaxReduceBlocks));
     if (nparts) *nparts = g;
     spmv_direct_kernel<V, DOT, EXACT><<<g, 256, 0, c->stream>>>(n_rows, pntr, indx, vals, spmv_end(alpha, beta), alpha, x, beta, y,
@@ -670,40 +695,43 @@ static int spmv_n_launch_mode(hgb_ctx *c, int n_rows, long nnz, const int *pntr,
 }
 
 template <typename V>
-int spmv_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals,
+int spmv_n_launch(hgb_ctx *c, int n_rows, CsrSize size, const int *pntr, const int *indx, const V *vals,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, typename Val<V>::X beta,
                   typename Val<V>::X *y, double *dot_out, const int *skip, int *nparts) {
     if (nparts) *nparts = 0;
     if (n_rows <= 0) return HGB_OK;
     const bool exact = c->spmv_mode == HGB_SPMV_EXACT;
     if (nparts)
-        return exact ? spmv_n_launch_mode<V, 2, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts)
-                     : spmv_n_launch_mode<V, 2, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts);
+        return exact ? spmv_n_launch_mode<V, 2, true>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts)
+                     : spmv_n_launch_mode<V, 2, false>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nparts);
     if (dot_out)
-        return exact ? spmv_n_launch_mode<V, 1, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr)
-                     : spmv_n_launch_mode<V, 1, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr);
-    return exact ? spmv_n_launch_mode<V, 0, true>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr)
-                 : spmv_n_launch_mode<V, 0, false>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr);
+        return exact ? spmv_n_launch_mode<V, 1, true>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr)
+                     : spmv_n_launch_mode<V, 1, false>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, dot_out, skip, nullptr);
+    return exact ? spmv_n_launch_mode<V, 0, true>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr)
+                 : spmv_n_launch_mode<V, 0, false>(c, n_rows, size, pntr, indx, vals, alpha, x, beta, y, nullptr, skip, nullptr);
 }
 
 template <typename V>
-int spmm_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *indx, const V *vals, int nrhs,
+int spmm_n_launch(hgb_ctx *c, int n_rows, CsrSize size, const int *pntr, const int *indx, const V *vals, int nrhs,
                   typename Val<V>::X alpha, const typename Val<V>::X *x, long ldx, typename Val<V>::X beta,
                   typename Val<V>::X *y, long ldy) {
     if (n_rows <= 0 || nrhs <= 0) return HGB_OK;
     if (!aligned16(vals) || !aligned16(indx)) {   // no staging: the single-column products
         for (int k = 0; k < nrhs; k++)
-            HGB_TRY(spmv_n_launch<V>(c, n_rows, nnz, pntr, indx, vals, alpha, x + (long)k * ldx, beta, y + (long)k * ldy,
+            HGB_TRY(spmv_n_launch<V>(c, n_rows, size, pntr, indx, vals, alpha, x + (long)k * ldx, beta, y + (long)k * ldy,
                                      nullptr));
         return HGB_OK;
     }
     const bool exact = c->spmv_mode == HGB_SPMV_EXACT;
     const int passes = (nrhs + kMmCols - 1) / kMmCols, cols = (nrhs + passes - 1) / passes;   // columns split evenly
-#define HGB_SPMM2(NC, CAP, EXACT)                                                                                   \
-    spmv_tile_launch<V, NC, CAP, 0, EXACT>(c, n_rows, pntr, indx, vals, nrhs, cols, alpha, x, ldx, beta, y, ldy, nullptr, \
+    // FP32 columns keep the lanes' own sums (spmv_wide_row)
+#define HGB_SPMM3(NC, CAP, EXACT, WIDE)                                                                             \
+    spmv_tile_launch<V, NC, CAP, 0, EXACT, WIDE>(c, n_rows, pntr, indx, vals, nrhs, cols, alpha, x, ldx, beta, y, ldy, nullptr, \
                                            nullptr, nullptr, nullptr, nullptr)
+#define HGB_SPMM2(NC, CAP, EXACT)                                                                                   \
+    (spmv_may_be_wide<V>(size) ? HGB_SPMM3(NC, CAP, EXACT, (NC == 1 || sizeof(V) == 8)) : HGB_SPMM3(NC, CAP, EXACT, false))
 #define HGB_SPMM(NC)                                                                               \
-    (spmv_long_rows(n_rows, nnz) ? (exact ? HGB_SPMM2(NC, kCapLong, true) : HGB_SPMM2(NC, kCapLong, false)) \
+    (spmv_long_rows(n_rows, size.nnz) ? (exact ? HGB_SPMM2(NC, kCapLong, true) : HGB_SPMM2(NC, kCapLong, false)) \
                                  : (exact ? HGB_SPMM2(NC, kCapShort, true) : HGB_SPMM2(NC, kCapShort, false)))
     switch (cols) {
         case 1: return HGB_SPMM(1);
@@ -712,21 +740,22 @@ int spmm_n_launch(hgb_ctx *c, int n_rows, long nnz, const int *pntr, const int *
         case 4: return HGB_SPMM(4);
         default: return HGB_SPMM(kMmCols);
     }
+#undef HGB_SPMM3
 #undef HGB_SPMM2
 #undef HGB_SPMM
 }
 
-template int spmv_n_launch<double>(hgb_ctx *, int, long, const int *, const int *, const double *, double,
+template int spmv_n_launch<double>(hgb_ctx *, int, CsrSize, const int *, const int *, const double *, double,
                                    const double *, double, double *, double *, const int *, int *);
-template int spmv_n_launch<float>(hgb_ctx *, int, long, const int *, const int *, const float *, float,
+template int spmv_n_launch<float>(hgb_ctx *, int, CsrSize, const int *, const int *, const float *, float,
                                   const float *, float, float *, double *, const int *, int *);
-template int spmv_n_launch<uint16_t>(hgb_ctx *, int, long, const int *, const int *, const uint16_t *, float,
+template int spmv_n_launch<uint16_t>(hgb_ctx *, int, CsrSize, const int *, const int *, const uint16_t *, float,
                                      const float *, float, float *, double *, const int *, int *);
-template int spmm_n_launch<double>(hgb_ctx *, int, long, const int *, const int *, const double *, int, double,
+template int spmm_n_launch<double>(hgb_ctx *, int, CsrSize, const int *, const int *, const double *, int, double,
                                    const double *, long, double, double *, long);
-template int spmm_n_launch<float>(hgb_ctx *, int, long, const int *, const int *, const float *, int, float,
+template int spmm_n_launch<float>(hgb_ctx *, int, CsrSize, const int *, const int *, const float *, int, float,
                                   const float *, long, float, float *, long);
-template int spmm_n_launch<uint16_t>(hgb_ctx *, int, long, const int *, const int *, const uint16_t *, int, float,
+template int spmm_n_launch<uint16_t>(hgb_ctx *, int, CsrSize, const int *, const int *, const uint16_t *, int, float,
                                      const float *, long, float, float *, long);
 
 template <typename V>
@@ -761,6 +790,7 @@ using namespace hgb;
 struct hgb_csr {
     hgb_ctx *ctx;
     int n_rows, n_cols, nnz;
+    int longest = -1;   // entries of the longest row
     const int *pntr, *indx;
     const void *vals;
     hgb_dtype dtype;
@@ -811,6 +841,7 @@ const void *csr_vals(const hgb_csr *A) { return A->vals; }
 int csr_rows(const hgb_csr *A) { return A->n_rows; }
 int csr_cols(const hgb_csr *A) { return A->n_cols; }
 int csr_nnz(const hgb_csr *A) { return A->nnz; }
+CsrSize csr_size(const hgb_csr *A) { return CsrSize{A->nnz, A->longest}; }
 hgb_dtype csr_dtype(const hgb_csr *A) { return A->dtype; }
 hgb_ctx *csr_ctx(const hgb_csr *A) { return A->ctx; }
 }  // namespace hgb
@@ -835,7 +866,7 @@ int hgb_spmv_f64(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, const 
                  const double *vals, double alpha, const double *x, double beta, double *y) {
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     DeviceGuard g(c->device);
-    if (trans == 'N' || trans == 'n') return spmv_n_launch<double>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    if (trans == 'N' || trans == 'n') return spmv_n_launch<double>(c, n_rows, CsrSize{nnz}, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
     return spmv_t_launch<double>(c, n_rows, n_cols, pntr, indx, vals, alpha, x, beta, y, nullptr);
 }
 
@@ -843,7 +874,7 @@ int hgb_spmv_f32(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, const 
                  const float *vals, float alpha, const float *x, float beta, float *y) {
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     DeviceGuard g(c->device);
-    if (trans == 'N' || trans == 'n') return spmv_n_launch<float>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    if (trans == 'N' || trans == 'n') return spmv_n_launch<float>(c, n_rows, CsrSize{nnz}, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
     return spmv_t_launch<float>(c, n_rows, n_cols, pntr, indx, vals, alpha, x, beta, y, nullptr);
 }
 
@@ -852,7 +883,7 @@ int hgb_spmv_bf16f32(hgb_ctx *c, char trans, int n_rows, int n_cols, int nnz, co
     HGB_TRY(check_spmv_args(c, trans, n_rows, n_cols, nnz, pntr, indx, vals, x, y));
     if (trans != 'N' && trans != 'n') return fail(HGB_ERR_UNSUPPORTED, "spmv_bf16f32: only trans 'N'");
     DeviceGuard g(c->device);
-    return spmv_n_launch<uint16_t>(c, n_rows, nnz, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
+    return spmv_n_launch<uint16_t>(c, n_rows, CsrSize{nnz}, pntr, indx, vals, alpha, x, beta, y, nullptr, nullptr);
 }
 
 int hgb_csr_create(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr, const int *indx,
@@ -863,8 +894,10 @@ int hgb_csr_create(hgb_ctx *c, int n_rows, int n_cols, int nnz, const int *pntr,
     if (dtype != HGB_F64 && dtype != HGB_F32 && dtype != HGB_BF16 && dtype != HGB_C128 && dtype != HGB_C64)
         return fail(HGB_ERR_ARG, "csr_create: dtype");
     DeviceGuard g(c->device);
-    HGB_TRY(csr_check(c, n_rows, n_cols, nnz, pntr, indx));
+    int longest = 0;
+    HGB_TRY(csr_check(c, n_rows, n_cols, nnz, pntr, indx, &longest));
     hgb_csr *A = new hgb_csr();
+    A->longest = longest;
     A->ctx = c;
     A->n_rows = n_rows;
     A->n_cols = n_cols;
@@ -889,9 +922,9 @@ int hgb_csr_gemv(hgb_csr *A, char trans, double alpha, const void *x, double bet
     }
     if (nt) {
         switch (A->dtype) {
-            case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const double *)A->vals, alpha, (const double *)x, beta, (double *)y, nullptr, nullptr);
-            case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const float *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
-            default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const uint16_t *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
+            case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const double *)A->vals, alpha, (const double *)x, beta, (double *)y, nullptr, nullptr);
+            case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const float *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
+            default: return spmv_n_launch<uint16_t>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const uint16_t *)A->vals, (float)alpha, (const float *)x, (float)beta, (float *)y, nullptr, nullptr);
         }
     }
     if (A->dtype == HGB_BF16) return fail(HGB_ERR_UNSUPPORTED, "csr_gemv: transpose of a bf16 matrix");
@@ -945,9 +978,9 @@ int hgb_csr_gemv_dot(hgb_csr *A, const void *x, void *y, double *dot_out) {
     hgb_ctx *c = A->ctx;
     DeviceGuard g(c->device);
     switch (A->dtype) {
-        case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const double *)A->vals, 1.0, (const double *)x, 0.0, (double *)y, dot_out, nullptr);
-        case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const float *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
-        default: return spmv_n_launch<uint16_t>(c, A->n_rows, A->nnz, A->pntr, A->indx, (const uint16_t *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
+        case HGB_F64: return spmv_n_launch<double>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const double *)A->vals, 1.0, (const double *)x, 0.0, (double *)y, dot_out, nullptr);
+        case HGB_F32: return spmv_n_launch<float>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const float *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
+        default: return spmv_n_launch<uint16_t>(c, A->n_rows, csr_size(A), A->pntr, A->indx, (const uint16_t *)A->vals, 1.0f, (const float *)x, 0.0f, (float *)y, dot_out, nullptr);
     }
 }
 
