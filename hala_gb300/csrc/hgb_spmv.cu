@@ -150,7 +150,7 @@ spmv_wide_tiles(int tb, int te, int n_rows, const int *__restrict__ pntr, const 
     const int lane = threadIdx.x & 31;
     for (int k = tb; k < te; k++) {
         const int row = k * 32 + lane;
-        const int ps = __ldg(pntr + min(row, n_rows)), pe = __ldg(pntr + min(row + 1, n_rows));
+        const int ps = __ldg(pntr + min(row, n_rows)), pe = __ldg(pntr + min(row, n_rows - 1) + 1);
         const int total = __shfl_sync(0xffffffffu, pe, 31) - __shfl_sync(0xffffffffu, ps, 0);
         if (total <= CAP || !spmv_wide<X>(__reduce_max_sync(0xffffffffu, pe - ps), total)) continue;
         for (int m = 0; m < nrhs; m++) {
@@ -221,9 +221,10 @@ spmv_tile_kernel(int n_rows, const int *__restrict__ pntr, const int *__restrict
 
     // lane's row pointers of tile k (loads only; nothing waits on them yet)
     auto load_ptrs = [&](int k, int &ps, int &pe) {
-        const int row = min(k, ntiles) * 32 + lane;
-        ps = __ldg(pntr + min(row, n_rows));
-        pe = __ldg(pntr + min(row + 1, n_rows));
+        // unsigned: the row behind the last tile may be 2^31 (a clamp to the last tile: 128^3 FP32 28.4 -> 32.0 us)
+        const unsigned row = (unsigned)min(k, ntiles) * 32u + lane, rows = n_rows;
+        ps = __ldg(pntr + min(row, rows));
+        pe = __ldg(pntr + min(row + 1, rows));
     };
     // tile k's copy into buffer buf when it fits (one commit per call)
     auto stage = [&](int k, int ps, int pe, int buf) {
