@@ -354,27 +354,31 @@ static int cg_iteration(hgb_ctx *c, hgb_csr *A, hgb_ilu *M, CgWork<X> &w, X *x, 
 // (about 27 us per iteration for six launches), not by bytes.  One cooperative launch runs up to
 // kCgpChunk iterations.  Every CTA keeps its rows for the whole launch.  What bounds an iteration is the latency of
 // its exchanges between CTAs and of FP64 instructions (each holds an SM quarter's unit for 62 cycles), so
-// it has one reduction (Chronopoulos and Gear's form of the method):
+// it has one reduction (after Chronopoulos and Gear's form of the method):
 //   x += a p, r -= a q                       (q = A p)
-//   s = A r, with the neighbours' r taken as they arrive (below), and <r, r> and <r, s> in one reduction
-//   b = <r, r> / <r, r>_old,  <p, A p> = <r, s> - b <r, r> / a,  a = <r, r> / <p, A p>
-//   p = r + b p, q = s + b q
-// FP32 vectors take <p, q> by a second reduction instead: the difference loses the condition number's share of
-// the digits, which FP64 has to spare and FP32 has not.  A launch starts with q = A p and <p, q> itself.  Every CTA sums all CTAs' parts in the same order, so
-// every CTA takes the same decision with the same bits.  Rounding differs from the graph path's, so the iteration
-// count can differ from it by a few.  Every wait is bounded: one that runs out of polls sets DEV_ERR_TIMEOUT and
-// every CTA returns.
-// Per iteration, before (two reductions by a counter that every CTA polls) and now: 24x24 7.5 -> 4.1 us, 256^2
-// 9.5 -> 5.9, 300^2 15.5 -> 7.3, 500^2 21.5 -> 16.1; FP32 256^2 8.3 -> 8.3.  Of the 12,000 cycles at 256^2 the mail
-// takes 2100, the neighbours' r 1300 to 2300, FP64 instructions of the rows 3100, and the sums with one
-// division 5000.
+//   s = A r, with the neighbours' r taken as they arrive (below); one reduction of <r, r>, <r, s>, <r, q> + <p, s>, <p, q>
+//   b = <r, r> / <r, r>_old, <p', q'> = <r, s> + b (<r, q> + <p, s>) + b^2 <p, q>, a = <r, r> / <p', q'>
+//   p' = r + b p, q' = s + b q
+// That is <p', q'> of the vectors as they are, whatever became of the residuals' orthogonality (the shorter form of the
+// method, <r, s> - b <r, r> / a, relies on it: 18 % more iterations on a 300-point biharmonic operator to 1e-13, 22 % on a
+// spectrum over 13 decades).  Where the terms cancel to less than a quarter of <r, s>, more than two bits, the CTAs sum
+// <p', q'> itself in a second reduction; on Poisson operators it stays near a half.  FP32 vectors and the rows in memory
+// (RPT = 0) always take that second reduction: the first has only <r, r>.  A launch starts with q = A p and <p, q> itself.
+// Every CTA sums all CTAs' parts in the same order, so every CTA takes the same decision with the same bits.  Rounding
+// differs from the graph path's, so the iteration count can differ from it.  Every wait is bounded: one that
+// runs out of polls sets DEV_ERR_TIMEOUT and every CTA returns.
+// Per iteration, in two reductions by a counter that every CTA polls, and so: 24x24 7.1 -> 4.4 us, 256^2
+// 9.5 -> 6.4, 300^2 15.4 -> 8.7, 500^2 21.4 -> 15.5; FP32 256^2 8.3 -> 8.1.  (With the shorter form 256^2 took 5.9, 300^2 7.3: two
+// sums fewer.  Of its 12,000 cycles at 256^2 the mail took 2100, the neighbours' r 1300 to 2300, FP64 instructions of the rows
+// 3100, and the sums with one division 5000.)
 constexpr int kCgpThreads = 256;
 constexpr int kCgpChunk = 4096;                 // iterations per launch
 constexpr long kCgpMaxRows = 1L << 20;          // larger systems take the graph path
 constexpr size_t kCgpMaxBytes = 48u << 20;      // matrix + vectors resident in L2 (129 MB)
 constexpr int kCgpCluster = 8;                  // CTAs of a cluster at most (8, 4 or 2)
 constexpr int kCgpLead = 4;                     // the warp that posts and polls
-constexpr int kCgpMail = 4;                     // mail entries per lane: at most 64 clusters
+constexpr unsigned kCgpClusters = 64;           // clusters at most: mail entries of a sum
+constexpr int kCgpSums = 4;                     // sums of a reduction at most
 
 // acc += v * x: separately rounded (the exact SpMV mode) or one fused multiply-add
 template <bool EXACT, typename X>
@@ -433,42 +437,49 @@ __device__ __forceinline__ bool cgp_wait_on(int &spins, const int *err) {
     return (spins & 1023) != 0 || !(*(const volatile int *)err & DEV_ERR_TIMEOUT);
 }
 
-// A reduction of two sums: the CTAs of a cluster exchange theirs through distributed shared memory, then the CTAs of
+// A reduction of up to kCgpSums sums: the CTAs of a cluster exchange theirs through distributed shared memory, then the CTAs of
 // equal rank exchange the clusters' through mailboxes in memory (every CTA has its own, one entry per cluster).
 // 256^2, 128 CTAs: 2100 cycles for the mail, where 128 CTAs polling one set of entries waited 6500 and each its own
 // mailbox of 128 entries 5000.  Two sets of entries take turns: a CTA posts to a set again only after every CTA
 // has posted to the other one, which each does after reading this one.
 // The sums are shaped to have few FP64 instructions in a row: the upper four warps' values are folded into the
-// lower four (one per quarter), whose lanes then add one of the two sums each, the first in lanes 0 to 15, the
-// second in 16 to 31, here and in the steps after it; the lead warp adds the warps' sums, posts, polls, and adds
-// the rest in one order, the same bits in every CTA.
+// lower four (one per quarter), whose lanes then add one of the NV sums each, a group of 32 / NV lanes a sum, here
+// and in the steps after it; the lead warp adds the warps' sums, posts, polls, and adds the rest in one order, the same
+// bits in every CTA.
 struct CgpShared {
-    CgpWord peer[2][kCgpCluster][2];
-    double fold[2][kCgpThreads / 2], warp[8], sum, alpha, beta;
-    int ok;
+    CgpWord peer[2][kCgpCluster][kCgpSums];
+    double fold[kCgpSums][kCgpThreads / 2], warp[4 * kCgpSums], sum, alpha, beta;
+    int ok, again;
 };
 __device__ __forceinline__ double cgp_add_xor(double v, int o) { return v + __shfl_xor_sync(0xffffffffu, v, o); }
 // All threads call it.  ORDER: what every CTA wrote before is in memory for all after the caller's next barrier.
-// meanwhile(): the lead warp's work between posting and polling.  The lead warp gets both sums;
+// meanwhile(): the lead warp's work between posting and polling.  The lead warp gets the sums;
 // false when a wait ran out.
-template <bool ORDER, typename F>
-__device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned number, CgpWord *mail, int *err, CgpShared &sh,
-                                             F meanwhile, double (&sum)[2]) {
+template <bool ORDER, int NV, typename F>
+__device__ __forceinline__ bool cgp_exchange(double (&v)[NV], unsigned number, CgpWord *mail, int *err, CgpShared &sh, F meanwhile,
+                                             double (&sum)[NV]) {
+    constexpr unsigned G = 32 / NV;   // lanes of a sum
+    static_assert(G >= kCgpCluster && NV <= kCgpSums, "a lane per peer");
     const int tid = threadIdx.x, wid = tid >> 5, set = number & 1;
-    const unsigned lane = tid & 31, half = lane >> 4, at = lane & 15;
+    const unsigned lane = tid & 31, own = lane / G, at = lane % G;
     if (tid >= kCgpThreads / 2) {
-        sh.fold[0][tid - kCgpThreads / 2] = v0;
-        sh.fold[1][tid - kCgpThreads / 2] = v1;
+#pragma unroll
+        for (int j = 0; j < NV; j++) sh.fold[j][tid - kCgpThreads / 2] = v[j];
     }
     __syncthreads();
     if (tid < kCgpThreads / 2) {
-        v0 += sh.fold[0][tid];
-        v1 += sh.fold[1][tid];
-        const double other = __shfl_xor_sync(0xffffffffu, half ? v0 : v1, 16);
-        double v = (half ? v1 : v0) + other;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) v = cgp_add_xor(v, o);
-        if (at == 0) sh.warp[half * 4 + wid] = v;
+        for (int j = 0; j < NV; j++) v[j] += sh.fold[j][tid];
+#pragma unroll
+        for (int h = NV / 2, o = 16; h > 0; h >>= 1, o >>= 1)   // each step leaves a lane half of its sums
+#pragma unroll
+            for (int j = 0; j < h; j++) {
+                const double keep = lane & o ? v[j + h] : v[j], send = lane & o ? v[j] : v[j + h];
+                v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v[0] = cgp_add_xor(v[0], o);
+        if (at == 0) sh.warp[own * 4 + wid] = v[0];
     } else if (ORDER && wid == kCgpLead) {
         cgp_fence();   // the CTA's writes, ordered before this by the barrier, before the posts below
     }
@@ -478,15 +489,15 @@ __device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned numb
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
     asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(clusters));
-    double t = sh.warp[half * 4 + (lane & 3)];
+    double t = sh.warp[own * 4 + (lane & 3)];
     t = cgp_add_xor(cgp_add_xor(t, 1), 2);
     if (at < size) {
         unsigned to;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"((unsigned)__cvta_generic_to_shared(&sh.peer[set][rank][half])), "r"(at));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"((unsigned)__cvta_generic_to_shared(&sh.peer[set][rank][own])), "r"(at));
         const CgpWord w = cgp_tag(t, number);
         asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(to), "l"(w.x), "l"(w.y) : "memory");
     }
-    const unsigned from = (unsigned)__cvta_generic_to_shared(&sh.peer[set][at & (size - 1)][half]);
+    const unsigned from = (unsigned)__cvta_generic_to_shared(&sh.peer[set][at & (size - 1)][own]);
     for (int spins = 0;;) {
         CgpWord w;
         asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "r"(from) : "memory");
@@ -496,20 +507,21 @@ __device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned numb
     for (unsigned o = 1; o < size; o *= 2) t = cgp_add_xor(t, o);
     if (ORDER) cgp_fence();   // what the peers ordered before their posts, before this CTA's
     if (clusters > 1) {
-        mail += (size_t)set * gridDim.x * clusters * 2;
-        for (unsigned k = at; k < clusters; k += 16)
-            cgp_store(mail + ((size_t)(k * size + rank) * clusters + blockIdx.x / size) * 2 + half, cgp_tag(t, number));
+        mail += (size_t)set * gridDim.x * clusters * kCgpSums;
+        for (unsigned k = at; k < clusters; k += G)
+            cgp_store(mail + ((size_t)(k * size + rank) * clusters + blockIdx.x / size) * kCgpSums + own, cgp_tag(t, number));
     }
     meanwhile();
     if (clusters > 1) {
-        mail += (size_t)blockIdx.x * clusters * 2 + half;
-        double part[kCgpMail];
+        constexpr int Q = kCgpClusters / G;   // entries a lane reads
+        mail += (size_t)blockIdx.x * clusters * kCgpSums + own;
+        double part[Q];
         for (int spins = 0;;) {
             bool here = true;
 #pragma unroll
-            for (int q = 0; q < kCgpMail; q++) {
+            for (int q = 0; q < Q; q++) {
                 CgpWord w = {(unsigned long long)number << 32, (unsigned long long)number << 32};   // whole, and zero
-                if (16 * q + at < clusters) w = cgp_load(mail + 2 * (16 * q + at));
+                if (G * q + at < clusters) w = cgp_load(mail + kCgpSums * (G * q + at));
                 here = cgp_whole(w, number, part[q]) && here;
             }
             if (__all_sync(0xffffffffu, here)) break;
@@ -517,19 +529,19 @@ __device__ __forceinline__ bool cgp_exchange(double v0, double v1, unsigned numb
         }
         if (ORDER) cgp_fence();
         t = part[0];
-        HGB_UNIFORM_IF(clusters > 16) t += part[1];
-        HGB_UNIFORM_IF(clusters > 32) t += part[2] + part[3];
-        for (unsigned o = 1; o < clusters && o < 16; o *= 2) t = cgp_add_xor(t, o);
+#pragma unroll
+        for (int q = 1; q < Q; q++) HGB_UNIFORM_IF(clusters > G * q) t += part[q];
+        for (unsigned o = 1; o < clusters && o < G; o *= 2) t = cgp_add_xor(t, o);
     }
-    sum[0] = __shfl_sync(0xffffffffu, t, 0);
-    sum[1] = __shfl_sync(0xffffffffu, t, 16);
+#pragma unroll
+    for (int j = 0; j < NV; j++) sum[j] = __shfl_sync(0xffffffffu, t, j * G);
     return true;
 }
 // RPT > 0: a CTA owns RPT * 256 consecutive rows (RPT: 1, 2 or 4 per thread) for the whole launch and keeps their
 // x, r, p, q and (rows of at most kCgpMaxE entries) their matrix entries in registers; r goes to shared memory for the
 // CTA's own rows and to memory tagged with the iteration for the others', and a row's sum waits for its neighbours'
 // entries alone.  RPT = 0: the rows are walked with grid-stride loops and every vector lives in memory (systems too
-// large for one register-resident row set; rt is s there); a reduction orders the writes of r before the products.
+// large for one register-resident row set; rt is not used); a reduction orders the writes of r before the products.
 constexpr int kCgpMaxE = 8;
 
 template <typename V, typename X, bool EXACT, int RPT>
@@ -550,9 +562,9 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
     bool done = false, good = true;
     const bool lead = threadIdx.x >> 5 == kCgpLead;
     if (threadIdx.x == 0) sh.ok = 1;
-    if (threadIdx.x < 2 * kCgpCluster * 2) (&sh.peer[0][0][0])[threadIdx.x] = CgpWord{0, 0};
+    if (threadIdx.x < 2 * kCgpCluster * kCgpSums) (&sh.peer[0][0][0])[threadIdx.x] = CgpWord{0, 0};
     cgp_cluster_sync();   // before a peer's first post
-    constexpr bool ONE = sizeof(X) == 8;   // one reduction per iteration
+    constexpr bool ONE = sizeof(X) == 8 && RPT > 0;   // one reduction per iteration, or two where it takes a second
     constexpr int K = RPT > 0 ? RPT : 1;
     long row[K];
     int beg[K], len[K], most[K], ci[K][kCgpMaxE];
@@ -601,13 +613,14 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
         return acc;
     };
     // The lead warp's last step: b = sum / den0 and a = sum / den1, one division in two lanes; then every thread's
-    auto finish = [&](bool ok, double sum, double den0, double den1) {
+    auto finish = [&](bool ok, double sum, double den0, double den1, bool second = false) {
         if (lead) {
             const double q = sum / (threadIdx.x & 1 ? den1 : den0);
             if ((threadIdx.x & 31) == 0) {
                 if (!ok) sh.ok = 0;
                 sh.sum = sum;
                 sh.beta = q;
+                sh.again = second;
             }
             if ((threadIdx.x & 31) == 1) sh.alpha = q;
         }
@@ -618,6 +631,12 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
     };
     auto nothing = [] {};
     double sum[2] = {0.0, 0.0};
+    // one sum of the whole grid, to the lead warp
+    auto exchange = [&](double v) {
+        number++;
+        double two[2] = {v, 0.0};
+        return cgp_exchange<false>(two, number, mail, err, sh, nothing, sum);
+    };
     // q = A p for the direction the launch starts from, and a = <r, r> / <p, q>
     {
         DotAcc<X> pq;
@@ -641,15 +660,13 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
                 pq.add(p[i], q);
             }
         }
-        number++;
-        const bool ok = cgp_exchange<false>(pq.get(), 0.0, number, mail, err, sh, nothing, sum);
+        const bool ok = exchange(pq.get());
         finish(ok, zr, 1.0, sum[0]);
     }
     for (int c = 0; c < kCgpChunk && good; c++) {
         const X a = (X)alpha, ma = -a, bta = (X)beta;
-        const double alpha_was = alpha;
         const bool next = ONE && c > 0;   // p and q of this direction are still to be formed
-        DotAcc<X> rrd, rsd;
+        DotAcc<X> rrd, rsd, crd, pqd;   // <r, r>, <r, s>, <r, q> + <p, s>, <p, q>
         if (RPT > 0) {
             const unsigned tag = c + 1;
             X was[K];   // r first: the others wait for it
@@ -666,6 +683,10 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
                 if (next) pr[k] = cgp_acc<EXACT, X>(was[k], bta, pr[k]);
                 xr[k] = cgp_acc<EXACT, X>(xr[k], a, pr[k]);
                 rrd.add(rr[k], rr[k]);
+                if (ONE) {
+                    crd.add(rr[k], qr[k]);
+                    pqd.add(pr[k], qr[k]);
+                }
             }
             __syncthreads();
             // the neighbours' r: the whole warp waits as one (lanes leaving a loop one by one would stay apart)
@@ -699,40 +720,35 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
                             }
                         return v;
                     });
-                    rsd.add(rr[k], sr[k]);
+                    if (ONE) {
+                        rsd.add(rr[k], sr[k]);
+                        crd.add(pr[k], sr[k]);
+                    }
                 }
             }
         } else {
             for (long i = t0; i < n; i += stride) {
-                X pi = p[i], qi = Ap[i], ri = r[i];
-                if (next) {
-                    p[i] = pi = cgp_acc<EXACT, X>(ri, bta, pi);
-                    Ap[i] = qi = cgp_acc<EXACT, X>(((const X *)rt)[i], bta, qi);
-                }
-                x[i] = cgp_acc<EXACT, X>(x[i], a, pi);
-                r[i] = ri = cgp_acc<EXACT, X>(ri, ma, qi);
+                x[i] = cgp_acc<EXACT, X>(x[i], a, p[i]);
+                const X ri = cgp_acc<EXACT, X>(r[i], ma, Ap[i]);
+                r[i] = ri;
                 rrd.add(ri, ri);
             }
             number++;
-            const bool ok = cgp_exchange<true>(rrd.get(), 0.0, number, mail, err, sh, nothing, sum);
+            double two[2] = {rrd.get(), 0.0};
+            const bool ok = cgp_exchange<true>(two, number, mail, err, sh, nothing, sum);
             finish(ok, sum[0], zr, 1.0);
             if (!good) break;
-            for (long i = t0; i < n; i += stride) {
-                const X si = memory_product(i, r);
-                rsd.add(r[i], si);
-                ((X *)rt)[i] = si;
-            }
         }
-        if (ONE || RPT > 0) {
+        if (ONE) {
             number++;
-            double ig = 0.0, ia = 0.0;
-            const bool ok = cgp_exchange<false>(rrd.get(), rsd.get(), number, mail, err, sh, [&] {
-                if (!ONE) return;
-                const double inv = 1.0 / (threadIdx.x & 1 ? alpha_was : zr);
-                ig = __shfl_sync(0xffffffffu, inv, 0);
-                ia = __shfl_sync(0xffffffffu, inv, 1);
-            }, sum);
-            finish(ok, sum[0], zr, sum[1] - (sum[0] * ig) * (sum[0] * ia));
+            double four[4] = {rrd.get(), rsd.get(), crd.get(), pqd.get()}, s4[4] = {0.0, 0.0, 0.0, 0.0}, inv = 0.0;
+            const bool ok = cgp_exchange<false>(four, number, mail, err, sh, [&] { inv = 1.0 / zr; }, s4);
+            const double b = s4[0] * inv, pq = fma(b, fma(b, s4[3], s4[2]), s4[1]);
+            finish(ok, s4[0], zr, pq, !(4.0 * pq > s4[1]));
+            if (!good) break;
+        } else if (RPT > 0) {
+            const bool ok = exchange(rrd.get());
+            finish(ok, sum[0], zr, 1.0);
             if (!good) break;
         }
         rrv = sh.sum;
@@ -740,38 +756,38 @@ cg_persistent_kernel(long n, const int *__restrict__ pntr, const int *__restrict
         done = (it >= max_iter) || (rrv < tol2) || !(rrv == rrv);
         if (done) break;
         zr = rrv;
-        if (!ONE) {
+        if (!ONE || sh.again) {   // the same in every CTA
             const X bt = (X)beta;
+            const double beta_was = beta;
             DotAcc<X> pq;
             if (RPT > 0) {
 #pragma unroll
                 for (int k = 0; k < K; k++) {
-                    pr[k] = cgp_acc<EXACT, X>(rr[k], bt, pr[k]);
-                    qr[k] = cgp_acc<EXACT, X>(sr[k], bt, qr[k]);
-                    pq.add(pr[k], qr[k]);
+                    const X pn = cgp_acc<EXACT, X>(rr[k], bt, pr[k]), qn = cgp_acc<EXACT, X>(sr[k], bt, qr[k]);
+                    pq.add(pn, qn);
+                    if (!ONE) {   // else formed with the next update
+                        pr[k] = pn;
+                        qr[k] = qn;
+                    }
                 }
             } else {
                 for (long i = t0; i < n; i += stride) {
                     const X pi = cgp_acc<EXACT, X>(r[i], bt, p[i]);
-                    const X qi = cgp_acc<EXACT, X>(((const X *)rt)[i], bt, Ap[i]);
+                    const X qi = cgp_acc<EXACT, X>(memory_product(i, r), bt, Ap[i]);
                     p[i] = pi;
                     Ap[i] = qi;
                     pq.add(pi, qi);
                 }
             }
-            number++;
-            const bool ok = cgp_exchange<false>(pq.get(), 0.0, number, mail, err, sh, nothing, sum);
+            const bool ok = exchange(pq.get());
             finish(ok, zr, 1.0, sum[0]);
+            beta = beta_was;
         }
     }
     if (ONE && good && !done) {   // the chunk's end: the next launch starts from this direction
         const X bt = (X)beta;
-        if (RPT > 0) {
 #pragma unroll
-            for (int k = 0; k < K; k++) pr[k] = cgp_acc<EXACT, X>(rr[k], bt, pr[k]);
-        } else {
-            for (long i = t0; i < n; i += stride) p[i] = cgp_acc<EXACT, X>(r[i], bt, p[i]);
-        }
+        for (int k = 0; k < K; k++) pr[k] = cgp_acc<EXACT, X>(rr[k], bt, pr[k]);
     }
     cgp_cluster_sync();   // no CTA ends before its peers' last posts to it
     if (!good) {
@@ -845,7 +861,7 @@ static CgpShape cgp_shape(const hgb_ctx *c, long n) {
                 }
                 known = clusters + 1;
             }
-            clusters = std::min(clusters, 16 * kCgpMail);
+            clusters = std::min(clusters, (int)kCgpClusters);
             const long rows = (rpt ? rpt : 4) * (long)kCgpThreads * cluster;   // of a cluster
             const long want = (n + rows - 1) / rows;
             if (clusters < 1 || (rpt && want > clusters)) continue;
@@ -871,9 +887,9 @@ static int cgp_run(hgb_ctx *c, hgb_csr *A, CgWork<X> &w, X *x, long n, long long
     const CgpShape sh = exact ? cgp_shape<V, X, true>(c, n) : cgp_shape<V, X, false>(c, n);
     const int G = sh.grid;
     if (G < 1) return fail(HGB_ERR_UNSUPPORTED, "persistent cg: no co-resident grid");
-    CgpWord *mail = nullptr;   // two sets of an entry (two words) per CTA and cluster
+    CgpWord *mail = nullptr;   // two sets of an entry (kCgpSums words) per CTA and cluster
     typename CgpR<X>::T *rt = nullptr;
-    const size_t nmail = 2 * (size_t)G * (G / sh.cluster) * 2;
+    const size_t nmail = 2 * (size_t)G * (G / sh.cluster) * kCgpSums;
     int st = HGB_OK;
     if (ws_alloc(c, &mail, nmail) || ws_alloc(c, &rt, n)) st = cuda_fail(cudaErrorMemoryAllocation, "persistent cg");
     const int *pntr = csr_pntr(A), *indx = csr_indx(A);
