@@ -13,7 +13,9 @@
 //    the values are read at every solve.  Inner products are compensated FP32 sums (two-product and
 //    two-sum), and the scalars are formed from such pairs: an FP64 instruction holds its SM quarter's
 //    unit for 62 cycles, and FP64 inner products with a division per thread took more time than
-//    the matrix.  Four shapes by the system's size in shared memory (kShapes).
+//    the matrix.  A pair holds 46 to 48 bits, of which the step and the direction's factor, floats, keep 24.  Its range
+//    is FP32's: a matrix far from 1 is solved scaled by a power of two, and the residual and the direction change
+//    their unit as they shrink.  Four shapes by the system's size in shared memory (kShapes).
 //    Bound: the shared-memory gathers of the direction (about 3.5 of 5.5 cycles per 32 entries).
 //  - batch_cg_kernel for systems that do not fit: vectors in shared memory, the matrix streamed from
 //    L2; a "large" item is one system solved by the whole CTA, a "small" item packs up to (threads/32)
@@ -241,6 +243,22 @@ __device__ void solve_system(const G &g, const BatchArgs &A, int s, float *sm) {
     g.sync();
 }
 
+// A pair of floats has FP32's range.  A matrix whose largest diagonal entry (its largest entry, A being positive
+// definite; top: its bits) lies outside [2^-10, 2^20) is solved as 2^-k A, that entry in [1, 2), for 2^k x.  Scales the image
+// and the solution; returns the matrix's factor (as two: 2^-k alone may be out of range) and leaves the solution's in *back.
+// (A function of its own: inlined, it took the systems that need none of it 4.9 -> 5.0 ms per 4,096.)
+template <int T>
+__device__ __noinline__ float2 onchip_scale(int top, float *v, int ne, double *xs, int n, double *back) {
+    if (!(top > 0 && top < 0x7f800000 && (unsigned)(ilogbf(__int_as_float(top)) + 10) >= 30u)) return make_float2(1.0f, 1.0f);
+    const int t = threadIdx.x, k = ilogbf(__int_as_float(top));
+    const float s1 = scalbnf(1.0f, -k / 2), s2 = scalbnf(1.0f, -(k - k / 2));
+    for (int i = t; i < ne; i += T) v[i] = v[i] * s1 * s2;
+    for (int i = t; i < n; i += T) xs[i] *= scalbn(1.0, k);
+    if (t == 0) *back = scalbn(1.0, -k);
+    __threadfence_block();
+    __syncthreads();
+    return make_float2(s1, s2);
+}
 template <int T, int RPT, int MINB>
 __global__ void __launch_bounds__(T, MINB)
 batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, int nitems, int *ticket) {
@@ -249,7 +267,10 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
     Df *red = (Df *)osm;   // [2][NW + 1]
     static_assert(sizeof(Df) * 2 * (NW + 1) <= kOnchipHead && NW <= 32, "head");
     __shared__ double dred[33];
-    __shared__ int item;
+    __shared__ int item, top;
+    __shared__ double back;   // the solution's scale
+    __shared__ double stop;   // the inner iteration's limit on <r, r>, and as a pair
+    __shared__ Df stop_pair;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     int buf = 0;
     // the CTA's sum, the same bits in every thread.  The second stage in one warp: in all of them at
@@ -271,7 +292,11 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
     float *p = (float *)(osm + kOnchipHead);
     for (;;) {
         __syncthreads();
-        if (t == 0) item = atomicAdd(ticket, 1);
+        if (t == 0) {
+            item = atomicAdd(ticket, 1);
+            top = 0;
+            back = 1.0;
+        }
         __syncthreads();
         if (item >= nitems) break;
         const int s = items[item], r0 = A.sys_ptr[s], n = A.sys_ptr[s + 1] - r0, ns = (n + 31) >> 5;
@@ -300,6 +325,7 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
         int slice[RPT];   // {first entry / 32, width (8 bits)}
         float diag[RPT];
         double bb = 0.0;
+        int big = 0;   // the bits of the largest |diagonal|
 #pragma unroll
         for (int j = 0; j < RPT; j++) {
             const int row = t + j * T;
@@ -313,13 +339,19 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
             if (row < n) {
                 const int d = Y.dpos[r0 + row], o = r0 + Y.orig[r0 + row];
                 if (d >= 0) diag[j] = __ldg(A.vals + d);
+                big = max(big, __float_as_int(diag[j]) & 0x7fffffff);
                 Y.xs[r0 + row] = A.x[o];
                 const double bi = A.b[o];
                 bb += bi * bi;
             }
         }
+        big = __reduce_max_sync(0xffffffffu, big);
+        if (lane == 0) atomicMax(&top, big);
         __threadfence_block();
         const double bnorm = sqrt(g.sum(bb));   // its barriers: the image is in
+        const float2 sc = onchip_scale<T>(top, v, ne, Y.xs + r0, n, &back);
+#pragma unroll
+        for (int j = 0; j < RPT; j++) diag[j] = diag[j] * sc.x * sc.y;
         const double target = A.rtol * bnorm;
         int total = 0;
         double res = 0.0;
@@ -356,7 +388,7 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
             // the FP32 right-hand side, scaled by a power of two to a norm near 1 (exact, and taken back
             // from the correction): its squares stay far from FP32's range limits
             const int ex = min(max(ilogb(res), -1000), 1000);
-            const double down = scalbn(1.0, -ex), up = scalbn(1.0, ex);
+            const double down = scalbn(1.0, -ex);
             float r[RPT], d[RPT], q[RPT];
             Df acc{0.0f, 0.0f};
 #pragma unroll
@@ -367,8 +399,15 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
                 df_fma(acc, r[j], r[j]);
             }
             Df rz = sum(acc);
-            const double st = A.inner_rtol * A.inner_rtol * ((double)rz.s + (double)rz.c);
-            const Df stop2{(float)st, (float)(st - (double)(float)st)};
+            auto set_stop = [&](double v) {   // (the pair not 0: a residual that vanishes ends the iteration)
+                const float h = fmaxf((float)v, 0x1p-126f);
+                stop = v;
+                stop_pair = Df{h, (float)v >= h ? (float)(v - (double)h) : 0.0f};
+            };
+            if (t == 0) set_stop(A.inner_rtol * A.inner_rtol * ((double)rz.s + (double)rz.c));
+            __syncthreads();
+            Df stop2 = stop_pair;
+            float unit = 1.0f;   // of d, the residual and the direction
             // inner FP32 CG on A d = r from d = 0 (solve_cg_core's order, identity preconditioner)
             for (int it = 0; it < A.max_inner; it++) {
                 acc = Df{0.0f, 0.0f};
@@ -416,12 +455,30 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
                 total++;
                 if (nr.s < stop2.s || (nr.s == stop2.s && nr.c < stop2.c) || !(nr.s == nr.s)) break;
                 const float beta = df_div(nr, rz);
+                rz = nr;
+                if (__builtin_expect(nr.s < 0x1p-40f || nr.s > 0x1p60f, 0)) {
+                    // another unit (a power of two): <r, r> leaves the range in which its parts' products are exact
+                    const float f = nr.s < 1.0f ? 0x1p20f : 0x1p-20f;
+                    if (unit < 0x1p-100f) break;   // the rest of d is far below its last bits
+                    unit /= f;
+                    rz = Df{nr.s * f * f, nr.c * f * f};
+                    if (t == 0) set_stop(stop * ((double)f * (double)f));
+                    __syncthreads();
+                    stop2 = stop_pair;
+#pragma unroll
+                    for (int j = 0; j < RPT; j++)
+                        if (w + j * NW < ns) {
+                            r[j] *= f;
+                            d[j] *= f;
+                            p[t + j * T] *= f;
+                        }
+                }
 #pragma unroll
                 for (int j = 0; j < RPT; j++)
                     if (w + j * NW < ns) p[t + j * T] = r[j] + beta * p[t + j * T];
-                rz = nr;
                 __syncthreads();
             }
+            const double up = scalbn((double)unit, ex);
 #pragma unroll
             for (int j = 0; j < RPT; j++)
                 if (t + j * T < n) Y.xs[r0 + t + j * T] += (double)d[j] * up;
@@ -430,7 +487,7 @@ batch_onchip_kernel(BatchArgs A, OnchipLayout Y, const int *__restrict__ items, 
         }
 #pragma unroll
         for (int j = 0; j < RPT; j++)
-            if (t + j * T < n) A.x[r0 + Y.orig[r0 + t + j * T]] = Y.xs[r0 + t + j * T];
+            if (t + j * T < n) A.x[r0 + Y.orig[r0 + t + j * T]] = Y.xs[r0 + t + j * T] * back;
         if (t == 0) {
             if (A.iters) A.iters[s] = total;
             if (A.relres) A.relres[s] = bnorm > 0 ? res / bnorm : res;
