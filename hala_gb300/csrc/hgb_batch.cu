@@ -1041,15 +1041,20 @@ int hgb_batch_autotune(hgb_batch *B, const double *b, double *x, double rtol, co
     if (!B || !b || !x) return fail(HGB_ERR_ARG, "batch_autotune: bad arguments");
     hgb_ctx *c = B->ctx;
     DeviceGuard g(c->device);
-    // signature: number of systems and the size histogram in powers of two
+    if (B->nitems == 0) {   // every system is on chip: the configuration changes nothing
+        if (best) *best = B->cfg;
+        return HGB_OK;
+    }
+    // signature: number of systems and the streamed ones' size histogram in powers of two
     std::ostringstream sig;
     int hist[16] = {0};
-    for (int s : B->sizes) {
+    for (int s = 0; s < B->S; s++) {
+        if (onchip_shape(B, s) >= 0) continue;
         int k = 0;
-        while ((1 << (k + 1)) <= s && k < 15) k++;
+        while ((1 << (k + 1)) <= B->sizes[s] && k < 15) k++;
         hist[k]++;
     }
-    sig << "S" << B->S << "_rt" << rtol;
+    sig << "streamed_of_S" << B->S << "_rt" << rtol;
     for (int k = 0; k < 16; k++) if (hist[k]) sig << "_" << k << ":" << hist[k];
     if (cache_path) {
         std::ifstream in(cache_path);

@@ -367,7 +367,8 @@ int hgb_batch_get_config(hgb_batch *batch, hgb_batch_config *cfg);
 int hgb_batch_cg_solve(hgb_batch *batch, const double *b, double *x, double rtol, double inner_rtol,
                        int max_inner, int max_outer, int *iters, double *relres);
 /* Times the launch shapes on this batch (x is overwritten) and keeps the fastest; the choice
- * is cached under a size-histogram key in cache_path (text, may be NULL). */
+ * is cached under a size-histogram key of the systems that do not fit on chip in cache_path (text,
+ * may be NULL).  Where every system fits, the present configuration is returned at once. */
 int hgb_batch_autotune(hgb_batch *batch, const double *b, double *x, double rtol,
                        const char *cache_path, hgb_batch_config *best);
 int hgb_batch_destroy(hgb_batch *batch);
