@@ -67,6 +67,24 @@ __device__ __forceinline__ int wait_row(const int *lev, int j, int lane, int *er
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
+// The levels of up to 32 rows, one per lane (j < 0: none, -1): all lanes poll until each has its own, with the pauses and
+// the bound of wait_row.
+__device__ __forceinline__ int wait_level(const int *lev, int j, int *err) {
+    int v = j < 0 ? -1 : ld_acquire(lev + j);
+    for (int spins = 0; __any_sync(0xffffffffu, j >= 0 && v < 0); spins++) {
+        if (spins > kSpinLimit || ((spins & 255) == 255 && (*(volatile int *)err & DEV_ERR_TIMEOUT))) {
+            if (j >= 0 && v < 0) {
+                atomicOr(err, DEV_ERR_TIMEOUT);
+                v = 0;
+            }
+            continue;
+        }
+        __nanosleep(spins < 8 ? 20 : (spins < 64 ? 100 : 400));
+        if (j >= 0 && v < 0) v = ld_acquire(lev + j);
+    }
+    return v;
+}
+
 // Starts of the chunks (by position in solve order): every 32nd position, and the rows without an entry in
 // the row before (columns are sorted: it would sit beside the diagonal).
 __global__ void chunk_flag_kernel(int n, const int *__restrict__ pntr, const int *__restrict__ indx,
@@ -109,10 +127,19 @@ __global__ void __launch_bounds__(256) levels_kernel(int n, const int *__restric
             const int a = lower ? __ldg(pntr + row) : __ldg(diag + row) + 1;
             const int b = lower ? __ldg(diag + row) : __ldg(pntr + row + 1);
             int m = -1;
-            for (int p = a; p < b; p++) {
-                const int j = __ldg(indx + p), jpos = lower ? j : n - 1 - j;
-                m = max(m, jpos >= p0 ? chunk_lev[w][jpos - p0] : wait_row(lev, j, lane, err));
+            for (int p = a; p < b; p += 32) {   // the entries' levels 32 at a time: rows may have hundreds
+                int j = -1;
+                if (p + lane < b) {
+                    j = __ldg(indx + p + lane);
+                    const int jpos = lower ? j : n - 1 - j;
+                    if (jpos >= p0) {
+                        m = max(m, chunk_lev[w][jpos - p0]);
+                        j = -1;
+                    }
+                }
+                m = max(m, wait_level(lev, j, err));
             }
+            m = __reduce_max_sync(0xffffffffu, m);
             if (lane == 0) {
                 chunk_lev[w][pos - p0] = m + 1;
                 st_release(lev + row, m + 1);
