@@ -64,6 +64,8 @@ struct BsPlan {
     // deep: the pattern of a 3D grid (hgb_bsplan.cu)
     int n = 0, nblk = 0, cl = 1, nslots = 0, nflag = 0, nonunit = 0, lower = 1, rev = 0, xsize = 8, deep = 0;
     long units = 0;                 // 16-byte units of the packet buffer
+    long path = 0;                  // length of the sweep in steps, hand-overs included (hgb_bsplan.cu)
+    int levels = 0;                 // levels of the strip with the most: the pattern has no fewer
     std::vector<int4> blk;          // [4 nblk] {first strip, strips, flagged slots, slots} {first watch, watches, mailbox or
                                     // -1, 0} {per strip: first and end mail unit}; units of 16 bytes
     long mail_units = 0;

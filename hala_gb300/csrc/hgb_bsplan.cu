@@ -100,6 +100,12 @@ struct Rows {   // a row's strictly lower / upper entries, in solve order of the
 struct Halo {
     int row, slot, key;
 };
+struct Use {   // a step (a sample of them) that reads a row of an earlier block, and its begin on its strip's clock
+    int row, strip, begin;
+};
+struct Lag {
+    int strip, offset;   // a strip starts at least so long after that one
+};
 
 struct BlockOut {
     int nflag = 0, nslots = 0, seg[kBsW + 1] = {};   // seg: first halo slot of every strip
@@ -107,10 +113,14 @@ struct BlockOut {
     std::vector<int4> strip, chunk, step;
     std::vector<int> ext_codes, ext_map, direct;
     std::vector<Halo> halo;
+    std::vector<Use> use;             // by strip
+    int span[kBsW] = {};              // the strips' clocks at their ends
+    int late[kBsW][kBsW];             // of strip k behind strip s of the block (INT_MIN: does not read it)
+    int levels = 0;                   // of its strip with the most
 };
 
 struct Scratch {   // one thread's working arrays
-    std::vector<int> lev, cnt, start, order, step_of, last, flag, tslot, next, head, time, window, touched;
+    std::vector<int> lev, cnt, start, order, step_of, last, flag, tslot, next, head, time, clock, window, touched;
     std::vector<int> strip_steps, step_base, free_q;
 };
 
@@ -147,10 +157,17 @@ static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool
     cut.push_back(n);
 }
 
+// Clock of the plan, in steps of rows of up to three entries (0.14 us in FP32, 0.35 in FP64): a step with rows of kx entries in
+// the ext arrays (0.2 us an entry, 0.24) ...
+static int bs_step_cost(int xsize, int kx) { return kx == 0 ? 1 : (xsize == 8 ? 1 + (2 * kx + 2) / 3 : 1 + (3 * kx + 1) / 2); }
+// ... and a hand-over inside a cluster, and across
+static int bs_hop_cost(int xsize, bool near) { return xsize == 8 ? (near ? 1 : 4) : (near ? 2 : 9); }
+constexpr int kPathSample = 16;   // every so many steps of a strip are looked at for the strips that it waits for
+
 // One block: its strips' steps, slots, chunks and packets (into pk from position P0 on).  Where the block's own
 // rows take more than cap slots, only B.nslots is set.
 static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, int bw, const int *cut, int s0, int s1,
-                          int4 *pk, int *pk_of_row, BlockOut &B, Scratch &S) {
+                          int4 *pk, int *pk_of_row, int *done, BlockOut &B, Scratch &S) {
     const int P0 = cut[s0], P1 = cut[s1], rows = P1 - P0, ns = s1 - s0;
     const int RA = bs_ra(xsize), D = bs_d(xsize);
     S.lev.resize(rows);
@@ -177,6 +194,7 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
             S.cnt[lv]++;
         }
         const int nl = (int)S.cnt.size();
+        B.levels = std::max(B.levels, nl);
         S.start.assign(nl + 1, 0);
         for (int l = 0; l < nl; l++) S.start[l + 1] = S.start[l] + S.cnt[l];
         int steps = 0;
@@ -244,6 +262,8 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
     S.window.resize(std::max<size_t>(S.window.size(), std::min(P0, bw)), 0);   // by distance from the block
     S.touched.clear();
     S.time.assign(nsteps, 0);
+    S.clock.assign(nsteps, 0);   // end of every step, on its strip's clock (bs_step_cost)
+    std::fill(&B.late[0][0], &B.late[0][0] + kBsW * kBsW, INT_MIN);
     int nh = 0;
     for (int k = 0; k < ns; k++) {
         const int p0 = cut[s0 + k];
@@ -256,11 +276,14 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
         }
         B.seg[k] = (1 + nf + nh + 16 / xsize - 1) / (16 / xsize) * (16 / xsize);
         for (int st = S.strip_steps[k]; st < S.strip_steps[k + 1]; st++) {
-            int t = st > S.strip_steps[k] ? S.time[st - 1] + 1 : 0;
+            int t = st > S.strip_steps[k] ? S.time[st - 1] + 1 : 0, kx = 0;
+            const int begin = st > S.strip_steps[k] ? S.clock[st - 1] : 0;
+            const bool sample = (st - S.strip_steps[k]) % kPathSample == 0;
             for (int pass = 0; pass < 2; pass++) {   // the step's time, then its halo
                 for (int q = S.step_base[st]; q < S.step_base[st + 1]; q++) {
                     int a, e;
                     R.deps(R.row_of(S.order[q]), a, e);
+                    bool ext = e - a > 3;
                     for (int i = a; i < e; i++) {
                         const int pj = R.pos_of(R.indx[i]);
                         if (pj >= p0) continue;
@@ -268,7 +291,9 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
                             if (pass == 0) {
                                 int s = 0;
                                 while (cut[s0 + s + 1] <= pj) s++;
-                                t = std::max(t, S.time[S.strip_steps[s] + S.step_of[pj - P0]] + 1);
+                                const int from = S.strip_steps[s] + S.step_of[pj - P0];
+                                t = std::max(t, S.time[from] + 1);
+                                if (sample) B.late[k][s] = std::max(B.late[k][s], S.clock[from] + 1 - begin);
                             }
                         } else if (pass == 1) {
                             int &w = S.window[P0 - 1 - pj];
@@ -285,11 +310,17 @@ static void bs_plan_block(const Rows &R, int rev, int np, int xsize, int cap, in
                                 Halo &h = B.halo[w - 1 - nf];
                                 h.key = std::min(h.key, t);
                             }
+                            if (sample) B.use.push_back({R.indx[i], k, begin});
+                            ext = ext || w < 0;
                         }
                     }
+                    if (pass == 1 && ext) kx = std::max(kx, e - a);
                 }
                 if (pass == 0) S.time[st] = t;
             }
+            S.clock[st] = begin + bs_step_cost(xsize, kx);
+            for (int q = S.step_base[st]; q < S.step_base[st + 1]; q++) done[S.order[q]] = S.clock[st];
+            B.span[k] = S.clock[st];
         }
     }
     for (int k = ns; k <= kBsW; k++) B.seg[k] = (1 + nf + nh + 16 / xsize - 1) / (16 / xsize) * (16 / xsize);
@@ -391,6 +422,8 @@ struct Sweep {
     std::vector<BlockOut> out;
     std::vector<std::vector<int2>> watch;
     std::vector<std::vector<Halo>> far;   // entries from earlier clusters
+    BsArray<int> done;                    // end of the step of every row (by position), on its strip's clock
+    std::vector<std::vector<Lag>> lag;    // of every strip, behind strips of earlier blocks
     std::vector<char> mailed;
     struct Base {
         size_t strip, chunk, step, watch, ext;
@@ -439,6 +472,7 @@ struct Sweep {
         P.pk.resize(n);
         P.pk_of_row.resize(n);
         P.watched.assign(n, 0);
+        done.resize(n);
         group(cluster_of);
         return HGB_OK;
     }
@@ -450,6 +484,7 @@ struct Sweep {
         out.assign(nblk, BlockOut());
         watch.resize(nblk);
         far.resize(nblk);
+        lag.resize(nstrips);
         mailed.assign(nblk, 0);
     }
     // after the blocks are planned: whether all of them fit.  Where one does not, the sweep takes blocks of
@@ -465,16 +500,17 @@ struct Sweep {
     }
     void block(int b, Scratch &scr) {
         bs_plan_block(R, rev, np, xsize, cap, bw, cut.data(), b * spb, std::min(nstrips, (b + 1) * spb), P.pk.data(),
-                      P.pk_of_row.data(), out[b], scr);
+                      P.pk_of_row.data(), done.data(), out[b], scr);
     }
     // where the halos of a cluster's blocks come from: inside the cluster they are pushed
     void halos(int run) {
         const int b0 = run * cl, b1 = std::min(nblk, b0 + cl);
-        for (int b = b0; b < b1; b++)
+        for (int b = b0; b < b1; b++) {
+            lags(b, b0);
             for (const Halo &h : out[b].halo) {
                 if (h.row < 0) continue;   // padding
                 const int pj = R.pos_of(h.row);
-                const int pb = (int)(std::upper_bound(cut.begin(), cut.end(), pj) - cut.begin() - 1) / spb;
+                const int pb = strip_of(pj) / spb;
                 int4 &k = P.pk[P.pk_of_row[h.row]];
                 if (pb >= b0 && !(k.w & kBsPush)) {
                     k.z |= (int)((unsigned)h.slot << 16);
@@ -483,6 +519,39 @@ struct Sweep {
                     far[b].push_back({h.row, h.slot, h.key << 8 | std::min(b - pb, 255)});
                 }
             }
+        }
+    }
+    int strip_of(int pos) const { return (int)(std::upper_bound(cut.begin(), cut.end(), pos) - cut.begin() - 1); }
+    // how far the strips of a block start behind those of earlier ones (b0: the first block of its cluster)
+    void lags(int b, int b0) {
+        std::vector<Lag> *to = nullptr;
+        int of = -1;
+        for (const Use &u : out[b].use) {
+            if (u.strip != of) {
+                of = u.strip;
+                to = &lag[b * spb + of];
+            }
+            const int pj = R.pos_of(u.row), ps = strip_of(pj), late = done[pj] + bs_hop_cost(xsize, ps / spb >= b0) - u.begin;
+            size_t i = 0;
+            while (i < to->size() && (*to)[i].strip != ps) i++;
+            if (i == to->size()) to->push_back({ps, late});
+            else (*to)[i].offset = std::max((*to)[i].offset, late);
+        }
+    }
+    // the sweep's length on the strips' clocks, each strip running as a whole from the time at which all that it waits
+    // for comes no later than it reads it
+    void path() {
+        std::vector<long> start(nstrips, 0);
+        P.path = P.levels = 0;
+        for (const BlockOut &B : out) P.levels = std::max(P.levels, B.levels);
+        for (int k = 0; k < nstrips; k++) {
+            const BlockOut &B = out[k / spb];
+            const int first = k / spb * spb;
+            for (int s = first; s < k; s++)
+                if (B.late[k - first][s - first] != INT_MIN) start[k] = std::max(start[k], start[s] + B.late[k - first][s - first]);
+            for (const Lag &l : lag[k]) start[k] = std::max(start[k], start[l.strip] + l.offset);
+            P.path = std::max(P.path, start[k] + B.span[k - first]);
+        }
     }
     // the rows that push to no block of their own cluster mail to the first block that needs them (in
     // block order: a row's readers in several clusters are told apart by the order of the blocks)
@@ -640,7 +709,10 @@ int bs_plan_sweeps(int n, const int *pntr, const int *indx, const int *diag, int
         }
     }
     phase([](Sweep &s) { return s.runs; }, [](Sweep &s, int r) { s.halos(r); });
-    phase([](Sweep &) { return 1; }, [](Sweep &s, int) { s.mails(); });
+    phase([](Sweep &) { return 1; }, [](Sweep &s, int) {
+        s.mails();
+        s.path();
+    });
     phase(blocks, [](Sweep &s, int b) { s.watches(b); });
     for (Sweep &s : S) HGB_TRY(s.sizes());
     phase(blocks, [](Sweep &s, int b) { s.gather(b); });

@@ -21,6 +21,7 @@
 #include "hgb_complex.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <string>
 #include <thread>
@@ -263,19 +264,22 @@ __global__ void task_fill_kernel(int nl, const int *__restrict__ cnt, const int 
     }
 }
 
-// Build the schedule from a completed level array (S.level filled, S.n set).
-static int build_schedule(hgb_ctx *c, Schedule &S, int lower) {
-    const int n = S.n;
-    int *dmax = nullptr;
-    HGB_CUDA(cudaMalloc(&dmax, sizeof(int) * 2));
+// Levels of a completed level array (S.level filled, S.n set).
+static int count_levels(hgb_ctx *c, const Schedule &S, int *levels) {
+    int *dmax = (int *)c->result, mx = -1;
     HGB_CUDA(cudaMemsetAsync(dmax, 0xff, sizeof(int), c->stream));
-    int g = std::max(1, std::min((n + 255) / 256, c->num_sms * 8));
-    max_level_kernel<<<g, 256, 0, c->stream>>>(n, S.level, dmax);
-    int mx = -1;
+    max_level_kernel<<<std::max(1, std::min((S.n + 255) / 256, c->num_sms * 8)), 256, 0, c->stream>>>(S.n, S.level, dmax);
     HGB_CUDA(cudaMemcpyAsync(&mx, dmax, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     HGB_CUDA(cudaStreamSynchronize(c->stream));
-    const int nl = mx + 1;
-    S.nlevels = nl;
+    *levels = mx + 1;
+    return HGB_OK;
+}
+
+// Build the schedule from a completed level array.
+static int build_schedule(hgb_ctx *c, Schedule &S, int lower) {
+    const int n = S.n, g = std::max(1, std::min((n + 255) / 256, c->num_sms * 8));
+    HGB_TRY(count_levels(c, S, &S.nlevels));
+    const int nl = S.nlevels;
     int *cnt = nullptr, *lptr = nullptr, *tcnt = nullptr, *tptr = nullptr, *scratch = nullptr;
     size_t nb = (size_t)(nl + 1 + 1023) / 1024 + 2;
     HGB_CUDA(cudaMalloc(&cnt, sizeof(int) * (nl + 1)));
@@ -301,7 +305,6 @@ static int build_schedule(hgb_ctx *c, Schedule &S, int lower) {
     task_fill_kernel<<<gl, 256, 0, c->stream>>>(nl, cnt, lptr, tptr, S.tasks);
     HGB_TRY(launch_check("build_schedule"));
     HGB_CUDA(cudaStreamSynchronize(c->stream));
-    cudaFree(dmax);
     cudaFree(cnt);
     cudaFree(lptr);
     cudaFree(tcnt);
@@ -371,7 +374,7 @@ struct SolveArgs {
     int *ticket;
     const int *pntr, *indx, *diag;   // diag[i] = position of the diagonal entry of row i
     const int *map;                  // optional value gather (transposed view), may be null
-    const double *piv;               // optional FP64 pivots (division in FP64), may be null
+    const double *piv;               // optional FP64 pivots (their FP32 reciprocals are multiplied by), may be null
     int lower, unit, mode, rev;
     int *err;
     const int *skip;                 // optional device flag: the launch is a no-op when set
@@ -425,6 +428,8 @@ __global__ void __launch_bounds__(256) trsv_kernel(SolveArgs A, const V *__restr
             else { a = d + 1; b = __ldg(A.pntr + row + 1); }
             const X xin = in[row];
             const X dval = A.unit ? X(1) : Val<V>::get(__ldg(vals + (A.map ? __ldg(A.map + d) : d)));
+            X dinv = X(1);   // of an FP64 pivot in a lower-precision store, as the strips' packets carry it
+            if (A.piv && !A.unit) dinv = (X)(1.0 / __ldg(A.piv + row));
             X acc = (A.mode == MODE_ILU) ? xin : X(0);
             const int len = b - a;
             for (int k0 = 0; k0 < len; k0 += 8) {
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(SolveArgs A, const V *__restr
             }
             if (A.mode == MODE_TRSV) acc = sub_rn(mul_rn(alpha, xin), acc);
             if (!A.unit) {
-                if (A.piv) acc = (X)__ddiv_rn((double)acc, __ldg(A.piv + row));
+                if (A.piv) acc = mul_rn(acc, dinv);
                 else acc = div_rn(acc, dval);
             }
             st_relaxed(out + row, Pending<X>::canon(acc));
@@ -742,6 +747,32 @@ static int ilu_schedules(hgb_ilu *M) {
     return HGB_OK;
 }
 
+// Strips or levels.  A strip sweep takes its plan's path times a step (0.14 us in FP32, 0.35 in FP64).  A global-level
+// sweep takes its levels times a hand-over through L2, which grows with the tasks that poll: 0.7 us in FP32 and 1.5 in FP64
+// where a level is one row (a band of 4: 20,000 levels), 1.3 and 2.2 at 150 rows (a 301 x 290 grid), 2.0 and 2.7 at 1,300
+// (61 x 60 x 63), 2.5 to 3 at 10,000 (random patterns).  Strips of a grid in its natural order pipeline: 301 x 290 155 us a
+// pair of FP32 sweeps against 1530 by levels.  Elsewhere their steps follow one another, the more so where rows list more
+// than three entries: 27 points on 40^3 20.8 ms against 1.4, 200k rows of 6 random entries 32.6 against 0.16, 40^3
+// in a random order 6.7 against 0.09, by reverse Cuthill-McKee 0.55 against 0.32.  The estimates hold to a fifth; strips are given 1.15.
+static double strips_us(const BsPlan &P) { return P.path * (P.xsize == 8 ? 0.35 : 0.14); }
+static double levels_us(const BsPlan &P, int levels) {
+    const double width = std::log10(std::max(1.0, (double)P.n / levels));
+    return levels * (P.xsize == 8 ? 1.5 + 0.35 * width : 0.7 + 0.4 * width);
+}
+static int ilu_prefer_levels(hgb_ilu *M, const BsPlanPair &P, bool &by_level) {
+    const double kStrips = 1.15;
+    by_level = false;
+    // a strip's own levels are a lower bound of the pattern's: enough to decide for the grids, without the count
+    if (strips_us(P.A) <= kStrips * levels_us(P.A, std::max(1, P.A.levels))) return HGB_OK;
+    int levels = 0;
+    HGB_TRY(count_levels(M->ctx, M->L, &levels));
+    if (strips_us(P.A) <= kStrips * levels_us(P.A, std::max(1, levels))) return HGB_OK;
+    HGB_TRY(ilu_schedules(M));   // the upper triangle's levels too
+    by_level = strips_us(P.A) + strips_us(P.B) >
+               kStrips * (levels_us(P.A, std::max(1, M->L.nlevels)) + levels_us(P.B, std::max(1, M->U.nlevels)));
+    return HGB_OK;
+}
+
 // The device part of ILU(0) creation.  plan: when given, the block-solve schedules were planned on
 // the host already (from host arrays); otherwise they are planned here from D2H copies.
 static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const int *indx, const void *vals,
@@ -810,7 +841,12 @@ static int ilu_create_device(hgb_ctx *c, int n, int nnz, const int *pntr, const 
             if ((st = launch_check("ilu store conversion"))) break;
         }
         if (cudaMalloc(&M->tmp, xsize(store) * n) != cudaSuccess) { st = cuda_fail(cudaGetLastError(), "ilu0_create"); break; }
-        // patterns that the strip plan cannot hold fall back to the global-level solve
+        // patterns that the strip plan cannot hold, or whose strips wait for one another, take the global-level solve
+        if (!bs) {
+            bool by_level = false;
+            if ((st = ilu_prefer_levels(M, *plan, by_level))) break;
+            if (by_level) bs = HGB_ERR_UNSUPPORTED;
+        }
         if (!bs) bs = bsolve_load(c, plan->A, M->BL, pntr, M->diag, M->svals, (int)vsize(store), nullptr);
         if (!bs) bs = bsolve_load(c, plan->B, M->BU, pntr, M->diag, M->svals, (int)vsize(store), M->piv);
         if (bs == HGB_OK) M->use_bs = true;

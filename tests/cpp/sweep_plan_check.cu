@@ -166,7 +166,8 @@ struct Sim {
 }  // namespace
 
 extern "C" {
-// Plans both sweeps and runs them; bad[2][6]: what was found wrong in each.  most: the largest cluster.
+// Plans both sweeps and runs them; bad[2][6]: what was found wrong in each; shape[2][4]: blocks, slots, path, levels of
+// the strip with the most.  most: the largest cluster.
 // Returns the planner's status.
 int sweep_plan_check(int n, const int *pntr, const int *indx, const int *diag, int xsize, int most, int nonunit_a, int nonunit_b,
                      int rev_b, long *bad, int *shape) {
@@ -179,8 +180,10 @@ int sweep_plan_check(int n, const int *pntr, const int *indx, const int *diag, i
         Sim s{*plan[k], Rows{n, kind[k].lower, pntr, indx, diag}, kind[k].nonunit, kind[k].rev};
         s.run();
         std::memcpy(bad + k * COUNT, s.bad, sizeof(s.bad));
-        shape[2 * k] = plan[k]->nblk;
-        shape[2 * k + 1] = plan[k]->nslots;
+        shape[4 * k] = plan[k]->nblk;
+        shape[4 * k + 1] = plan[k]->nslots;
+        shape[4 * k + 2] = (int)std::min<long>(plan[k]->path, INT_MAX);
+        shape[4 * k + 3] = plan[k]->levels;
     }
     delete pair;
     return st;

@@ -105,9 +105,49 @@ def test_plan(lib, name):
     for xsize in (8, 4):
         for most in (16, 3):
             for nonunit_a, nonunit_b, rev_b in ((0, 1, 0), (1, 0, 1)):      # the applications of M and M^T
-                bad, shape = (ctypes.c_long * 12)(), (ctypes.c_int * 4)()
+                bad, shape = (ctypes.c_long * 12)(), (ctypes.c_int * 8)()
                 st = lib.sweep_plan_check(n, *at, xsize, most, nonunit_a, nonunit_b, rev_b, bad, shape)
                 where = (name, xsize, most, rev_b, list(shape))
                 assert st == 0, where
                 found = np.array(list(bad)).reshape(2, 6)      # rows, slots, values, stuck steps, targets, strips
                 assert not found.any(), (where, found.tolist())
+
+
+def levels(pntr, indx, diag):
+    lev = np.zeros(len(pntr) - 1, int)
+    for r in range(len(lev)):
+        for q in range(pntr[r], diag[r]):
+            lev[r] = max(lev[r], lev[indx[q]] + 1)
+    return int(lev.max()) + 1
+
+
+def permuted(pattern, seed):
+    pntr, indx, _ = pattern
+    n = len(pntr) - 1
+    q = np.random.default_rng(seed).permutation(n)
+    return csr(sp.csr_matrix((np.ones(len(indx)), indx, pntr), shape=(n, n))[q][:, q])
+
+
+# the most and the fewest steps of a sweep for each of the pattern's levels: strips of a grid in its order pipeline; in a random
+# order, or where rows list more than three entries, they follow one another
+PATHS = {
+    "grid_63x65x61": (lambda: grid(63, 65, 61), 1.0, 2.0),
+    "grid_301x97": (lambda: grid(301, 97, 1), 1.0, 2.0),
+    "line_5000": (lambda: grid(5000, 1, 1), 1.0, 1.1),
+    "random_30000": (lambda: random(30000, 6), 50.0, 1e4),
+    "grid_20x20x20_permuted": (lambda: permuted(grid(20, 20, 20), 1), 20.0, 1e4),
+}
+
+
+@pytest.mark.parametrize("name", list(PATHS))
+def test_path(lib, name):
+    make, fewest, most = PATHS[name]
+    pntr, indx, diag = make()
+    at = [a.ctypes.data_as(ctypes.c_void_p) for a in (pntr, indx, diag)]
+    nlev = levels(pntr, indx, diag)
+    for xsize in (8, 4):
+        bad, shape = (ctypes.c_long * 12)(), (ctypes.c_int * 8)()
+        assert lib.sweep_plan_check(len(pntr) - 1, *at, xsize, 16, 0, 1, 0, bad, shape) == 0
+        for k in (0, 1):
+            path, own = shape[4 * k + 2], shape[4 * k + 3]
+            assert own <= nlev and fewest * nlev <= path <= most * nlev, (xsize, k, path, own, nlev)
