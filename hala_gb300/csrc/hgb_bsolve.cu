@@ -283,7 +283,9 @@ __device__ __forceinline__ void bs_step_wait(int id) { asm volatile("bar.sync %0
 // LOOK: look for the values from other strips before a step's turn (always in FP64; in FP32 not for the
 // patterns of 3D grids, where they are never in that early: 180 us per 128^3 BF16-store application
 // without, 204 with; the 512^2 one 260 without, 232 with).
-template <typename X, int MODE, int DIAG, bool LOOK>
+// EXT: some row of the plan lists its entries in the ext arrays (a form of its own: without it all sweeps took 6 to 12 %
+// longer, 128^3 FP32 194 us a pair against 184, 512^2 254 against 228, FP64 596 against 528).
+template <typename X, int MODE, int DIAG, bool LOOK, bool EXT>
 __global__ void __launch_bounds__(kBsThreads, 1)
 bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
     constexpr int XS = sizeof(X), W = kBsW, K = kBsK, D = bs_d(XS), RA = bs_ra(XS);
@@ -469,6 +471,24 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                 const bool early0 = h.x & kBsEarly0, early2 = h.x & kBsEarly2, no2 = h.x & kBsNo2;   // uniform
                 X ax = X(0);
                 if (MODE == 1) ax = mul_rn(alpha, xin);
+                // rows with their entries in the ext arrays: the first ones' codes and values, of all rows' count
+                constexpr int PE = XS == 8 ? 2 : 4;   // registers: four in FP64 cost a grid with a few long rows 7.1 -> 7.6 ms
+                int nd = 0, most = 0, ecode[PE];
+                X evalue[PE];
+                auto load_ext = [&](int q0) {
+#pragma unroll
+                    for (int u = 0; u < PE; u++)
+                        if (q0 + u < nd) {
+                            const long e = (long)p.x + (long)(q0 + u) * cnt;
+                            ecode[u] = __ldg(A.ext_codes + e);
+                            evalue[u] = __ldg((const X *)A.ext_vals + e);
+                        }
+                };
+                if (EXT && (h.x & kBsStepExt)) {
+                    nd = ext && act ? p.y & 0xFFFF : 0;
+                    most = __reduce_max_sync(0xFFFFFFFFu, nd);
+                    load_ext(0);
+                }
                 // ---- before the step's turn: whether all values that come from other strips and blocks (far) are
                 // in, so that its turn need not poll; FP64: the arithmetic that needs no others, an operation taking 64 cycles
                 X acc = (MODE == 0) ? xin : X(0), m2 = X(0);
@@ -527,18 +547,25 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                     acc = bs_term<MODE>(acc, mul_rn(rw.v[1], x1));
                     acc = bs_term<MODE>(acc, mul_rn(rw.v[2], x2));
                 }
-                if (h.x & kBsStepExt) {   // some row of the step lists its entries in the ext arrays
-                    if (ext && act) {
-                        const int nd = p.y & 0xFFFF;
-                        for (int q = 0; q < nd; q++) {
-                            const long e = (long)p.x + (long)q * cnt;
-                            const int cd = __ldg(A.ext_codes + e);
-                            const X vk = __ldg((const X *)A.ext_vals + e);
-                            X xk;
-                            if (cd >= 0) xk = bs_wait_slot(sbase + cd * XS, bs_slot(sbase + cd * XS, X(0)), A.err);
-                            else xk = wait_value(out + (-cd - 1), A.err);
-                            acc = bs_term<MODE>(acc, mul_rn(vk, xk));
-                        }
+                if (EXT && (h.x & kBsStepExt)) {   // PE entries at a time, the next ones' loads in flight
+                    for (int q0 = 0; q0 < most; q0 += PE) {
+                        X xk[PE], vk[PE];
+                        int cd[PE];
+#pragma unroll
+                        for (int u = 0; u < PE; u++)
+                            if (q0 + u < nd) {
+                                cd[u] = ecode[u];
+                                vk[u] = evalue[u];
+                                xk[u] = cd[u] >= 0 ? bs_slot(sbase + cd[u] * XS, X(0)) : ld_relaxed(out + (-cd[u] - 1));
+                            }
+                        load_ext(q0 + PE);
+#pragma unroll
+                        for (int u = 0; u < PE; u++)
+                            if (q0 + u < nd) {
+                                if (cd[u] >= 0) xk[u] = bs_wait_slot(sbase + cd[u] * XS, xk[u], A.err);
+                                else if (Pending<X>::is(xk[u])) xk[u] = wait_value(out + (-cd[u] - 1), A.err);
+                                acc = bs_term<MODE>(acc, mul_rn(vk[u], xk[u]));
+                            }
                     }
                     __syncwarp();
                 }
@@ -700,7 +727,7 @@ static int bs_clusters_fit(hgb_ctx *c, int cl, int xsize) {
         return n;
     };
     DeviceGuard g(c->device);
-    const int n = xi ? fits(bsolve_kernel<double, 0, BS_DIV, true>) : fits(bsolve_kernel<float, 0, BS_DIV, false>);
+    const int n = xi ? fits(bsolve_kernel<double, 0, BS_DIV, true, true>) : fits(bsolve_kernel<float, 0, BS_DIV, false, true>);
     cache[c->device][xi][cl] = n;
     init[c->device][xi][cl] = true;
     return n;
@@ -782,6 +809,7 @@ int bsolve_load(hgb_ctx *c, const BsPlan &P, BlockSolve &S, const int *pntr, con
     S.xsize = P.xsize;
     S.nonunit = P.nonunit;
     S.deep = P.deep;
+    S.ext = !P.ext_map.empty();
     S.dv_recip = (piv != nullptr && P.xsize == 4) ? 1 : 0;
     BsParts dev, tmp;   // what stays, and what only the packing needs
     const size_t o_blk = dev.add(sizeof(int4) * P.blk.size()), o_strip = dev.add(sizeof(int4) * P.strip.size()),
@@ -827,12 +855,12 @@ int bsolve_load(hgb_ctx *c, const BsPlan &P, BlockSolve &S, const int *pntr, con
     return st;
 }
 
-template <typename X, int MODE, int DIAG, bool LOOK>
-static int bs_launch_look(hgb_ctx *c, const BlockSolve &S, const BsArgs &A, X alpha, const X *in, X *out, X *pend) {
+template <typename X, int MODE, int DIAG, bool LOOK, bool EXT>
+static int bs_launch_form(hgb_ctx *c, const BlockSolve &S, const BsArgs &A, X alpha, const X *in, X *out, X *pend) {
     constexpr int XS = sizeof(X), CTA = kBsThreads;
     const size_t smem = bs_ring_bytes(XS, DIAG != BS_UNIT) + (size_t)S.nslots * XS;
     if (smem > (size_t)kBsSmemMax) return fail(HGB_ERR_UNSUPPORTED, "bsolve: %d slots per block", S.nslots);
-    auto kernel = bsolve_kernel<X, MODE, DIAG, LOOK>;
+    auto kernel = bsolve_kernel<X, MODE, DIAG, LOOK, EXT>;
     // per device: the kernel's attributes; per (device, cluster size, shared memory): how many clusters
     // are co-resident
     struct FitKey { int dev, cl; size_t smem; int n; };
@@ -878,8 +906,11 @@ static int bs_launch_look(hgb_ctx *c, const BlockSolve &S, const BsArgs &A, X al
 template <typename X, int MODE, int DIAG>
 static int bs_launch_one(hgb_ctx *c, const BlockSolve &S, const BsArgs &A, X alpha, const X *in, X *out, X *pend) {
     if constexpr (sizeof(X) == 4)
-        if (S.deep) return bs_launch_look<X, MODE, DIAG, false>(c, S, A, alpha, in, out, pend);
-    return bs_launch_look<X, MODE, DIAG, true>(c, S, A, alpha, in, out, pend);
+        if (S.deep)
+            return S.ext ? bs_launch_form<X, MODE, DIAG, false, true>(c, S, A, alpha, in, out, pend)
+                         : bs_launch_form<X, MODE, DIAG, false, false>(c, S, A, alpha, in, out, pend);
+    return S.ext ? bs_launch_form<X, MODE, DIAG, true, true>(c, S, A, alpha, in, out, pend)
+                 : bs_launch_form<X, MODE, DIAG, true, false>(c, S, A, alpha, in, out, pend);
 }
 
 template <typename X>

@@ -87,7 +87,7 @@ struct BsPlanPair {
 
 // Device copy of a plan with the values in the packets.
 struct BlockSolve {
-    int n = 0, nblk = 0, cl = 1, nslots = 0, nflag = 0, xsize = 8, nonunit = 0, dv_recip = 0, deep = 0;
+    int n = 0, nblk = 0, cl = 1, nslots = 0, nflag = 0, xsize = 8, nonunit = 0, dv_recip = 0, deep = 0, ext = 0;
     unsigned char *base = nullptr;   // the one allocation that holds all of the below
     int4 *blk = nullptr, *strip = nullptr;
     unsigned char *packets = nullptr;

@@ -158,8 +158,8 @@ static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool
 }
 
 // Clock of the plan, in steps of rows of up to three entries (0.14 us in FP32, 0.35 in FP64): a step with rows of kx entries in
-// the ext arrays (0.2 us an entry, 0.24) ...
-static int bs_step_cost(int xsize, int kx) { return kx == 0 ? 1 : (xsize == 8 ? 1 + (2 * kx + 2) / 3 : 1 + (3 * kx + 1) / 2); }
+// the ext arrays (0.17 us an entry, 0.2) ...
+static int bs_step_cost(int xsize, int kx) { return kx == 0 ? 1 : (xsize == 8 ? 1 + (4 * kx + 3) / 7 : 1 + (6 * kx + 4) / 5); }
 // ... and a hand-over inside a cluster, and across
 static int bs_hop_cost(int xsize, bool near) { return xsize == 8 ? (near ? 1 : 4) : (near ? 2 : 9); }
 constexpr int kPathSample = 16;   // every so many steps of a strip are looked at for the strips that it waits for
