@@ -26,7 +26,6 @@
 #include <exception>
 #include <functional>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace hgb {
@@ -64,7 +63,7 @@ class HostTeam {
                         busy.fetch_sub(1);
                     }
                 });
-        } catch (const std::system_error &) {   // no more threads: those that run take the work
+        } catch (const std::exception &) {   // no more threads, or no memory for them: those that run take the work
         }
     }
     ~HostTeam() {

@@ -166,6 +166,17 @@ struct Sim {
 }  // namespace
 
 extern "C" {
+// Plans the lower sweep only; -1 where it threw.
+int sweep_plan_throws(int n, const int *pntr, const int *indx, const int *diag) {
+    BsPlan P;
+    BsPlan *plan[1] = {&P};
+    const BsSweepKind kind[1] = {{1, 0, 0}};
+    try {
+        return bs_plan_sweeps(n, pntr, indx, diag, 8, [](int nblk) { return std::min(2, nblk); }, 1, kind, plan);
+    } catch (const std::exception &) {
+        return -1;
+    }
+}
 // Plans both sweeps and runs them; bad[2][6]: what was found wrong in each; shape[2][4]: blocks, slots, path, levels of
 // the strip with the most.  most: the largest cluster.
 // Returns the planner's status.

@@ -17,6 +17,19 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "cpp", "sweep_plan_check.cu")
 
 
+def test_failing_allocations(tmp_path):
+    """the planner's threads end, and the caller gets the exception, whichever allocation fails (a thread that cannot be
+    started is done without)"""
+    obj, exe = str(tmp_path / "check.o"), str(tmp_path / "alloc")
+    inc = "-I" + os.path.join(ROOT, "include")
+    for cmd in ([build.nvcc_path(), "-std=c++17", "-O2", *build.ARCH, inc, "-c", "-o", obj, SRC],
+                [build.nvcc_path(), "-std=c++17", "-O2", "-o", exe, obj, os.path.join(os.path.dirname(SRC), "sweep_plan_alloc.cpp"), "-lpthread"]):
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
+
+
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("plan") / "sweep_plan_check.so")
