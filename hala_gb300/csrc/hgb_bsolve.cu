@@ -390,16 +390,12 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
             continue;
         }
 
-        // ---- solver warps: warp k of group g takes the steps k, k + K, ... of the strips g, g + W, ...
+        // ---- solver warps: warp k of group g takes the steps k, k + K, ... of strip g (a block has at most W)
         const int4 bi = __ldg(A.blk + 4 * b);
-        const int g = warp / K, k = warp % K, nstrips = bi.y;
-        // barrier of the last step of the group's strip before (first: none; the group's warp 0 takes a
-        // strip's first step, so where it took that last step too, its program order is enough)
-        int prev = g * K;
-        for (int si = g; si < nstrips; si += W) {
-            const int4 sd = __ldg(A.strip + 2 * ((bi.x + si) * K + k)), sz = __ldg(A.strip + 2 * ((bi.x + si) * K + k) + 1);
+        const int g = warp / K, k = warp % K;
+        if (g < bi.y) {
+            const int4 sd = __ldg(A.strip + 2 * ((bi.x + g) * K + k)), sz = __ldg(A.strip + 2 * ((bi.x + g) * K + k) + 1);
             const int ns = sd.y, nch = (ns - k + K - 1) / K;   // steps of the strip, and this warp's
-            const bool more = si + W < nstrips;
             const X *inb = in + sd.x;
             X *outb = out + sd.x, *pendb = pend ? pend + sd.x : nullptr;
             const unsigned char *src = A.packets + (size_t)sd.z * 16;   // next chunk to copy (lane 0)
@@ -510,7 +506,7 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                 }
                 // ---- its turn: the strip's own values are in; the far ones are polled.  The warp polls as one:
                 // lanes that left a loop one by one would run the rest of the step apart.
-                if (s > 0 || prev > g * K) bs_step_wait(s > 0 ? g * K + (k + K - 1) % K : prev);
+                if (s > 0) bs_step_wait(g * K + (k + K - 1) % K);
                 X x0 = bs_slot(a0, X(0)), x1 = bs_slot(a1, X(0)), x2 = bs_slot(a2, X(0));
                 if (!early)
                     for (int spins = 1; __any_sync(0xFFFFFFFFu, bs_pending(x0) || bs_pending(x1) || bs_pending(x2)); spins++) {
@@ -575,7 +571,7 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                 if (push) bs_offer(offer_a, acc);
                 if (post) st_relaxed(mail, acc);
                 __syncwarp();
-                if (s + 1 < ns || (more && k > 0)) bs_step_done(g * K + k);
+                if (s + 1 < ns) bs_step_done(g * K + k);
                 // ---- after it
                 if (act) {
                     const int row = p.z & 0xFFFF;
@@ -595,7 +591,6 @@ bsolve_kernel(BsArgs A, X alpha, const X *in, X *out, X *pend) {
                 if (wslot == 0) wpar ^= 1;
             }
             cp_async_wait<0>();
-            prev = g * K + (ns - 1) % K;
         }
     }
     // the last CTA to leave resets the ticket for the next launch
@@ -733,7 +728,7 @@ static int bs_clusters_fit(hgb_ctx *c, int cl, int xsize) {
     return n;
 }
 
-// Cluster size.  Every hop between clusters goes through L2 and the fetcher warps, a hop inside a
+// Cluster size.  Every hop between clusters goes through L2 and the mail warps, a hop inside a
 // cluster through distributed shared memory; and a block whose cluster is not co-resident starts
 // only when another cluster has finished all its blocks.  So: the largest size (up to 16, sizes
 // above 8 being non-portable) at which the clusters of all nblk blocks are co-resident; failing

@@ -1,7 +1,7 @@
 // The host's plan of a strip-scheduled triangular sweep (hgb_bsolve.cu runs it).
 //
-// Rows are cut, in solve order, into strips (one warp solves a strip) and runs of strips into blocks
-// (one CTA).  Inside a strip the rows are grouped by their level over the dependencies that stay in
+// Rows are cut, in solve order, into strips (kBsK warps solve a strip, its steps in turn) and runs of up to kBsW strips
+// into blocks (one CTA).  Inside a strip the rows are grouped by their level over the dependencies that stay in
 // the strip, each level cut into steps of at most 32 rows, one row per lane.  Every value that a
 // block's rows read has a slot in the CTA's shared memory:
 //  - slot 0 holds 0 (the padding of rows with fewer than three entries);
