@@ -22,7 +22,7 @@
 //    systems, one per warp.  Its block size and warp/CTA threshold are the batch's configuration,
 //    which hgb_batch_autotune chooses by timing the candidates and caches in a small text file.
 //
-// 4,096 graph Laplacians of 64 to 4,096 rows to 1e-12 (GB300): 4.8 ms; 15.0 ms with every system in
+// 4,096 graph Laplacians of 64 to 4,096 rows to 1e-12 (GB300): 4.9 ms; 15.0 ms with every system in
 // batch_cg_kernel.
 #include "hgb_internal.cuh"
 #include "hgb_kernels.cuh"
@@ -724,7 +724,7 @@ struct hgb_batch {
     hgb_batch_config cfg{256, 256};
     int nitems = 0;
     int *item_sys = nullptr, *item_large = nullptr, *ticket = nullptr;
-    // graph of the single launch, keyed by the vectors it was captured with
+    // graph of the launches, keyed by the vectors it was captured with
     cudaGraphExec_t exec = nullptr;
     BatchArgs captured{};
 };
@@ -1009,7 +1009,7 @@ int hgb_batch_cg_solve(hgb_batch *B, const double *b, double *x, double rtol, do
     hgb_ctx *c = B->ctx;
     DeviceGuard g(c->device);
     BatchArgs A = batch_args(B, b, x, rtol, inner_rtol, max_inner, max_outer, iters, relres);
-    // the single persistent launch is captured once into a graph and replayed while the
+    // the persistent launches are captured once into a graph and replayed while the
     // vectors and controls stay the same
     bool same = B->exec && same_args(A, B->captured);
     if (!same) {

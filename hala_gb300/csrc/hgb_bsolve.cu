@@ -4,9 +4,9 @@
 // 128^3), and the time is levels x (time of one step) + hand-overs x (time of one hand-over); the
 // bytes (about 48 per row) are a tenth of it.  So everything that a step does not have to wait
 // for is off its path, and a hand-over is one store.  Measured (GB300, both sweeps): 128^3 with BF16
-// or FP32 store 179 us (a step about 140 ns, a hand-over 0.25 us inside a cluster and 1.2 us between
-// clusters), FP64 386 us (a step 300-430 ns: six to nine dependent FP64 operations of 62 cycles);
-// 512^2 FP32 225 us (1023 levels).  Before, with steps of 128 rows between barriers and every value of
+// or FP32 store 168 us (a step about 130 ns, a hand-over 0.25 us inside a cluster and 1.2 us between
+// clusters), FP64 361 us (a step 280-400 ns: six to nine dependent FP64 operations of 62 cycles);
+// 512^2 FP32 209 us (1023 levels).  With steps of 128 rows between barriers and every value of
 // another block through a ring: 322, 576 and 4550 us.
 //
 // A strip of consecutive rows (hgb_bsplan.cu) is solved a step at a time, a step being at most 32 rows

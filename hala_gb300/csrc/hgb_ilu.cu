@@ -554,7 +554,7 @@ struct hgb_ilu {
     void *svalsT = nullptr;
     double *pivT = nullptr;     // same pivots as piv (diagonal entries are their own transpose)
     Schedule LT, UT;
-    // block-local level schedules (hgb_bsolve.cu); the global-level kernel is the fallback
+    // strip schedules (hgb_bsolve.cu), where they are the shorter (ilu_prefer_levels); else L and U by level
     bool use_bs = false, use_bsT = false;
     BlockSolve BL, BU, BLT, BUT;
     hgb_zilu *z = nullptr;      // the complex factor (C128 / C64); none of the fields above is used then

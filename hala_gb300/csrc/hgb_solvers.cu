@@ -1401,8 +1401,9 @@ extern "C" int hgb_ru_pcg_solve_op(hgb_ctx *c, hgb_csr *A64, hgb_csr *Ai, hgb_il
 // last CTA of the projection's grid reduction.  Inner iteration j of a cycle always projects
 // against j+1 basis vectors, so one whole restart cycle is captured once into a CUDA graph; the
 // launches of iterations after the inner stop are no-ops, and the host reads the state once per
-// cycle.  The arithmetic of the rotations, of tpsv and of the x update is the reference's
-// operation for operation (explicitly rounded, no contraction); the inner products are parallel.
+// cycle.  The arithmetic of the rotations and of tpsv is the reference's operation for operation
+// (explicitly rounded, no contraction); the inner products are parallel, and the updates of r and x take the
+// columns in the reference's order with fused multiply-adds.
 namespace hgb {
 
 constexpr int kGmresMaxRestart = 512;   // the Hessenberg factor (1 MB) lives in device memory
@@ -1694,7 +1695,7 @@ __global__ void gm_end_kernel(GmresState *st) {
     }
 }
 
-// x += W[:, 0..k-1] Z   (krylov_combine, :53-60), column by column in the reference's order
+// x += W[:, 0..k-1] Z   (krylov_combine, :53-60), column by column, a fused multiply-add each
 template <typename X>
 __global__ void __launch_bounds__(256, 4)
 gm_xupdate_kernel(long n, const GmresState *__restrict__ st, const X *__restrict__ W, X *__restrict__ x) {
