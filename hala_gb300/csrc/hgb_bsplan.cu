@@ -129,10 +129,11 @@ struct Scratch {   // one thread's working arrays
 // line is read off the entries' distances: the largest one at most half the bandwidth (the
 // second stride of a 3D grid), or the bandwidth itself where that is the stride of a 2D grid.
 // Where the bandwidth is a whole number of lines (a grid plane), strips are cut evenly inside it, so
-// that every plane has the same ones.  No strip has more than kBsMaxStrip rows: a packet holds its row's
+// that every plane has the same ones: strips of several planes and a part run up to twice as long (15 x 13 x 13: 87 steps against
+// 54; planes of fewer than ten lines leave a strip's steps too few rows: 96 x 8 x 40 153 against 190).  No strip has more than kBsMaxStrip rows: a packet holds its row's
 // place in the strip in 16 bits, and a strip's own rows have to fit the slots.
 static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool &deep) {
-    constexpr int kMaxT = kBsMaxStrip, kMinT = 512;
+    constexpr int kMaxT = kBsMaxStrip, kMinT = 512, kMinLines = 10;
     deep = d2 >= 8;
     const int u = deep ? d2 : std::max(bw, 1);
     cut.assign(1, 0);
@@ -141,7 +142,7 @@ static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool
     } else {
         T = u > kMaxT ? kMaxT : (int)std::min<long>(32L * u, (long)(kMaxT / u) * u);
         if (T < kMinT) T = (kMinT + T - 1) / T * T;
-        if (deep && u <= kMaxT && bw % u == 0 && bw / u >= 16 && bw <= n) {
+        if (deep && u <= kMaxT && bw % u == 0 && bw / u >= kMinLines && bw <= n) {
             const int ny = bw / u, k = (bw + T - 1) / T, lines = (ny + k - 1) / k;
             T = lines * u;
             for (long p = 0; p < n; p += bw)

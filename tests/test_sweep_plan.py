@@ -93,6 +93,7 @@ def arrows(n, m, last):
 
 CASES = {
     "grid_33x17x5": lambda: grid(33, 17, 5),
+    "grid_15x13x13": lambda: grid(15, 13, 13),
     "grid_64x65x30": lambda: grid(64, 65, 30),
     "grid_256x160x40": lambda: grid(256, 160, 40),
     "grid_16384x16x3": lambda: grid(16384, 16, 3),
@@ -145,6 +146,7 @@ def permuted(pattern, seed):
 # order, or where rows list more than three entries, they follow one another
 PATHS = {
     "grid_63x65x61": (lambda: grid(63, 65, 61), 1.0, 2.0),
+    "grid_15x13x13": (lambda: grid(15, 13, 13), 1.0, 1.6),      # planes of 13 lines: a strip each
     "grid_301x97": (lambda: grid(301, 97, 1), 1.0, 2.0),
     "line_5000": (lambda: grid(5000, 1, 1), 1.0, 1.1),
     "random_30000": (lambda: random(30000, 6), 50.0, 1e4),
