@@ -44,13 +44,15 @@ constexpr int kWideMin = 64;      // entries from which a row of a tile that is 
 //   384 entries (rows of 9, which 256 would send to the direct path): FP64 2 CTAs 30.8, 3: 35.2; FP32 3 CTAs of
 //   4 gathers 16.9, of 8 20.2, 2 of 4 18.5.
 //   columns: FP64 3 CTAs with one gather per column 66.6, with two and passes of 3 + 2 columns 78.7; FP32 3 CTAs
-//   with two 28.8, 4 with three 39.0.
+//   with two 28.8, 4 with three 39.0.  Three FP32 columns (and passes of six) run 4 CTAs of three gathers: a 5-point 369 x 408
+//   grid, whose 4,705 tiles are two for some warps of 3 CTAs, 6.2 us and six columns 8.2, with 3 CTAs of four 8.2 and 10.3 (768 x
+//   700: 12.4 and 18.6, both ways).  Four columns would gain there (8.2 -> 6.2), and lose on 768 x 700 (14.4 -> 16.4).
 // One shape for all, 4 gathers, passes of 4 columns with one: 55.4 / 28.9 (25.0), 33.2 / 26.7, 108.6 / 43.1.
 template <typename X, int NC, int CAP>
 struct TileShape {
     static constexpr bool f64 = sizeof(X) == 8, wide = CAP > kCapShort;
-    static constexpr int ctas = NC == 1 ? (f64 ? (wide ? 2 : 3) : (wide ? 3 : 4)) : (wide ? 2 : (f64 && NC == 2 ? 4 : 3));
-    static constexpr int gathers = NC == 1 ? (wide ? 4 : 8) : (f64 ? (NC == 2 ? 2 : 1) : (NC == 2 ? 6 : 12 / NC));
+    static constexpr int ctas = NC == 1 ? (f64 ? (wide ? 2 : 3) : (wide ? 3 : 4)) : (wide ? 2 : (NC == (f64 ? 2 : 3) ? 4 : 3));
+    static constexpr int gathers = NC == 1 ? (wide ? 4 : 8) : (f64 ? (NC == 2 ? 2 : 1) : (NC == 2 ? 6 : (NC == 3 ? (wide ? 4 : 3) : 12 / NC)));
 };
 
 // acc += v * x in the mode's rounding
