@@ -129,9 +129,10 @@ struct Scratch {   // one thread's working arrays
 // line is read off the entries' distances: the largest one at most half the bandwidth (the
 // second stride of a 3D grid), or the bandwidth itself where that is the stride of a 2D grid.
 // Where the bandwidth is a whole number of lines (a grid plane), strips are cut evenly inside it, so
-// that every plane has the same ones: strips of several planes and a part run up to twice as long (15 x 13 x 13: 87 steps against
-// 54; planes of fewer than ten lines leave a strip's steps too few rows: 96 x 8 x 40 153 against 190).  No strip has more than kBsMaxStrip rows: a packet holds its row's
-// place in the strip in 16 bits, and a strip's own rows have to fit the slots.
+// that every plane has the same ones: strips of several planes and a part run up to twice as long (15 x 13 x 13:
+// 87 steps against 54; planes of fewer than ten lines leave a strip's steps too few rows: 96 x 8 x 40 153 against
+// 190).  No strip has more than kBsMaxStrip rows: a packet holds its row's place in the strip in 16 bits, and a
+// strip's own rows have to fit the slots.
 static void bs_strips(int n, int bw, int d2, std::vector<int> &cut, int &T, bool &deep) {
     constexpr int kMaxT = kBsMaxStrip, kMinT = 512, kMinLines = 10;
     deep = d2 >= 8;
@@ -524,18 +525,18 @@ struct Sweep {
     int strip_of(int pos) const { return (int)(std::upper_bound(cut.begin(), cut.end(), pos) - cut.begin() - 1); }
     // how far the strips of a block start behind those of earlier ones (b0: the first block of its cluster)
     void lags(int b, int b0) {
-        std::vector<Lag> *to = nullptr;
-        int of = -1;
-        for (const Use &u : out[b].use) {
-            if (u.strip != of) {
-                of = u.strip;
-                to = &lag[b * spb + of];
+        std::vector<int> late(b * spb, INT_MIN), seen;   // behind every strip of an earlier block
+        const std::vector<Use> &use = out[b].use;
+        for (size_t i = 0; i < use.size(); i++) {
+            const int pj = R.pos_of(use[i].row), ps = strip_of(pj);
+            if (late[ps] == INT_MIN) seen.push_back(ps);
+            late[ps] = std::max(late[ps], done[pj] + bs_hop_cost(xsize, ps / spb >= b0) - use[i].begin);
+            if (i + 1 < use.size() && use[i + 1].strip == use[i].strip) continue;
+            for (int s : seen) {
+                lag[b * spb + use[i].strip].push_back({s, late[s]});
+                late[s] = INT_MIN;
             }
-            const int pj = R.pos_of(u.row), ps = strip_of(pj), late = done[pj] + bs_hop_cost(xsize, ps / spb >= b0) - u.begin;
-            size_t i = 0;
-            while (i < to->size() && (*to)[i].strip != ps) i++;
-            if (i == to->size()) to->push_back({ps, late});
-            else (*to)[i].offset = std::max((*to)[i].offset, late);
+            seen.clear();
         }
     }
     // the sweep's length on the strips' clocks, each strip running as a whole from the time at which all that it waits

@@ -752,8 +752,8 @@ static int ilu_schedules(hgb_ilu *M) {
 // where a level is one row (a band of 4: 20,000 levels), 1.3 and 2.2 at 150 rows (a 301 x 290 grid), 2.0 and 2.7 at 1,300
 // (61 x 60 x 63), 2.5 to 3 at 10,000 (random patterns).  Strips of a grid in its natural order pipeline: 301 x 290 139 us a
 // pair of FP32 sweeps against 1530 by levels.  Elsewhere their steps follow one another, the more so where rows list more
-// than three entries: 27 points on 40^3 20.8 ms against 1.4, 200k rows of 6 random entries 32.6 against 0.16, 40^3
-// in a random order 6.7 against 0.09, by reverse Cuthill-McKee 0.55 against 0.32.  The estimates hold to a fifth; strips are given 1.15.
+// than three entries: 27 points on 40^3 14.0 ms against 1.4, 30k rows of 6 random entries 2.35 against 0.12, 40^3 by
+// reverse Cuthill-McKee 0.55 against 0.32.  The estimates hold to a fifth; strips are given 1.15.
 static double strips_us(const BsPlan &P) { return P.path * (P.xsize == 8 ? 0.35 : 0.14); }
 static double levels_us(const BsPlan &P, int levels) {
     const double width = std::log10(std::max(1.0, (double)P.n / levels));
