@@ -89,3 +89,42 @@ def test_apply_bit_exact(eng, rng, name, dtype):
         lev, nl = M.levels(uplo)
         lo, nlo = O.levels(p, i, do, uplo)
         assert nl == nlo and np.array_equal(lev.cpu().numpy(), lo)
+
+
+@pytest.mark.parametrize("name", ["grid_some_long_rows", "grid_permuted"])
+@pytest.mark.parametrize("host", [False, True])
+def test_mixed_store_bit_exact(eng, rng, name, host):
+    """an FP64 factor stored in FP32 (FP64 pivots), from device and from host buffers, by strips and by levels"""
+    A = sp.csr_matrix(CASES[name](rng))
+    A = sp.csr_matrix(A + sp.diags(np.asarray(abs(A).sum(1)).ravel() + 1.0 - A.diagonal()))
+    A.sort_indices()
+    p, i, v = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    fo, do, _ = O.ilu_factor(p, i, v)
+    M = E.make_ilu_host(eng, p, i, v, store=torch.float32) if host else E.make_ilu(eng, T(p), T(i), T(v), store=torch.float32)
+    for _ in range(2):
+        x = rng.standard_normal(A.shape[0]).astype(np.float32)
+        assert np.array_equal(M.apply(T(x)).cpu().numpy(), O.ilu_apply_mixed(p, i, do, fo.astype(np.float32), fo[do], x))
+
+
+def test_solves_by_levels(eng, rng):
+    """whole solves (graph replay, launches after the end as no-ops) with a preconditioner applied by levels"""
+    A = reorder(matrix(P.aniso3d(24, 23, 22)), rng.permutation(24 * 23 * 22))
+    A.sort_indices()
+    n = A.shape[0]
+    p, i, v = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    xt = rng.standard_normal(n)
+    b = A @ xt
+    tol = 1e-10 * np.linalg.norm(b)
+    fo, do, _ = O.ilu_factor(p, i, v)
+    _, ito, _ = O.cg(p, i, v, b, tol=tol, diag=do, ilu=fo)
+    a = [T(p), T(i), T(v)]
+    A64 = E.make_sparse_matrix(eng, n, *a)
+    for trans in "NT":
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        info = E.solve_cg_op(eng, A64, E.make_ilu(eng, *a), trans, T(b), x, tol, max_iter=5000)
+        assert abs(info.iterations - ito) <= max(1, ito // 20)
+        assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.01 * tol
+    A32 = E.make_sparse_matrix(eng, n, a[0], a[1], a[2].float())
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    info = E.solve_ru_pcg(eng, A64, A32, E.make_ilu(eng, *a, store=torch.bfloat16), T(b), x, tol, delta=0.01)
+    assert np.linalg.norm(b - A @ x.cpu().numpy()) <= 1.01 * tol and info.iterations <= 1.1 * ito + 2
